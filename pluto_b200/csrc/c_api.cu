@@ -289,7 +289,7 @@ size_t pluto_gqa_prefill_bwd_workspace_bytes(int batch, int seq, int q_heads, in
 
 size_t pluto_qk_prepare_bwd_workspace_bytes(int batch, int tokens, int heads, int head_dim) {
   if (batch <= 0 || tokens <= 0 || heads <= 0 || head_dim <= 0) return 0;
-  return pluto::qk_prepare_bwd_workspace_bytes(static_cast<long long>(batch) * tokens * heads, head_dim);
+  return pluto::qk_prepare_bwd_workspace_bytes(static_cast<long long>(batch) * tokens * heads, heads, head_dim);
 }
 
 int pluto_qk_prepare_bwd(pluto_stream_t stream, const void* x, size_t x_token_stride,
@@ -597,14 +597,13 @@ int pluto_gdn_out_norm_gate_bwd(pluto_stream_t stream, const void* core, int cor
                                         dcore, dz, parts),
                      "sequence DeltaNet backward (output)");
   if (rc != PLUTO_OK || !d_norm_weight) return rc;
-  return from_cuda(pluto::reduce_rows_accumulate(stream, parts, rows, dim,
-                                                 parts + static_cast<size_t>(rows) * dim, d_norm_weight),
+  return from_cuda(pluto::reduce_strips_accumulate(stream, parts, pluto::strip_count(rows), dim, d_norm_weight),
                    "sequence DeltaNet backward (norm gradient)");
 }
 
 size_t pluto_gdn_out_norm_gate_bwd_workspace_bytes(long long rows, int dim) {
   if (rows <= 0 || dim <= 0) return 0;
-  return (static_cast<size_t>(rows) * dim + pluto::reduce_rows_scratch_floats(rows, dim)) * sizeof(float);
+  return static_cast<size_t>(pluto::strip_count(rows)) * dim * sizeof(float);
 }
 
 size_t pluto_gdn_recurrence_bwd_workspace_bytes(int batch, int tokens, int key_heads, int value_heads,

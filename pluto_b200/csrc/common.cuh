@@ -148,6 +148,21 @@ __device__ __forceinline__ void sts_b32x4(uint32_t addr, uint32_t x, uint32_t y,
                : "memory");
 }
 
+// Barrier over all threads of the cluster, and a read of a peer CTA's shared memory: `addr` is this
+// CTA's address of the same variable.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float lds_cluster_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
+      : "=f"(v)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
 // ----------------------------------------------------------------------------------------------
 // TMA
 // ----------------------------------------------------------------------------------------------

@@ -74,7 +74,7 @@ struct NormBwdArgs {
   float epsilon, log_theta;
   int round;
 };
-size_t qk_prepare_bwd_workspace_bytes(long long rows, int head_dim);
+size_t qk_prepare_bwd_workspace_bytes(long long rows, int heads, int head_dim);
 cudaError_t qk_prepare_bwd(cudaStream_t stream, NormBwdArgs args, float* d_weight, void* workspace);
 
 // ---- attn_bwd_sm100.cu: tcgen05 backward, bf16, head_dim 64 or 128 -----------------------------
@@ -310,11 +310,15 @@ cudaError_t gdn_bwd_chunked(cudaStream_t stream, GdnBwdArgs& args, float* dq_out
 cudaError_t gdn_conv_bwd(cudaStream_t stream, const void* input, int in_is_bf16, const float* weight,
                          const float* dpost, int batch, int tokens, int channels, int width, int round,
                          float* dx, float* d_weight);
-// qwen_bwd.cu: dst[c] += sum over rows of parts[row, c] in a fixed order; chunk_scratch holds
-// ceil(rows / 1024) * dim floats
-cudaError_t reduce_rows_accumulate(cudaStream_t stream, const float* parts, long long rows, int dim,
-                                   float* chunk_scratch, float* dst);
-size_t reduce_rows_scratch_floats(long long rows, int dim);
+// Kernels that sum a gradient over many rows run as strip_count(rows) CTAs of eight warps, one row
+// per warp at a time, and leave one partial row per CTA: four CTAs per SM, or fewer when there are
+// not that many rows.
+inline int strip_count(long long rows) {
+  const long long wanted = (rows + 7) / 8;
+  return static_cast<int>(wanted < 4 * 148 ? wanted : 4 * 148);
+}
+// qwen_bwd.cu: dst[c] += sum over the strips of parts[strip, c] in a fixed order
+cudaError_t reduce_strips_accumulate(cudaStream_t stream, const float* parts, int strips, int dim, float* dst);
 cudaError_t gdn_gates(cudaStream_t stream, const void* a_in, const void* b_in, const float* a_log,
                       const float* dt_bias, int in_is_bf16, long long tokens, int heads, int round,
                       float* g, float* beta);

@@ -175,7 +175,8 @@ __global__ void gdn_gates_kernel(const void* a_in, const void* b_in, const float
 // `state` [B, channels, width] holds the last `width` inputs (oldest first; zero for a fresh
 // sequence).  y_t = R(SiLU(R(sum_tap w[c][tap] * x[t + tap - width + 1]))) with inputs rounded
 // first; on return the state holds the last `width` inputs of this call (the reference's
-// shift register).  One thread per (batch, channel), sequential in t.
+// shift register).  One thread per (batch, channel), sequential in t: windows wider than four
+// taps, channel counts that are not a multiple of four, and single tokens.
 __global__ void gdn_conv_kernel(const void* input, const float* weight, int in_is_bf16, int batch,
                                 int tokens, int channels, int width, int round, float* state,
                                 void* output, int out_is_bf16) {
@@ -203,9 +204,145 @@ __global__ void gdn_conv_kernel(const void* input, const float* weight, int in_i
     state[(static_cast<size_t>(b) * channels + c) * width + tap] = window[tap];
 }
 
+// Four consecutive elements of a bf16 or fp32 array (8- or 16-byte access).
+template <bool BF16>
+__device__ __forceinline__ float4 load_four(const void* p, size_t i) {
+  if (BF16) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p) + i);
+    return make_float4(bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y));
+  }
+  return *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
+}
+template <bool BF16>
+__device__ __forceinline__ void store_four(void* p, size_t i, const float (&v)[4]) {
+  if (BF16)
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p) + i) =
+        make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+  else
+    *reinterpret_cast<float4*>(static_cast<float*>(p) + i) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// The same convolution cut along the tokens: a thread owns four channels of kConvSegment tokens,
+// with the window in registers.  It is a stream (every input and output element once), so what
+// counts is that there are enough threads to keep HBM busy: one thread per channel walked all
+// tokens of a sequence by itself, 80 CTAs of dependent loads (565 us at 1000 tokens x 10240
+// channels; 30 us in this form).  Segment 0 is the only reader of the state, so it also writes the
+// new one: it never races with a later segment, which takes its history from the input.
+constexpr int kConvSegment = 16;
+template <int W, bool IN_BF16, bool OUT_BF16>
+__global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* __restrict__ input,
+                                                               const float* __restrict__ weight, int tokens,
+                                                               int channels, int round, float* state,
+                                                               void* __restrict__ output) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (c >= channels) return;
+  const int b = blockIdx.z, t0 = blockIdx.y * kConvSegment, t1 = min(tokens, t0 + kConvSegment);
+  const size_t seq = static_cast<size_t>(b) * tokens * channels + c;
+  float* own_state = state + (static_cast<size_t>(b) * channels + c) * W;   // [4][W]
+  float w[4][W], x[W][4];   // x[W-1] is the current token
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int tap = 0; tap < W; ++tap) w[i][tap] = weight[static_cast<size_t>(c + i) * W + tap];
+#pragma unroll
+  for (int tap = 1; tap < W; ++tap) {   // tokens t0 - W + tap
+    const int t = t0 - W + tap;
+    if (t >= 0) {
+      const float4 v = load_four<IN_BF16>(input, seq + static_cast<size_t>(t) * channels);
+      x[tap][0] = rnd(v.x, round); x[tap][1] = rnd(v.y, round);
+      x[tap][2] = rnd(v.z, round); x[tap][3] = rnd(v.w, round);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[tap][i] = own_state[i * W + W + t];
+    }
+  }
+#pragma unroll 4
+  for (int t = t0; t < t1; ++t) {
+    const size_t at = seq + static_cast<size_t>(t) * channels;
+    const float4 v = load_four<IN_BF16>(input, at);
+#pragma unroll
+    for (int tap = 0; tap + 1 < W; ++tap)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[tap][i] = x[tap + 1][i];
+    x[W - 1][0] = rnd(v.x, round); x[W - 1][1] = rnd(v.y, round);
+    x[W - 1][2] = rnd(v.z, round); x[W - 1][3] = rnd(v.w, round);
+    float y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int tap = 0; tap + 1 < W; ++tap) sum += x[tap][i] * w[i][tap];
+      sum = rnd(sum + x[W - 1][i] * w[i][W - 1], round);
+      y[i] = rnd(sum / (1.0f + expf(-sum)), round);
+    }
+    store_four<OUT_BF16>(output, at, y);
+  }
+  if (t0 == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float kept[W];
+#pragma unroll
+      for (int tap = 0; tap < W; ++tap) {   // token tokens - W + tap, or an entry of the old window
+        const int t = tokens - W + tap;
+        kept[tap] = t >= 0 ? rnd(load_any(input, seq + static_cast<size_t>(t) * channels + i, IN_BF16), round)
+                           : own_state[i * W + W + t];
+      }
+#pragma unroll
+      for (int tap = 0; tap < W; ++tap) own_state[i * W + tap] = kept[tap];
+    }
+  }
+}
+
 // Per (token, head): RMSNorm * weight * SiLU(z) with the reference's rounding after every product;
 // final_round = 0 leaves the last product unrounded before the store (OutputForward).
-// grid = rows (token-heads), 256 threads.
+__device__ __forceinline__ float norm_gate(float x, float inverse, float weight, float gate, int round,
+                                           int final_round) {
+  const float normalized = rnd(x * inverse, round);
+  const float affine = rnd(normalized * weight, round);
+  return rnd(affine * (gate / (1.0f + expf(-gate))), round && final_round);
+}
+
+// One warp per row, eight rows per CTA, a lane owning four consecutive channels of every 128.  HBM
+// bound; the earlier form (a CTA of 256 threads per row, half of them idle at width 128, two
+// barriers) took 49 us where this takes 14 (48000 rows of 128).
+template <int G, bool CORE_BF16, bool Z_BF16, bool OUT_BF16>   // G groups of 128 channels
+__global__ void __launch_bounds__(256) gdn_output_rows_kernel(const void* __restrict__ core, const void* __restrict__ z,
+                                                              const float* __restrict__ norm_weight, long long rows,
+                                                              int dim, float epsilon, int round, int final_round,
+                                                              void* __restrict__ output) {
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + threadIdx.x / 32;
+  if (row >= rows) return;
+  const int lane = threadIdx.x % 32;
+  const size_t base = static_cast<size_t>(row) * dim;
+  float4 x[G], gate[G];
+  float sq = 0.0f;
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    const int c = i * 128 + lane * 4;
+    x[i] = gate[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < dim) {
+      x[i] = load_four<CORE_BF16>(core, base + c);
+      gate[i] = load_four<Z_BF16>(z, base + c);
+    }
+    sq += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  const float inverse = rsqrtf(sq / static_cast<float>(dim) + epsilon);
+#pragma unroll
+  for (int i = 0; i < G; ++i) {
+    const int c = i * 128 + lane * 4;
+    if (c >= dim) continue;
+    const float4 w = *reinterpret_cast<const float4*>(norm_weight + c);
+    const float y[4] = {norm_gate(x[i].x, inverse, w.x, gate[i].x, round, final_round),
+                        norm_gate(x[i].y, inverse, w.y, gate[i].y, round, final_round),
+                        norm_gate(x[i].z, inverse, w.z, gate[i].z, round, final_round),
+                        norm_gate(x[i].w, inverse, w.w, gate[i].w, round, final_round)};
+    store_four<OUT_BF16>(output, base + c, y);
+  }
+}
+
+// The same for widths or addresses the four-channel accesses do not fit: grid = rows, 256 threads.
 __global__ void __launch_bounds__(256) gdn_output_kernel(const void* core, const void* z,
                                                          const float* norm_weight, int core_is_bf16,
                                                          int z_is_bf16, int dim, float epsilon,
@@ -225,11 +362,19 @@ __global__ void __launch_bounds__(256) gdn_output_kernel(const void* core, const
   for (int w = 0; w < 8; ++w) total += red[w];
   if (c >= dim) return;
   const float inverse = rsqrtf(total / static_cast<float>(dim) + epsilon);
-  const float normalized = rnd(x * inverse, round);
-  const float affine = rnd(normalized * norm_weight[c], round);
-  const float gate = load_any(z, row * dim + c, z_is_bf16);
-  const float silu = gate / (1.0f + expf(-gate));
-  store_any(output, row * dim + c, out_is_bf16, rnd(affine * silu, round && final_round));
+  store_any(output, row * dim + c, out_is_bf16,
+            norm_gate(x, inverse, norm_weight[c], load_any(z, row * dim + c, z_is_bf16), round, final_round));
+}
+
+bool aligned_to(const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; }
+
+template <int W>
+void launch_conv_segments(cudaStream_t stream, const void* input, const float* weight, int in_is_bf16, int batch,
+                          int tokens, int channels, int round, float* state, void* output, int out_is_bf16) {
+  const dim3 grid((channels / 4 + 127) / 128, (tokens + kConvSegment - 1) / kConvSegment, batch);
+  auto kernel = in_is_bf16 ? (out_is_bf16 ? gdn_conv_segment_kernel<W, true, true> : gdn_conv_segment_kernel<W, true, false>)
+                           : (out_is_bf16 ? gdn_conv_segment_kernel<W, false, true> : gdn_conv_segment_kernel<W, false, false>);
+  kernel<<<grid, 128, 0, stream>>>(input, weight, tokens, channels, round, state, output);
 }
 
 }  // namespace
@@ -252,6 +397,15 @@ cudaError_t gdn_gates(cudaStream_t stream, const void* a_in, const void* b_in, c
 cudaError_t gdn_conv(cudaStream_t stream, const void* input, const float* weight, int in_is_bf16,
                      int batch, int tokens, int channels, int width, int round, float* state,
                      void* output, int out_is_bf16) {
+  // four-tap windows and shorter over several tokens: cut along the tokens (a single token has
+  // nothing to cut, and grid.y / grid.z bound what one launch can hold)
+  if (width >= 2 && width <= 4 && tokens > 1 && channels % 4 == 0 && batch <= 65535 &&
+      (tokens + kConvSegment - 1) / kConvSegment <= 65535 && aligned_to(input, in_is_bf16 ? 8 : 16) &&
+      aligned_to(output, out_is_bf16 ? 8 : 16)) {
+    auto launch = width == 4 ? launch_conv_segments<4> : width == 3 ? launch_conv_segments<3> : launch_conv_segments<2>;
+    launch(stream, input, weight, in_is_bf16, batch, tokens, channels, round, state, output, out_is_bf16);
+    return cudaGetLastError();
+  }
   const long long count = static_cast<long long>(batch) * channels;
   gdn_conv_kernel<<<static_cast<unsigned>((count + 127) / 128), 128, 0, stream>>>(
       input, weight, in_is_bf16, batch, tokens, channels, width, round, state, output, out_is_bf16);
@@ -262,6 +416,21 @@ cudaError_t gdn_output(cudaStream_t stream, const void* core, const void* z,
                        const float* norm_weight, int core_is_bf16, int z_is_bf16, long long rows,
                        int dim, float epsilon, int round, int final_round, void* output,
                        int out_is_bf16) {
+  if (dim % 4 == 0 && aligned_to(core, core_is_bf16 ? 8 : 16) && aligned_to(z, z_is_bf16 ? 8 : 16) &&
+      aligned_to(norm_weight, 16) && aligned_to(output, out_is_bf16 ? 8 : 16)) {
+    using Kernel = void (*)(const void*, const void*, const float*, long long, int, float, int, int, void*);
+#define OUTPUT_ROWS(G)                                                                                  \
+    {gdn_output_rows_kernel<G, false, false, false>, gdn_output_rows_kernel<G, false, false, true>,     \
+     gdn_output_rows_kernel<G, false, true, false>,  gdn_output_rows_kernel<G, false, true, true>,      \
+     gdn_output_rows_kernel<G, true, false, false>,  gdn_output_rows_kernel<G, true, false, true>,      \
+     gdn_output_rows_kernel<G, true, true, false>,   gdn_output_rows_kernel<G, true, true, true>}
+    static const Kernel kernels[2][8] = {OUTPUT_ROWS(1), OUTPUT_ROWS(2)};
+#undef OUTPUT_ROWS
+    kernels[dim <= 128 ? 0 : 1][(core_is_bf16 ? 4 : 0) + (z_is_bf16 ? 2 : 0) + (out_is_bf16 ? 1 : 0)]
+        <<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(core, z, norm_weight, rows, dim, epsilon, round,
+                                                                    final_round, output);
+    return cudaGetLastError();
+  }
   gdn_output_kernel<<<static_cast<unsigned>(rows), 256, 0, stream>>>(
       core, z, norm_weight, core_is_bf16, z_is_bf16, dim, epsilon, round, final_round, output,
       out_is_bf16);

@@ -2,7 +2,7 @@
 // (src/llm/layers/qwen_attention.cc:120-239): the sigmoid output gate, the inverse partial RoPE
 // followed by the per-head RMSNorm backward, and the deterministic reduction of the shared
 // norm-weight gradient.  The attention core between them runs in attn_generic.cu
-// (gqa_generic_bwd).  One CTA of 256 threads per (token, head); head width <= 256.
+// (gqa_generic_bwd).  Head width <= 256.
 #include "common.cuh"
 #include "engine.h"
 
@@ -11,17 +11,10 @@ namespace {
 
 __device__ __forceinline__ float rnd(float v, int round) { return round ? bf16_round(v) : v; }
 
-// Sum over the 256 threads of a CTA in a fixed order (warp shuffles, then warp 0..7 in sequence).
-__device__ __forceinline__ float block_sum(float v, float* red) {
+__device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();   // red may still be read from a previous call
-  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = v;
-  __syncthreads();
-  float total = 0.0f;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) total += red[w];
-  return total;
+  return v;
 }
 
 // GateBackwardKernel (:123-138): dc = dy * R(sigmoid(gate)); d_gate = dy * R(core) * s * (1 - s),
@@ -76,60 +69,132 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwdArgs a, long long 
 }
 
 // NormBackwardKernel (:196-226): rotate the gradient back with the rounded cos/sin of the forward,
-// then the RMSNorm backward; `parts` (optional) receives normalized_grad * x * inv per row.
-__global__ void __launch_bounds__(256) norm_bwd_kernel(NormBwdArgs a) {
-  __shared__ float red[8];
-  const int token = blockIdx.x / a.heads, h = blockIdx.x % a.heads;
-  const int b = token / a.tokens, t = token % a.tokens;
-  const int c = threadIdx.x, D = a.head_dim;
-  const int position = (a.positions ? a.positions[b] : 0) + t;
-  const size_t dense = (static_cast<size_t>(token) * a.heads + h) * D;
-  const size_t in0 = static_cast<size_t>(token) * a.x_token + static_cast<size_t>(h) * a.x_head;
-  const float x = c < D ? __bfloat162float(a.x[in0 + c]) : 0.0f;
-  const float inv = rsqrtf(block_sum(x * x, red) / static_cast<float>(D) + a.epsilon);
-  float ng = 0.0f, weighted = 0.0f;
-  if (c < D) {
-    ng = a.grad[dense + c];
-    if (c < a.rotary) {
-      const int half = a.rotary / 2;
-      const int partner = c < half ? c + half : c - half;
-      const int f = c < half ? c : c - half;
+// then the RMSNorm backward; `parts` (optional) receives one row per CTA of the sums of
+// normalized_grad * x * inv, the norm-weight gradient.
+// A CTA walks blocks of `per_block` tokens: their cos / sin tables go to shared memory, then every
+// warp takes (token, head) rows, a lane owning kPer channels of every 32 * kPer.  HBM bound; the
+// earlier form (a CTA per row with its own sines, the per-row parts written out and reduced from
+// memory by 24 CTAs) took 64 + 71 us at 1000 tokens of 24 and 4 heads of 256, this 29 + 8.
+constexpr int kBlockTokens = 8;   // tokens of one block when a token has a single head
+template <int kPer>
+__global__ void __launch_bounds__(256) norm_bwd_kernel(NormBwdArgs a, int per_block) {
+  constexpr int kOwn = 8;   // channels a lane owns at width 256
+  __shared__ float cosine[kBlockTokens][128], sine[kBlockTokens][128];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int D = a.head_dim, half = a.rotary / 2, tokens = a.batch * a.tokens;
+  auto channel = [&](int i) { return (i / kPer) * 32 * kPer + lane * kPer; };   // first of the kPer at i
+  float weight[kOwn], sum[kOwn];
+#pragma unroll
+  for (int i = 0; i < kOwn; ++i) {
+    const int c = channel(i) + i % kPer;
+    weight[i] = c < D ? 1.0f + a.weight[c] : 0.0f;
+    sum[i] = 0.0f;
+  }
+  for (int first = blockIdx.x * per_block; first < tokens; first += gridDim.x * per_block) {
+    const int count = min(per_block, tokens - first);
+    __syncthreads();   // the previous block's rows are done with the tables
+    for (int i = threadIdx.x; i < count * half; i += 256) {
+      const int token = first + i / half, f = i % half;
+      const int position = (a.positions ? a.positions[token / a.tokens] : 0) + token % a.tokens;
       const float angle = static_cast<float>(position) *
                           expf(static_cast<float>(f) * (-2.0f * a.log_theta / static_cast<float>(a.rotary)));
-      const float co = rnd(cosf(angle), a.round), si = rnd(sinf(angle), a.round);
-      const float gp = a.grad[dense + partner];
-      ng = ng * co + (c < half ? gp * si : -gp * si);
+      cosine[i / half][f] = rnd(cosf(angle), a.round);
+      sine[i / half][f] = rnd(sinf(angle), a.round);
     }
-    weighted = ng * (1.0f + a.weight[c]);
+    __syncthreads();
+    for (int row = warp; row < count * a.heads; row += 8) {
+      const int own = row / a.heads, token = first + own, h = row % a.heads;
+      const size_t dense = (static_cast<size_t>(token) * a.heads + h) * D;
+      const __nv_bfloat16* in = a.x + static_cast<size_t>(token) * a.x_token + static_cast<size_t>(h) * a.x_head;
+      float* out = a.dx + static_cast<size_t>(token) * a.dx_token + static_cast<size_t>(h) * a.dx_head;
+      float x[kOwn], ng[kOwn];
+      float sq = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kOwn; i += kPer) {
+        const int c = channel(i);
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) x[i + u] = ng[i + u] = 0.0f;
+        if (c >= D) continue;
+        if (kPer == 4) {
+          const uint2 raw = *reinterpret_cast<const uint2*>(in + c);
+          x[i] = bf16_lo(raw.x); x[i + 1] = bf16_hi(raw.x); x[i + 2] = bf16_lo(raw.y); x[i + 3] = bf16_hi(raw.y);
+          const float4 g = *reinterpret_cast<const float4*>(a.grad + dense + c);
+          ng[i] = g.x; ng[i + 1] = g.y; ng[i + 2] = g.z; ng[i + 3] = g.w;
+        } else {
+          x[i] = __bfloat162float(in[c]);
+          ng[i] = a.grad[dense + c];
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) sq += x[i + u] * x[i + u];
+        if (c < a.rotary) {
+          float p[kPer];
+          const size_t partner = dense + (c < half ? c + half : c - half);
+          if (kPer == 4) {
+            const float4 g = *reinterpret_cast<const float4*>(a.grad + partner);
+            p[0] = g.x; p[1] = g.y; p[2] = g.z; p[3] = g.w;
+          } else {
+            p[0] = a.grad[partner];
+          }
+#pragma unroll
+          for (int u = 0; u < kPer; ++u) {
+            const int f = (c < half ? c : c - half) + u;
+            ng[i + u] = ng[i + u] * cosine[own][f] + (c < half ? p[u] * sine[own][f] : -p[u] * sine[own][f]);
+          }
+        }
+      }
+      const float inv = rsqrtf(warp_sum(sq) / static_cast<float>(D) + a.epsilon);
+      float dot = 0.0f;
+#pragma unroll
+      for (int i = 0; i < kOwn; ++i) {
+        dot += ng[i] * weight[i] * x[i];
+        sum[i] = fmaf(ng[i] * x[i], inv, sum[i]);
+      }
+      dot = warp_sum(dot);
+      const float scale = inv * inv * inv / static_cast<float>(D);
+#pragma unroll
+      for (int i = 0; i < kOwn; i += kPer) {
+        const int c = channel(i);
+        if (c >= D) continue;
+        float dx[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) dx[u] = inv * (ng[i + u] * weight[i + u]) - x[i + u] * scale * dot;
+        if (kPer == 4) *reinterpret_cast<float4*>(out + c) = make_float4(dx[0], dx[1], dx[2], dx[3]);
+        else out[c] = dx[0];
+      }
+    }
   }
-  const float dot = block_sum(weighted * x, red);
-  if (c < D) {
-    a.dx[static_cast<size_t>(token) * a.dx_token + static_cast<size_t>(h) * a.dx_head + c] =
-        inv * weighted - x * (inv * inv * inv / static_cast<float>(D)) * dot;
-    if (a.parts) a.parts[dense + c] = ng * x * inv;
+  if (a.parts == nullptr) return;
+  __shared__ float strip[8][256];
+#pragma unroll
+  for (int i = 0; i < kOwn; ++i)
+    if (channel(i) + i % kPer < D) strip[warp][channel(i) + i % kPer] = sum[i];
+  __syncthreads();
+  if (static_cast<int>(threadIdx.x) < D) {
+    float total = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) total += strip[i][threadIdx.x];
+    a.parts[static_cast<size_t>(blockIdx.x) * D + threadIdx.x] = total;
   }
 }
 
-// ReduceNormKernel (:228-239) in two fixed-order levels: CTA i sums rows [i*kChunk, (i+1)*kChunk)
-// per column, then one CTA sums the chunk rows in order and accumulates into the gradient.
-constexpr int kChunk = 1024;
-__global__ void __launch_bounds__(256) norm_reduce_chunks(const float* parts, long long rows, int D,
-                                                          float* chunk_sums) {
-  const int c = threadIdx.x;
-  if (c >= D) return;
-  const long long r0 = static_cast<long long>(blockIdx.x) * kChunk;
-  const long long r1 = r0 + kChunk < rows ? r0 + kChunk : rows;
+// dst[c] += sum over the strips of parts[strip, c], in a fixed order: a CTA per 32 columns, whose 32
+// warps take contiguous runs of the strips and add the runs' sums in order.
+__global__ void __launch_bounds__(1024) reduce_strips_kernel(const float* __restrict__ parts, int strips, int dim,
+                                                             float* dst) {
+  __shared__ float run_sum[32][32];
+  const int lane = threadIdx.x % 32, run = threadIdx.x / 32, c = blockIdx.x * 32 + lane;
+  const int length = (strips + 31) / 32;
   float sum = 0.0f;
-  for (long long r = r0; r < r1; ++r) sum += parts[r * D + c];
-  chunk_sums[static_cast<size_t>(blockIdx.x) * D + c] = sum;
-}
-__global__ void __launch_bounds__(256) norm_reduce_final(const float* chunk_sums, int chunks, int D,
-                                                         float* dw) {
-  const int c = threadIdx.x;
-  if (c >= D) return;
-  float sum = 0.0f;
-  for (int i = 0; i < chunks; ++i) sum += chunk_sums[static_cast<size_t>(i) * D + c];
-  dw[c] += sum;
+  if (c < dim) {
+#pragma unroll 8
+    for (int s = run * length; s < min(strips, (run + 1) * length); ++s) sum += parts[static_cast<size_t>(s) * dim + c];
+  }
+  run_sum[run][lane] = sum;
+  __syncthreads();
+  if (run != 0 || c >= dim) return;
+#pragma unroll
+  for (int i = 1; i < 32; ++i) sum += run_sum[i][lane];
+  dst[c] += sum;
 }
 
 }  // namespace
@@ -147,32 +212,37 @@ cudaError_t gqa_gate_bwd(cudaStream_t stream, const GateBwdArgs& a) {
   return cudaGetLastError();
 }
 
-size_t qk_prepare_bwd_workspace_bytes(long long rows, int head_dim) {
-  const long long chunks = (rows + kChunk - 1) / kChunk;
-  return static_cast<size_t>(rows + chunks) * head_dim * sizeof(float);
+namespace {
+int norm_block_tokens(int heads) { return heads >= kBlockTokens ? 1 : kBlockTokens / heads; }
+int norm_strips(long long rows, int heads) {   // CTAs of the norm backward, and rows of its partial sums
+  const long long per_block = norm_block_tokens(heads), tokens = rows / heads;
+  const long long blocks = (tokens + per_block - 1) / per_block;
+  return static_cast<int>(blocks < 4 * 148 ? blocks : 4 * 148);
+}
+}  // namespace
+
+size_t qk_prepare_bwd_workspace_bytes(long long rows, int heads, int head_dim) {
+  return static_cast<size_t>(norm_strips(rows, heads)) * head_dim * sizeof(float);
 }
 
 cudaError_t qk_prepare_bwd(cudaStream_t stream, NormBwdArgs a, float* d_weight, void* workspace) {
   const long long rows = static_cast<long long>(a.batch) * a.tokens * a.heads;
   a.parts = d_weight ? static_cast<float*>(workspace) : nullptr;
-  norm_bwd_kernel<<<static_cast<unsigned>(rows), 256, 0, stream>>>(a);
+  const int strips = norm_strips(rows, a.heads);
+  const auto aligned = [](const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
+  // four-channel accesses: every row and the rotary halves start on a multiple of four elements
+  const bool vector = a.head_dim % 4 == 0 && a.rotary % 8 == 0 && a.x_token % 4 == 0 && a.x_head % 4 == 0 &&
+                      a.dx_token % 4 == 0 && a.dx_head % 4 == 0 && aligned(a.x, 8) && aligned(a.grad, 16) &&
+                      aligned(a.dx, 16);
+  auto kernel = vector ? norm_bwd_kernel<4> : norm_bwd_kernel<1>;
+  kernel<<<strips, 256, 0, stream>>>(a, norm_block_tokens(a.heads));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || d_weight == nullptr) return e;
-  return reduce_rows_accumulate(stream, a.parts, rows, a.head_dim,
-                                a.parts + static_cast<size_t>(rows) * a.head_dim, d_weight);
+  return reduce_strips_accumulate(stream, a.parts, strips, a.head_dim, d_weight);
 }
 
-size_t reduce_rows_scratch_floats(long long rows, int dim) {
-  return static_cast<size_t>((rows + kChunk - 1) / kChunk) * dim;
-}
-
-cudaError_t reduce_rows_accumulate(cudaStream_t stream, const float* parts, long long rows, int dim,
-                                   float* chunk_scratch, float* dst) {
-  const int chunks = static_cast<int>((rows + kChunk - 1) / kChunk);
-  norm_reduce_chunks<<<chunks, 256, 0, stream>>>(parts, rows, dim, chunk_scratch);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  norm_reduce_final<<<1, 256, 0, stream>>>(chunk_scratch, chunks, dim, dst);
+cudaError_t reduce_strips_accumulate(cudaStream_t stream, const float* parts, int strips, int dim, float* dst) {
+  reduce_strips_kernel<<<(dim + 31) / 32, 1024, 0, stream>>>(parts, strips, dim, dst);
   return cudaGetLastError();
 }
 
