@@ -161,16 +161,6 @@ attn_bwd_prep(const __nv_bfloat16* __restrict__ out, const float* __restrict__ d
   }
 }
 
-// One row of a TMA-written [rows x 64 bf16] slab (128-byte swizzle) into 32 registers: the 16-byte
-// chunk c of row r lies at chunk position c ^ (r & 7).
-__device__ __forceinline__ void load_swizzled_row(uint32_t slab, int row, uint32_t (&w)[32]) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const uint4 v = lds_b32x4(slab + row * 128 + ((c ^ (row & 7)) << 4));
-    w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
-  }
-}
-
 // 32 accumulator columns of one row, scaled, into the row's slot of a staging tile in shared
 // memory.  The tiles leave as one linear bulk copy per row: a thread writing its own row to global
 // memory touches 32 different lines per warp instruction, which cost 4 to 5 us per CTA.  Rows
@@ -1463,7 +1453,7 @@ cudaError_t attn_bwd_tc(cudaStream_t stream, const void* qkv, const void* out, c
   a.workspace = workspace;
   a.batch = batch; a.seq = seq; a.q_heads = heads; a.kv_heads = heads; a.head_dim = head_dim;
   a.status = status;
-  return gqa_bwd_tc(stream, a);
+  return head_dim == 256 ? attn_bwd_wide_tc(stream, a) : gqa_bwd_tc(stream, a);
 }
 
 }  // namespace pluto

@@ -52,7 +52,15 @@ int check_mha(int batch, int seq, int heads, int head_dim, int dtype) {
 }
 
 bool tensor_core_shape(int head_dim, int dtype) {
-  return dtype == PLUTO_BF16 && (head_dim == 64 || head_dim == 128);
+  return dtype == PLUTO_BF16 && (head_dim == 64 || head_dim == 128 || head_dim == 256);
+}
+
+cudaError_t launch_fwd_tc(cudaStream_t stream, const pluto::AttnFwdArgs& a) {
+  return a.head_dim == 256 ? pluto::attn_fwd_wide_tc(stream, a) : pluto::attn_fwd_tc(stream, a);
+}
+size_t bwd_tc_workspace_bytes(int batch, int seq, int heads, int head_dim) {
+  return head_dim == 256 ? pluto::attn_bwd_wide_workspace_bytes(batch, seq, heads)
+                         : pluto::attn_bwd_tc_workspace_bytes(batch, seq, heads, head_dim);
 }
 
 }  // namespace
@@ -87,7 +95,7 @@ int pluto_attn_fwd(pluto_stream_t stream, const void* qkv, void* out, float* max
     a.maxima = maxima; a.normalizers = normalizers;
     a.status = pluto::kernel_status_word();
     if (!a.status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
-    return from_cuda(pluto::attn_fwd_tc(stream, a), "attention forward (tcgen05) launch");
+    return from_cuda(launch_fwd_tc(stream, a), "attention forward (tcgen05) launch");
   }
   const char* base = static_cast<const char*>(qkv);
   const size_t es = dtype == PLUTO_BF16 ? 2 : 4;
@@ -131,7 +139,7 @@ int pluto_attn_bwd(pluto_stream_t stream, const void* qkv, const void* out, cons
 
 size_t pluto_attn_bwd_workspace_bytes(int batch, int seq, int heads, int head_dim, int dtype) {
   if (batch <= 0 || seq <= 0 || heads <= 0 || !tensor_core_shape(head_dim, dtype)) return 0;
-  return pluto::attn_bwd_tc_workspace_bytes(batch, seq, heads, head_dim);
+  return bwd_tc_workspace_bytes(batch, seq, heads, head_dim);
 }
 
 int pluto_attn_probs(pluto_stream_t stream, const void* qkv, const float* maxima,
@@ -174,7 +182,10 @@ int pluto_gqa_prefill_fwd(pluto_stream_t stream, const void* q, const void* gate
   const bool tma_ok = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
                       q_token_stride % 8 == 0 && q_head_stride % 8 == 0 &&
                       q_token_stride <= 0x7fffffffu;
-  if ((head_dim == 64 || head_dim == 128) && tma_ok) {
+  // head width 256 reads the gate and writes the core in 16-byte pieces
+  const bool wide_ok = head_dim == 256 && aligned16(core) &&
+                       (gate == nullptr || (aligned16(gate) && gate_token_stride % 8 == 0 && gate_head_stride % 8 == 0));
+  if ((head_dim == 64 || head_dim == 128 || wide_ok) && tma_ok) {
     pluto::AttnFwdArgs a{};
     a.q = q; a.k = k; a.v = v;
     a.q_cols = static_cast<int>((static_cast<size_t>(q_heads) - 1) * q_head_stride + head_dim);
@@ -188,12 +199,12 @@ int pluto_gqa_prefill_fwd(pluto_stream_t stream, const void* q, const void* gate
     a.gate = gate; a.gate_token = gate_token_stride; a.gate_head = gate_head_stride;
     a.round_gate = round_to_bf16;
     // the optional workspace enables the key/value split for shapes with few (sequence, head) units
-    if (workspace != nullptr && aligned16(workspace) &&
+    if (workspace != nullptr && head_dim != 256 && aligned16(workspace) &&
         workspace_bytes >= pluto::attn_fwd_tc_workspace_bytes(batch, seq, q_heads, head_dim))
       a.workspace = workspace;
     a.status = pluto::kernel_status_word();
     if (!a.status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
-    return from_cuda(pluto::attn_fwd_tc(stream, a), "GQA prefill (tcgen05) launch");
+    return from_cuda(launch_fwd_tc(stream, a), "GQA prefill (tcgen05) launch");
   }
   return from_cuda(
       pluto::attn_generic_fwd(stream, q, k, v, out, maxima, normalizers, batch, seq, q_heads,
@@ -247,7 +258,7 @@ int pluto_gqa_prefill_bwd(pluto_stream_t stream, const void* q, const void* k, c
   if (workspace != nullptr && tensor_core_shape(head_dim, dtype) && q_head_stride == D &&
       q_token_stride % 8 == 0 && q_token_stride <= 0x7fffffffu && aligned16(q) && aligned16(k) &&
       aligned16(v) && aligned16(dc) && aligned16(workspace)) {
-    if (workspace_bytes < pluto::attn_bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim))
+    if (workspace_bytes < bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim))
       return fail(PLUTO_E_INVALID, "attention backward workspace is too small");
     pluto::GqaBwdTcArgs t{};
     t.q = q; t.k = k; t.v = v; t.out = nullptr;
@@ -261,7 +272,8 @@ int pluto_gqa_prefill_bwd(pluto_stream_t stream, const void* q, const void* k, c
     t.batch = batch; t.seq = seq; t.q_heads = q_heads; t.kv_heads = kv_heads; t.head_dim = head_dim;
     t.status = pluto::kernel_status_word();
     if (!t.status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
-    return from_cuda(pluto::gqa_bwd_tc(stream, t), "sequence full attention backward (tcgen05)");
+    return from_cuda(head_dim == 256 ? pluto::attn_bwd_wide_tc(stream, t) : pluto::gqa_bwd_tc(stream, t),
+                     "sequence full attention backward (tcgen05)");
   }
   pluto::GqaBwdArgs a{};
   a.q = q; a.k = k; a.v = v; a.out = nullptr;
@@ -284,7 +296,7 @@ size_t pluto_gqa_prefill_fwd_workspace_bytes(int batch, int seq, int q_heads, in
 
 size_t pluto_gqa_prefill_bwd_workspace_bytes(int batch, int seq, int q_heads, int head_dim, int dtype) {
   if (batch <= 0 || seq <= 0 || q_heads <= 0 || !tensor_core_shape(head_dim, dtype)) return 0;
-  return pluto::attn_bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim);
+  return bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim);
 }
 
 size_t pluto_qk_prepare_bwd_workspace_bytes(int batch, int tokens, int heads, int head_dim) {

@@ -388,6 +388,16 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16_majors(int m, int n, bool
   return umma_idesc_bf16(m, n, b_mn_major) | (static_cast<uint32_t>(a_mn_major) << 15);
 }
 
+// One row of a TMA-written [rows x 64 bf16] slab (128-byte swizzle) into 32 registers: the 16-byte
+// chunk c of row r lies at chunk position c ^ (r & 7).
+__device__ __forceinline__ void load_swizzled_row(uint32_t slab, int row, uint32_t (&w)[32]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint4 v = lds_b32x4(slab + row * 128 + ((c ^ (row & 7)) << 4));
+    w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
+  }
+}
+
 // ----------------------------------------------------------------------------------------------
 // small math helpers
 // ----------------------------------------------------------------------------------------------

@@ -132,6 +132,12 @@ size_t attn_fwd_tc_split_workspace_bytes(int batch, int seq, int heads, int head
 bool make_token_map(CUtensorMap* map, const void* base, int cols, int seq, int batch,
                     size_t token_stride, int box_rows);
 
+// ---- attn_wide_sm100.cu: tcgen05 forward and backward, bf16, head_dim 256 -------------------------
+// Contracts as attn_fwd_tc (no workspace, no tile range) and gqa_bwd_tc; gate rows and core 16-byte
+// aligned, q dense (head stride 256).
+cudaError_t attn_fwd_wide_tc(cudaStream_t stream, const AttnFwdArgs& args);
+size_t attn_bwd_wide_workspace_bytes(int batch, int seq, int heads);
+cudaError_t attn_bwd_wide_tc(cudaStream_t stream, const GqaBwdTcArgs& args);
 
 // ---- gqa_decode.cu ------------------------------------------------------------------------------
 // Cache addressing: token t of sequence b, kv head h starts at element

@@ -1,0 +1,97 @@
+"""Head width 256 on the tensor cores (attn_wide_sm100.cu) against a float64 statement of the same
+attention and against the exact fp32 kernels, at the edges of its 128-row tiles and 64-row steps."""
+import math
+
+import pytest
+import torch
+
+from pluto_b200 import _capi
+from pluto_b200.layers import gqa_prefill
+
+pytestmark = pytest.mark.gpu
+D = 256
+# (batch, tokens, query heads, key/value heads): one row, either side of a step and of a tile, several
+# tiles, grouped and ungrouped heads, and a shape whose CTAs walk several heads of a group
+SHAPES = [(1, 1, 2, 1), (2, 63, 3, 3), (1, 65, 6, 1), (2, 127, 2, 2), (1, 128, 24, 4), (3, 129, 4, 2),
+          (1, 257, 6, 2), (1, 640, 12, 2), (1, 1000, 24, 4), (6, 300, 24, 2)]
+
+
+def make(shape, seed=0):
+    b, t, hq, hkv = shape
+    gen = torch.Generator(device="cuda").manual_seed(seed + t)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    return rnd(b, t, hq, D).bfloat16(), rnd(b, t, hkv, D).bfloat16(), rnd(b, t, hkv, D).bfloat16(), rnd(b, t, hq, D)
+
+
+def reference(q, k, v):
+    """(output, maxima, normalizers) in float64."""
+    b, t, hq, _ = q.shape
+    group = hq // k.shape[2]
+    kk, vv = (x.double().repeat_interleave(group, 2) for x in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), kk) / math.sqrt(D)
+    s = s.masked_fill(torch.triu(torch.ones(t, t, dtype=torch.bool, device="cuda"), 1), -math.inf)
+    m = s.amax(-1)
+    e = torch.exp(s - m[..., None])
+    l = e.sum(-1)
+    return torch.einsum("bhqk,bkhd->bqhd", e / l[..., None], vv), m, l
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_forward(shape):
+    q, k, v, _ = make(shape)
+    want, m, l = reference(q, k, v)
+    got = gqa_prefill(q, k, v, want_core=True, want_stats=True)
+    # P enters P V as two bf16 parts (2^-17 relative) and ex2.approx is good to 2^-22; values are sums
+    # of |p| <= 1 weighted N(0, 1) entries, so 2^-15 absolute leaves room for the fp32 accumulation
+    assert (got["core"].double() - want).abs().max().item() < 3.1e-5
+    assert torch.equal(got["out"], got["core"].bfloat16())
+    assert (got["maxima"].view_as(m).double() - m).abs().max().item() < 1e-5
+    assert ((got["normalizers"].view_as(l).double() - l) / l).abs().max().item() < 1e-4
+
+
+def test_forward_gate_strided_query_and_growing_maxima():
+    b, t, hq, hkv = 2, 300, 6, 2
+    q, k, v, g = make((b, t, hq, hkv), 3)
+    k = (k.float() * torch.linspace(0.2, 6.0, t, device="cuda")[None, :, None, None]).bfloat16()   # rescales in most steps
+    both = torch.stack([q, g.bfloat16()], 3)   # [b, t, hq, 2, D]
+    want = gqa_prefill(q, k, v, want_core=True)["core"]
+    got = gqa_prefill(both[:, :, :, 0], k, v, gate=both[:, :, :, 1], want_core=True)
+    assert (want.double() - reference(q, k, v)[0]).abs().max().item() < 6.2e-5   # |s| up to 100: 2^-24 * 100 in the exponent
+    assert torch.equal(got["core"], want)
+    sigmoid = torch.sigmoid(both[:, :, :, 1].float()).bfloat16().float()
+    expected = want.bfloat16().float() * sigmoid
+    assert ((got["out"].float() - expected).abs() <= 2 ** -7 * expected.abs() + 1e-30).all()   # one bf16 ulp: rounding ties of the sigmoid
+
+
+def backward(q, k, v, d_out, stats, workspace):
+    b, t, hq, _ = q.shape
+    hkv = k.shape[2]
+    L, stream = _capi.lib(), torch.cuda.current_stream().cuda_stream
+    dq, dk, dv = torch.empty_like(d_out), torch.empty(b, t, hkv, D, device="cuda"), torch.empty(b, t, hkv, D, device="cuda")
+    deltas = (d_out * stats["core"]).sum(-1).permute(0, 2, 1).contiguous()
+    size = L.pluto_gqa_prefill_bwd_workspace_bytes(b, t, hq, D, 1) if workspace else 0
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda") if workspace else None
+    _capi.check(L.pluto_gqa_prefill_bwd(stream, q.data_ptr(), k.data_ptr(), v.data_ptr(), 1, hq * D, D, d_out.data_ptr(),
+                                        stats["maxima"].data_ptr(), stats["normalizers"].data_ptr(), deltas.data_ptr(),
+                                        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr() if workspace else None,
+                                        size, b, t, hq, hkv, D))
+    torch.cuda.synchronize()
+    return dq, dk, dv
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_backward_matches_exact_kernels_and_repeats(shape):
+    q, k, v, d_out = make(shape)
+    stats = gqa_prefill(q, k, v, want_core=True, want_stats=True)
+    exact = backward(q, k, v, d_out, stats, False)
+    got = backward(q, k, v, d_out, stats, True)
+    again = backward(q, k, v, d_out, stats, True)
+    for name, x, y, z in zip(("dq", "dk", "dv"), got, exact, again):
+        assert torch.equal(x, z), name
+        # Every operand carries 16 bits (2^-17 relative, random signs), products accumulate in fp32: 3e-5
+        # of the largest gradient.  Where dP - delta cancels (a single visible key: dS is exactly 0), what is
+        # left is the rounding of dP's own terms: 256 products of N(0, 1) entries, 2^-17 * 16 = 1.2e-4,
+        # weighted by P (sums to 1), by |K|, |Q| <= 5 and by the scale 1/16: 4e-5.
+        scale = y.abs().max().item()
+        assert (x - y).abs().max().item() <= 3e-5 * scale + 4e-5, (name, (x - y).abs().max().item(), scale)
+    assert _capi.kernel_status() == 0
