@@ -306,6 +306,20 @@ attn_fwd_wide(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar->p_full[j & 1]);
     }
+    // The gate of the eight channels this thread will write of each of sixteen rows, requested while the
+    // last product runs and kept in shared memory behind the staging tile, so that the store loop
+    // below is a loop: unrolled, its 128 sigmoids are code that runs once and is fetched cold (13 us
+    // per CTA), and with the loads inside, every row waits for its own.
+    const int t256 = threadIdx.x - 128, c8 = t256 & 31;   // row t256 / 32 + 8 u, channels 8 c8 ..
+    uint4 gates[16];
+    if (p.gate) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int r = min(q_tile * kRows + (t256 >> 5) + 8 * u, p.seq - 1);
+        gates[u] = *reinterpret_cast<const uint4*>(p.gate + (static_cast<size_t>(batch) * p.seq + r) * p.gate_token +
+                                                   head * p.gate_head + c8 * 8);
+      }
+    }
     ok = ok && mbar_wait(&bar->pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, p.status, 108);
     // l of the whole row; the rows then leave through shared memory (Q and the first slots are free
     // by now), coalesced, with the gate applied on the way
@@ -313,8 +327,13 @@ attn_fwd_wide(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     sts_f32(own + g * kRows * 4, l);
     named_barrier_sync(1, 256);
     l += lds_f32(own + (g ^ 1) * kRows * 4);
-    const uint32_t stage = smem_u32(smem);
+    const uint32_t stage = smem_u32(smem), own_gate = stage + 2 * kTileBytes + t256 * 16;
+    static_assert(kTileBytes + kFwdSlots * kSlabBytes >= 3 * kTileBytes, "staging tile and gate");
     if (ok) {
+      if (p.gate) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) sts_b32x4(own_gate + u * 4096, gates[u].x, gates[u].y, gates[u].z, gates[u].w);
+      }
       tc_fence_after();
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
@@ -334,10 +353,9 @@ attn_fwd_wide(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
     named_barrier_sync(1, 256);
     if (ok) {
-      const int t256 = threadIdx.x - 128;
-#pragma unroll 2
-      for (int e = t256; e < kRows * 32; e += 256) {
-        const int r = e >> 5, c8 = e & 31;   // eight channels of a row
+#pragma unroll 1
+      for (int u = 0; u < 16; ++u) {
+        const int r = (t256 >> 5) + 8 * u;
         if (q_tile * kRows + r >= p.seq) continue;
         const size_t token = static_cast<size_t>(batch) * p.seq + q_tile * kRows + r;
         const size_t at = token * p.out_token + head * p.out_head + c8 * 8;
@@ -349,12 +367,12 @@ attn_fwd_wide(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           *reinterpret_cast<float4*>(p.core + at + 4) = b;
         }
         if (p.gate) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(p.gate + token * p.gate_token + head * p.gate_head + c8 * 8);
+          const uint4 raw = lds_b32x4(own_gate + u * 4096);   // written by this thread
           const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const float x = (i & 1) ? bf16_hi(w[i / 2]) : bf16_lo(w[i / 2]);
-            float sigmoid = 1.0f / (1.0f + expf(-x));
+            float sigmoid = sigmoid_fast(x);
             if (p.round_gate) {
               sigmoid = bf16_round(sigmoid);
               v[i] = bf16_round(v[i]);

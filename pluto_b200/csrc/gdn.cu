@@ -198,7 +198,7 @@ __global__ void gdn_conv_kernel(const void* input, const float* weight, int in_i
     const float current = rnd(load_any(input, idx, in_is_bf16), round);
     window[width - 1] = current;
     sum = rnd(sum + current * w[width - 1], round);
-    store_any(output, idx, out_is_bf16, rnd(sum / (1.0f + expf(-sum)), round));
+    store_any(output, idx, out_is_bf16, rnd(sum * sigmoid_fast(sum), round));
   }
   for (int tap = 0; tap < width; ++tap)
     state[(static_cast<size_t>(b) * channels + c) * width + tap] = window[tap];
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* _
 #pragma unroll
       for (int tap = 0; tap + 1 < W; ++tap) sum += x[tap][i] * w[i][tap];
       sum = rnd(sum + x[W - 1][i] * w[i][W - 1], round);
-      y[i] = rnd(sum / (1.0f + expf(-sum)), round);
+      y[i] = rnd(sum * sigmoid_fast(sum), round);
     }
     store_four<OUT_BF16>(output, at, y);
   }
@@ -299,7 +299,7 @@ __device__ __forceinline__ float norm_gate(float x, float inverse, float weight,
                                            int final_round) {
   const float normalized = rnd(x * inverse, round);
   const float affine = rnd(normalized * weight, round);
-  return rnd(affine * (gate / (1.0f + expf(-gate))), round && final_round);
+  return rnd(affine * (gate * sigmoid_fast(gate)), round && final_round);
 }
 
 // One warp per row, eight rows per CTA, a lane owning four consecutive channels of every 128.  HBM

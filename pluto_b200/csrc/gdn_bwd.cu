@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) gdn_out_bwd_kernel(const void* __restrict
     for (int i = 0; i < kOutChannels; ++i) {
       const float normalized = rnd(x[i] * inverse, round);
       const float affine = rnd(normalized * w[i], round);
-      const float sigmoid = 1.0f / (1.0f + expf(-gate[i]));
+      const float sigmoid = sigmoid_fast(gate[i]);
       const float dnorm = g[i] * gate[i] * sigmoid;
       dn[i] = dnorm * w[i];
       dot += dn[i] * x[i];
@@ -427,7 +427,7 @@ __device__ __forceinline__ float conv_dpre(const void* input, int in_is_bf16, co
              weight[static_cast<size_t>(c) * width + tap];
   }
   sum = rnd(sum, round);
-  const float sigmoid = 1.0f / (1.0f + expf(-sum));
+  const float sigmoid = sigmoid_fast(sum);
   return dpost[(seq_base + t) * channels + c] * sigmoid * (1.0f + sum * (1.0f - sigmoid));
 }
 
@@ -551,7 +551,7 @@ gdn_conv_bwd_kernel(const void* __restrict__ input, const float* __restrict__ we
 #pragma unroll
           for (int tap = 0; tap < W; ++tap) sum += x[tap][i] * w[tap][i];
           sum = rnd(sum, round);
-          const float sigmoid = 1.0f / (1.0f + expf(-sum));
+          const float sigmoid = sigmoid_fast(sum);
           const float d = (s < tokens ? up[u][i] : 0.0f) * sigmoid * (1.0f + sum * (1.0f - sigmoid));
           dpre[W - 1][i] = d;
           const float own = s < t1 ? d : 0.0f;

@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kMergeThreads) gqa_decode_merge(DecodeArgs a) 
       const size_t g = static_cast<size_t>(b) * a.gate_token + static_cast<size_t>(head) * a.gate_head + d;
       const float x = a.gate_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[g])
                                      : static_cast<const float*>(a.gate)[g];
-      float sigmoid = 1.0f / (1.0f + expf(-x));
+      float sigmoid = sigmoid_fast(x);
       if (a.round) sigmoid = bf16_round(sigmoid);
       value *= sigmoid;
       if (a.round) value = bf16_round(value);

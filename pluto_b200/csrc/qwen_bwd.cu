@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwdArgs a, long long 
     }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const float sigmoid = 1.0f / (1.0f + expf(-g[i]));
+      const float sigmoid = sigmoid_fast(g[i]);
       dc[i] = grad[i] * rnd(sigmoid, a.round);
       dg[i] = grad[i] * rnd(core[i], a.round) * sigmoid * (1.0f - sigmoid);
       part = fmaf(dc[i], core[i], part);
