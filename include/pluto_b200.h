@@ -335,6 +335,22 @@ int pluto_gqa_decode_probs(pluto_stream_t stream, const void* q, int q_dtype,
                            float* probs, size_t probs_batch_stride, size_t probs_head_stride,
                            int batch, int q_heads, int kv_heads, int head_dim);
 
+/* One token of batch-one attention against one contiguous cache, CachedAttentionStep
+ * (src/llm/layers/util/cached_attention_ops.cc:308-353): norm + RoPE of q_gate [Hq,2,D] and
+ * k [Hkv,D], append of k and v at row `position`, attention over position + 1 rows, sigmoid output
+ * gate into out [Hq,D].  Short contexts (position < 1024, head_dim 64/128/256, 16-byte aligned cache
+ * rows) run as one launch and leave the workspace alone; everything else is pluto_qk_prepare +
+ * pluto_gqa_decode with pluto_cached_attention_step_workspace_bytes of 16-byte aligned scratch.
+ * Nothing is read back and no device array of positions is needed.  The cache's position counter
+ * stays with the caller; position >= the cache's page_size (its capacity) is PLUTO_E_EXHAUSTED. */
+size_t pluto_cached_attention_step_workspace_bytes(int q_heads, int kv_heads, int head_dim, int length);
+int pluto_cached_attention_step(pluto_stream_t stream, const void* q_gate, const void* k, const void* v,
+                                int in_dtype, const float* q_norm, const float* k_norm,
+                                const pluto_kv_cache* cache /* host */, int position, void* out,
+                                int out_dtype, void* workspace, size_t workspace_bytes, int q_heads,
+                                int kv_heads, int head_dim, int rotary_dim, float rms_norm_epsilon,
+                                float rope_theta, int round_to_bf16);
+
 /* --------------------------------------------------------------------------------------------
  * Gated delta-net.
  * pluto_gdn_gates: g = exp(-exp(A_log) * softplus(a + dt_bias)), beta = R(sigmoid(b)); the decay
@@ -388,6 +404,19 @@ int pluto_gdn_step(pluto_stream_t stream, const void* q, const void* k, const vo
                    int in_dtype, const float* g, const float* beta, float* state, void* out,
                    int out_dtype, int batch, int key_heads, int value_heads, int key_dim,
                    int value_dim, int normalize_qk, float q_scale, int round_to_bf16);
+
+/* One token of one sequence through the whole delta-net step, DeltaNetState::Step
+ * (src/llm/layers/util/cached_attention_ops.cc:401-442): convolution + SiLU over qkv [channels],
+ * gates of a, b [Hv], recurrence on state, RMSNorm * weight * SiLU(z) into out [Hv, dv]; conv_state
+ * and state are updated in place.  Widths 128 with at most 4 taps and 8 value heads per key head run
+ * as one launch; other shapes as the four calls above and need the scratch (16-byte aligned). */
+size_t pluto_gdn_token_step_scratch_bytes(int key_heads, int value_heads, int key_dim, int value_dim);
+int pluto_gdn_token_step(pluto_stream_t stream, const void* qkv, int qkv_dtype, const void* z, int z_dtype,
+                         const void* a, const void* b, int ab_dtype, const float* conv_weight,
+                         const float* a_log, const float* dt_bias, const float* norm_weight,
+                         float* conv_state, float* state, void* out, int out_dtype, void* scratch,
+                         size_t scratch_bytes, int key_heads, int value_heads, int key_dim, int value_dim,
+                         int conv_width, float rms_norm_epsilon, int round_to_bf16);
 
 /* Per (token, head) RMSNorm * weight * SiLU(z).  Stands in for DeltaOutputKernel
  * (cached_attention_ops.cc:253-272; final_round = 1) and OutputForward

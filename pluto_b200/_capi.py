@@ -66,6 +66,12 @@ _SIGNATURES = {
                                  + [_i] * 5),
     "pluto_gqa_decode_builtin_scratch_bytes": (_sz, []),
     "pluto_gqa_decode_probs": (_i, [_vp, _vp, _i, _vp, _vp, _vp, _sz, _sz] + [_i] * 4),
+    "pluto_cached_attention_step_workspace_bytes": (_sz, [_i] * 4),
+    "pluto_cached_attention_step": (_i, [_vp] * 4 + [_i] + [_vp] * 3 + [_i, _vp, _i, _vp, _sz] + [_i] * 4
+                                    + [_fp, _fp, _i]),
+    "pluto_gdn_token_step_scratch_bytes": (_sz, [_i] * 4),
+    "pluto_gdn_token_step": (_i, [_vp, _vp, _i, _vp, _i, _vp, _vp, _i] + [_vp] * 7 + [_i, _vp, _sz] + [_i] * 5
+                             + [_fp, _i]),
     "pluto_gdn_gates": (_i, [_vp] * 5 + [_i, C.c_longlong, _i, _i, _vp, _vp]),
     "pluto_gdn_conv_silu": (_i, [_vp] * 3 + [_i] * 6 + [_vp, _vp, _i]),
     "pluto_gdn_prefill": (_i, [_vp] * 4 + [_i] + [_vp] * 4 + [_i] * 7 + [_sz, _sz, _i, _fp, _i, _vp,
@@ -103,6 +109,20 @@ def lib() -> C.CDLL:
             fn.argtypes = argtypes
         _lib = handle
     return _lib
+
+
+_fast = None
+
+
+def fast():
+    """The entry points as vectorcall functions (pluto_b200/host/fastcall.cc): the same names, plain
+    integers for pointers.  The per-call paths use these; `lib()` is the complete ctypes binding."""
+    global _fast
+    if _fast is None:
+        lib()
+        from . import _fastcall   # ImportError if it is not built: there is no fallback path
+        _fast = _fastcall
+    return _fast
 
 
 def exported_symbols():

@@ -9,6 +9,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -58,6 +59,7 @@ def build(verbose: bool = False) -> str:
         if proc.returncode != 0:
             raise RuntimeError(f"link failed:\n{proc.stdout}\n{proc.stderr}")
     build_host()
+    build_fastcall()
     return LIB
 
 
@@ -78,6 +80,24 @@ def build_host() -> str:
     if proc.returncode != 0:
         raise RuntimeError(f"host adapter build failed:\n{proc.stdout}\n{proc.stderr}")
     return HOST_LIB
+
+
+FASTCALL = os.path.join(HERE, "_fastcall.so")
+
+
+def build_fastcall() -> str:
+    """CPython binding of the C ABI (pluto_b200/host/fastcall.cc), imported as pluto_b200._fastcall."""
+    src = os.path.join(HERE, "host", "fastcall.cc")
+    deps = [src, LIB, os.path.join(HERE, "..", "include", "pluto_b200.h")]
+    if os.path.exists(FASTCALL) and os.path.getmtime(FASTCALL) > max(os.path.getmtime(p) for p in deps):
+        return FASTCALL
+    cxx = os.environ.get("CXX", "g++")
+    proc = subprocess.run([cxx, "-std=c++17", "-O2", "-fPIC", "-shared", src,
+                           "-I" + sysconfig.get_paths()["include"], "-L" + HERE, "-lpluto_b200",
+                           "-Wl,-rpath,$ORIGIN", "-o", FASTCALL], capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"CPython binding build failed:\n{proc.stdout}\n{proc.stderr}")
+    return FASTCALL
 
 
 if __name__ == "__main__":

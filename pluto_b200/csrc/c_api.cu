@@ -367,12 +367,13 @@ int decode_split_tokens(int batch, int kv_heads, int max_seq_len) {
 
 int fill_decode(pluto::DecodeArgs* a, const void* q, int q_dtype, const pluto_kv_cache* cache,
                 const int32_t* seq_lens, int max_seq_len, int batch, int q_heads, int kv_heads,
-                int head_dim) {
+                int head_dim, int one_length = 0) {
   if (batch <= 0 || q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || head_dim <= 0 ||
       head_dim > 256 || max_seq_len <= 0 || batch > 65535 || q_heads > 65535 || !dtype_ok(q_dtype))
     return fail(PLUTO_E_INVALID, "invalid full-attention dimensions or parameters");
   if (int c = check_cache(cache, kv_heads, head_dim)) return c;
-  if (!q || !seq_lens) return fail(PLUTO_E_INVALID, "attention requires non-null device pointers");
+  if (!q || (!seq_lens && one_length <= 0))
+    return fail(PLUTO_E_INVALID, "attention requires non-null device pointers");
   *a = pluto::DecodeArgs{};
   a->q = q;
   a->q_is_bf16 = q_dtype == PLUTO_BF16;
@@ -388,6 +389,7 @@ int fill_decode(pluto::DecodeArgs* a, const void* q, int q_dtype, const pluto_kv
   a->token_stride = cache->token_stride;
   a->num_pages = cache->num_pages;
   a->seq_lens = seq_lens;
+  a->one_length = one_length;
   a->batch = batch; a->q_heads = q_heads; a->kv_heads = kv_heads; a->head_dim = head_dim;
   a->split_tokens = decode_split_tokens(batch, kv_heads, max_seq_len);
   a->splits = pluto::decode_chunk_count(max_seq_len, a->split_tokens);
@@ -475,6 +477,71 @@ int pluto_gqa_decode(pluto_stream_t stream, const void* q, int q_dtype, const vo
   // only address here whose alignment does not depend on head_dim (odd widths are legal).
   a.partial_ml = static_cast<float*>(workspace);
   a.partial_acc = a.partial_ml + pluto::decode_ml_floats(batch, q_heads, a.splits);
+  return from_cuda(pluto::gqa_decode(stream, a), "Qwen full attention");
+}
+
+size_t pluto_cached_attention_step_workspace_bytes(int q_heads, int kv_heads, int head_dim, int length) {
+  if (q_heads <= 0 || kv_heads <= 0 || head_dim <= 0 || length <= 0) return 0;
+  const size_t queries = (static_cast<size_t>(q_heads) * head_dim * sizeof(float) + 255) / 256 * 256;
+  return queries + pluto_gqa_decode_workspace_bytes(1, q_heads, kv_heads, head_dim, length);
+}
+
+int pluto_cached_attention_step(pluto_stream_t stream, const void* q_gate, const void* k, const void* v,
+                                int in_dtype, const float* q_norm, const float* k_norm,
+                                const pluto_kv_cache* cache, int position, void* out, int out_dtype,
+                                void* workspace, size_t workspace_bytes, int q_heads, int kv_heads,
+                                int head_dim, int rotary_dim, float rms_norm_epsilon, float rope_theta,
+                                int round_to_bf16) {
+  if (q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads != 0 || head_dim <= 0 || head_dim > 256 ||
+      q_heads > 65535 || rotary_dim <= 0 || rotary_dim > head_dim || rotary_dim % 2 != 0 ||
+      !isfinite(rope_theta) || rope_theta <= 0.0f || !isfinite(rms_norm_epsilon) || rms_norm_epsilon <= 0.0f ||
+      !dtype_ok(in_dtype) || !dtype_ok(out_dtype))
+    return fail(PLUTO_E_INVALID, "invalid full-attention dimensions or parameters");
+  if (int c = check_cache(cache, kv_heads, head_dim)) return c;
+  if (cache->block_table || cache->k_bases)
+    return fail(PLUTO_E_INVALID, "a cached attention step takes one contiguous cache");
+  if (!q_gate || !k || !v || !q_norm || !k_norm || !out)
+    return fail(PLUTO_E_INVALID, "attention requires non-null device pointers");
+  if (position < 0) return fail(PLUTO_E_INVALID, "invalid full-attention dimensions or parameters");
+  if (position >= cache->page_size) return fail(PLUTO_E_EXHAUSTED, "full-attention cache capacity reached");
+  pluto::CachedStepArgs s{};
+  s.q_gate = q_gate; s.k = k; s.v = v; s.in_is_bf16 = in_dtype == PLUTO_BF16;
+  s.q_norm = q_norm; s.k_norm = k_norm;
+  s.k_cache = cache->k_base; s.v_cache = cache->v_base; s.kv_is_bf16 = cache->dtype == PLUTO_BF16;
+  s.token_stride = cache->token_stride;
+  s.out = out; s.out_is_bf16 = out_dtype == PLUTO_BF16;
+  s.position = position; s.q_heads = q_heads; s.kv_heads = kv_heads; s.head_dim = head_dim; s.rotary = rotary_dim;
+  s.epsilon = rms_norm_epsilon; s.log_theta = logf(rope_theta);
+  s.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
+  s.round = round_to_bf16;
+  if (pluto::cached_step_supported(s))
+    return from_cuda(pluto::cached_step(stream, s), "Qwen cached attention step");
+  // longer contexts and other widths: prepare, split decode, merge
+  const size_t need = pluto_cached_attention_step_workspace_bytes(q_heads, kv_heads, head_dim, position + 1);
+  if (!workspace || workspace_bytes < need || !aligned16(workspace))
+    return fail(PLUTO_E_INVALID, "attention decode workspace is too small or misaligned");
+  const size_t queries = (static_cast<size_t>(q_heads) * head_dim * sizeof(float) + 255) / 256 * 256;
+  const int q_dtype = round_to_bf16 ? PLUTO_BF16 : PLUTO_FP32;
+  pluto::DecodeArgs a;
+  if (int c = fill_decode(&a, workspace, q_dtype, cache, nullptr, position + 1, 1, q_heads, kv_heads, head_dim,
+                          position + 1))
+    return c;
+  pluto::PrepareArgs p{};
+  p.q_in = q_gate; p.k_in = k; p.v_in = v; p.in_is_bf16 = s.in_is_bf16;
+  p.q_token = 2 * static_cast<size_t>(q_heads) * head_dim; p.q_head = 2 * static_cast<size_t>(head_dim);
+  p.q_norm = q_norm; p.k_norm = k_norm; p.first_position = position;
+  p.q_out = workspace; p.q_out_is_bf16 = round_to_bf16;
+  p.k_cache = cache->k_base; p.v_cache = cache->v_base; p.kv_is_bf16 = s.kv_is_bf16;
+  p.page_size = cache->page_size; p.page_stride = cache->page_stride; p.token_stride = cache->token_stride;
+  p.batch = 1; p.tokens = 1; p.q_heads = q_heads; p.kv_heads = kv_heads; p.head_dim = head_dim; p.rotary = rotary_dim;
+  p.epsilon = rms_norm_epsilon; p.log_theta = s.log_theta; p.round = round_to_bf16;
+  if (int c = from_cuda(pluto::qk_prepare(stream, p), "prepare Qwen attention")) return c;
+  a.gate = static_cast<const char*>(q_gate) + static_cast<size_t>(head_dim) * (in_dtype == PLUTO_BF16 ? 2 : 4);
+  a.gate_is_bf16 = s.in_is_bf16; a.gate_token = p.q_token; a.gate_head = p.q_head;
+  a.out = out; a.out_is_bf16 = s.out_is_bf16;
+  a.round = round_to_bf16;
+  a.partial_ml = reinterpret_cast<float*>(static_cast<char*>(workspace) + queries);
+  a.partial_acc = a.partial_ml + pluto::decode_ml_floats(1, q_heads, a.splits);
   return from_cuda(pluto::gqa_decode(stream, a), "Qwen full attention");
 }
 
@@ -572,6 +639,53 @@ int pluto_gdn_step(pluto_stream_t stream, const void* q, const void* k, const vo
   return pluto_gdn_prefill(stream, q, k, v, in_dtype, g, beta, state, out, out_dtype, batch, 1,
                            key_heads, value_heads, key_dim, value_dim, 0, 0, normalize_qk, q_scale,
                            round_to_bf16, nullptr, 0);
+}
+
+size_t pluto_gdn_token_step_scratch_bytes(int key_heads, int value_heads, int key_dim, int value_dim) {
+  if (key_heads <= 0 || value_heads <= 0 || key_dim <= 0 || value_dim <= 0) return 0;
+  return (2 * static_cast<size_t>(key_heads) * key_dim + 2 * static_cast<size_t>(value_heads) * value_dim +
+          2 * static_cast<size_t>(value_heads)) * sizeof(float);
+}
+
+int pluto_gdn_token_step(pluto_stream_t stream, const void* qkv, int qkv_dtype, const void* z, int z_dtype,
+                         const void* a, const void* b, int ab_dtype, const float* conv_weight,
+                         const float* a_log, const float* dt_bias, const float* norm_weight,
+                         float* conv_state, float* state, void* out, int out_dtype, void* scratch,
+                         size_t scratch_bytes, int key_heads, int value_heads, int key_dim, int value_dim,
+                         int conv_width, float rms_norm_epsilon, int round_to_bf16) {
+  if (int c = check_gdn(1, 1, key_heads, value_heads, key_dim, value_dim)) return c;
+  if (conv_width <= 0 || conv_width > 32 || !dtype_ok(qkv_dtype) || !dtype_ok(z_dtype) || !dtype_ok(ab_dtype) ||
+      !dtype_ok(out_dtype) || !isfinite(rms_norm_epsilon) || rms_norm_epsilon <= 0.0f)
+    return fail(PLUTO_E_INVALID, "invalid DeltaNet dimensions or parameters");
+  if (!qkv || !z || !a || !b || !conv_weight || !a_log || !dt_bias || !norm_weight || !conv_state || !state || !out)
+    return fail(PLUTO_E_INVALID, "DeltaNet requires non-null device pointers");
+  if (pluto::gdn_token_supported(key_heads, value_heads, key_dim, value_dim, conv_width) && aligned16(state)) {
+    pluto::GdnTokenArgs t{};
+    t.qkv = qkv; t.z = z; t.a_in = a; t.b_in = b;
+    t.qkv_is_bf16 = qkv_dtype == PLUTO_BF16; t.z_is_bf16 = z_dtype == PLUTO_BF16; t.ab_is_bf16 = ab_dtype == PLUTO_BF16;
+    t.conv_weight = conv_weight; t.a_log = a_log; t.dt_bias = dt_bias; t.norm_weight = norm_weight;
+    t.conv_state = conv_state; t.state = state; t.out = out; t.out_is_bf16 = out_dtype == PLUTO_BF16;
+    t.key_heads = key_heads; t.value_heads = value_heads; t.width = conv_width;
+    t.epsilon = rms_norm_epsilon; t.round = round_to_bf16;
+    return from_cuda(pluto::gdn_token(stream, t), "Qwen gated delta token step");
+  }
+  if (!scratch || scratch_bytes < pluto_gdn_token_step_scratch_bytes(key_heads, value_heads, key_dim, value_dim) ||
+      !aligned16(scratch))
+    return fail(PLUTO_E_INVALID, "DeltaNet step scratch is too small or misaligned");
+  const int kq = key_heads * key_dim, channels = 2 * kq + value_heads * value_dim;
+  float* convolved = static_cast<float*>(scratch);
+  float* core = convolved + channels;
+  float* g = core + static_cast<size_t>(value_heads) * value_dim;
+  float* beta = g + value_heads;
+  if (int c = pluto_gdn_conv_silu(stream, qkv, conv_weight, qkv_dtype, 1, 1, channels, conv_width, round_to_bf16,
+                                  conv_state, convolved, PLUTO_FP32))
+    return c;
+  if (int c = pluto_gdn_gates(stream, a, b, a_log, dt_bias, ab_dtype, 1, value_heads, round_to_bf16, g, beta)) return c;
+  if (int c = pluto_gdn_step(stream, convolved, convolved + kq, convolved + 2 * kq, PLUTO_FP32, g, beta, state, core,
+                             PLUTO_FP32, 1, key_heads, value_heads, key_dim, value_dim, 1, 1.0f, round_to_bf16))
+    return c;
+  return pluto_gdn_out_norm_gate(stream, core, PLUTO_FP32, z, z_dtype, norm_weight, value_heads, value_dim,
+                                 rms_norm_epsilon, round_to_bf16, 1, out, out_dtype);
 }
 
 int pluto_gdn_out_norm_gate(pluto_stream_t stream, const void* core, int core_dtype, const void* z,

@@ -150,6 +150,8 @@ __device__ __forceinline__ void sts_b32x4(uint32_t addr, uint32_t x, uint32_t y,
 
 // Barrier over all threads of the cluster, and a read of a peer CTA's shared memory: `addr` is this
 // CTA's address of the same variable.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -159,7 +159,8 @@ struct DecodeArgs {
   size_t page_stride, token_stride;
   int num_pages;            // pages in the pool (needed for the TMA map when a block table is used)
   int box_rows;             // filled by gqa_decode: tokens per TMA box
-  const int32_t* seq_lens;  // [batch], number of cached tokens to attend to (>= 1)
+  const int32_t* seq_lens;  // [batch], number of cached tokens to attend to (>= 1), or null: one_length
+  int one_length;
   void* out;                // [batch, q_heads, head_dim]
   int out_is_bf16;
   float* lse;               // optional [batch, q_heads]
@@ -211,7 +212,8 @@ struct PrepareArgs {
   size_t q_token, q_head;
   const float* q_norm;      // [head_dim], zero-centred
   const float* k_norm;
-  const int32_t* positions; // optional [batch]: position of token 0 of each sequence
+  const int32_t* positions; // optional [batch]: position of token 0 of each sequence, null: first_position
+  int first_position;
   void* q_out;              // [batch*tokens, q_heads, head_dim]
   int q_out_is_bf16;
   void* k_cache;            // cache addressing as in DecodeArgs
@@ -227,6 +229,37 @@ struct PrepareArgs {
   int round;
 };
 cudaError_t qk_prepare(cudaStream_t stream, const PrepareArgs& args);
+
+// ---- token_step.cu: one token of one sequence in one launch ----------------------------------------
+constexpr int kCachedStepTokens = 1024;   // longest context cached_step takes
+struct CachedStepArgs {
+  const void *q_gate, *k, *v;   // [q_heads, 2, D], [kv_heads, D] x 2
+  int in_is_bf16;
+  const float *q_norm, *k_norm;
+  void *k_cache, *v_cache;      // [capacity, kv_heads, D], token_stride elements between tokens
+  int kv_is_bf16;
+  size_t token_stride;
+  void* out;                    // [q_heads, D]
+  int out_is_bf16;
+  int position, q_heads, kv_heads, head_dim, rotary;
+  float epsilon, log_theta, scale;
+  int round;
+};
+bool cached_step_supported(const CachedStepArgs& args);
+cudaError_t cached_step(cudaStream_t stream, const CachedStepArgs& args);
+struct GdnTokenArgs {
+  const void *qkv, *z, *a_in, *b_in;   // [channels], [value_heads, dv], [value_heads] x 2
+  int qkv_is_bf16, z_is_bf16, ab_is_bf16;
+  const float *conv_weight, *a_log, *dt_bias, *norm_weight;
+  float *conv_state, *state;           // [channels, width], [value_heads, dk, dv], updated in place
+  void* out;
+  int out_is_bf16;
+  int key_heads, value_heads, width;
+  float epsilon;
+  int round;
+};
+bool gdn_token_supported(int key_heads, int value_heads, int key_dim, int value_dim, int width);
+cudaError_t gdn_token(cudaStream_t stream, const GdnTokenArgs& args);
 
 // ---- gdn.cu -------------------------------------------------------------------------------------
 struct GdnArgs {

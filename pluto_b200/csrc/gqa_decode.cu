@@ -35,7 +35,7 @@ constexpr int kDecodeThreads = (kConsumerWarps + 1) * 32;
 // grid and the workspace for, [0, decode_chunk_capacity(splits, split_tokens)].  A value outside is a caller error; it
 // is reported through the status word and the launch stays inside its buffers.
 __device__ __forceinline__ int bounded_length(const DecodeArgs& a, int b, uint32_t site) {
-  const int length = a.seq_lens[b];
+  const int length = a.seq_lens ? a.seq_lens[b] : a.one_length;
   const long long limit = decode_chunk_capacity(a.splits, a.split_tokens);
   if (length < 0 || length > limit) {
     report_status(a.status, site, kBadLength);
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kMergeThreads) gqa_decode_merge(DecodeArgs a) 
       const size_t g = static_cast<size_t>(b) * a.gate_token + static_cast<size_t>(head) * a.gate_head + d;
       const float x = a.gate_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[g])
                                      : static_cast<const float*>(a.gate)[g];
-      float sigmoid = sigmoid_fast(x);
+      float sigmoid = 1.0f / (1.0f + expf(-x));
       if (a.round) sigmoid = bf16_round(sigmoid);
       value *= sigmoid;
       if (a.round) value = bf16_round(value);

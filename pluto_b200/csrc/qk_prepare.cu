@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(PrepareArgs a) {
   const int token = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int b = token / a.tokens, t = token % a.tokens;
   const int D = a.head_dim, half = a.rotary / 2;
-  const int position = (a.positions ? a.positions[b] : 0) + t;
+  const int position = (a.positions ? a.positions[b] : a.first_position) + t;
   if (static_cast<int>(threadIdx.x) < half) {
     const float angle = static_cast<float>(position) *
                         expf(static_cast<float>(threadIdx.x) * (-2.0f * a.log_theta / static_cast<float>(a.rotary)));

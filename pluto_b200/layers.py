@@ -73,8 +73,14 @@ def _invalid(message: str) -> PlutoStatusError:
     return PlutoStatusError("InvalidArgument", message, -1)
 
 
+# The current stream of the current device as a raw handle: 0.1 us, where building the Stream object
+# that torch.cuda.current_stream() returns takes 3.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -211,10 +217,10 @@ class AttentionLayer(Layer):
             raise _invalid("attention rows must be divisible by context_length")
         inspect = hooks is not None and hooks.attention_probabilities_hook is not None
         dtype = activation_torch_dtype(self.output_type_)
-        out = torch.empty((rows, E), dtype=dtype, device=qkv.device)
+        out = qkv.new_empty((rows, E)) if qkv.dtype == dtype else torch.empty((rows, E), dtype=dtype, device=qkv.device)
         maxima = torch.empty((rows * H,), dtype=torch.float32, device=qkv.device)
         normalizers = torch.empty_like(maxima)
-        L = _capi.lib()
+        L = _capi.fast()
         check(L.pluto_attn_fwd(_stream(), _ptr(qkv), _ptr(out), _ptr(maxima), _ptr(normalizers),
                                rows // S, S, H, E // H, self._dtype_code()))
         if inspect:
@@ -243,7 +249,7 @@ class AttentionLayer(Layer):
         _validate_buffer(normalizers, rows * H * 4, "attention saved normalizers")
         d_qkv = torch.empty((rows, 3 * E), dtype=torch.float32, device=d_out.device)
         deltas = torch.empty((rows * H,), dtype=torch.float32, device=d_out.device)
-        L = _capi.lib()
+        L = _capi.fast()
         ws_ptr, ws_bytes = None, 0
         need = L.pluto_attn_bwd_workspace_bytes(rows // S, S, H, E // H, self._dtype_code())
         if need and self.tensor_core_backward:
@@ -282,7 +288,7 @@ def gqa_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     # a few heads of a long prompt cannot load the SMs evenly with whole query tiles: the kernel
     # then cuts the longest tile pairs along their keys and needs scratch for the partial results
     # (the query returns 0 for shapes it would not cut); pass `workspace` to reuse one across calls
-    L = _capi.lib()
+    L = _capi.fast()
     ws_ptr, ws_bytes = None, 0
     if D in (64, 128):
         ws_bytes = L.pluto_gqa_prefill_fwd_workspace_bytes(B, T, Hq, D)
@@ -365,6 +371,7 @@ class KeyValueCache:
         self.keys_ = torch.zeros((capacity, key_value_heads, head_dim), dtype=dtype, device=device)
         self.values_ = torch.zeros_like(self.keys_)
         self.position_ = 0
+        self.packed_ = None
 
     @staticmethod
     def Create(capacity: int, key_value_heads: int, head_dim: int,
@@ -391,6 +398,13 @@ class KeyValueCache:
     def Reset(self) -> None:
         self.position_ = 0  # contents are not cleared, as in the reference
 
+    def packed_layout(self) -> bytes:
+        """struct pluto_kv_cache of this cache, for the vectorcall binding; the buffers never move."""
+        if self.packed_ is None:
+            row = self.key_value_heads_ * self.head_dim_
+            self.packed_ = _pack_cache(self.keys_, self.values_, None, self.capacity_, self.capacity_ * row, row)
+        return self.packed_
+
     def layout(self) -> "_capi.KvCacheStruct":
         return kv_layout(self.keys_, self.values_, None, self.capacity_,
                          self.capacity_ * self.key_value_heads_ * self.head_dim_,
@@ -407,6 +421,15 @@ def kv_layout(k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: Optional[
     s.dtype = 1 if k_pool.dtype == torch.bfloat16 else 0
     s.num_pages = k_pool.shape[0] if k_pool.dim() == 4 else 1
     return s
+
+
+def _pack_cache(k_pool, v_pool, block_table, page_size, page_stride, token_stride) -> bytes:
+    """kv_layout as the bytes the vectorcall binding takes."""
+    return _capi.fast().kv_cache(k_pool.data_ptr(), v_pool.data_ptr(),
+                                 None if block_table is None else block_table.data_ptr(),
+                                 0 if block_table is None else block_table.shape[1], page_size, page_stride,
+                                 token_stride, 1 if k_pool.dtype == torch.bfloat16 else 0,
+                                 k_pool.shape[0] if k_pool.dim() == 4 else 1)
 
 
 def gqa_decode_separate_caches(q: torch.Tensor, caches, seq_lens: torch.Tensor, *,
@@ -431,12 +454,12 @@ def gqa_decode_separate_caches(q: torch.Tensor, caches, seq_lens: torch.Tensor, 
     layout.dtype = 1 if first.keys().dtype == torch.bfloat16 else 0
     layout.num_pages = 0
     layout.k_bases, layout.v_bases = k_bases.data_ptr(), v_bases.data_ptr()
-    L = _capi.lib()
+    L = _capi.fast()
     out = torch.empty_like(q)
     nbytes = L.pluto_gqa_decode_workspace_bytes(B, Hq, Hkv, D, capacity)
     ws = _workspace(q.device, nbytes)
     lse = torch.empty((B, Hq), dtype=torch.float32, device=q.device) if want_lse else None
-    check(L.pluto_gqa_decode(_stream(), _ptr(q), _dt(q), None, 0, 0, 0, C_byref(layout), _ptr(seq_lens),
+    check(L.pluto_gqa_decode(_stream(), _ptr(q), _dt(q), None, 0, 0, 0, bytes(layout), _ptr(seq_lens),
                              capacity, _ptr(out), _dt(out), _ptr(lse), _ptr(ws), ws.numel(), B, Hq, Hkv, D,
                              int(round_to_bfloat16)))
     return (out, lse) if want_lse else out
@@ -471,7 +494,7 @@ _decode_workspaces = {}
 
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
-    key = (str(device), torch.cuda.current_stream().cuda_stream)
+    key = (device.index, _stream())
     ws = _decode_workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.empty((max(nbytes, 1 << 20),), dtype=torch.uint8, device=device)
@@ -494,31 +517,45 @@ def CachedAttentionStep(p: FullAttentionParameters, cache: KeyValueCache, q_gate
             raise _invalid("attention requires non-null device pointers")
     if cache.position() >= cache.capacity():
         raise _resource_exhausted("full-attention cache capacity reached")
-    L = _capi.lib()
-    device = output.device
-    position = cache.position()
+    _cached_step(p, cache, q_gate, k, v, q_norm, k_norm, output)
+    if probabilities is not None:
+        _cached_probabilities(p, cache, q_gate, k, v, q_norm, k_norm, probabilities)
+    cache.Advance()
+
+
+_ONE_LAUNCH_TOKENS = 1024   # contexts that pluto_cached_attention_step attends to without scratch
+
+
+def _cached_step(p, cache, q_gate, k, v, q_norm, k_norm, output) -> None:
+    """The launches of CachedAttentionStep at the cache's position, which stays where it is."""
+    L = _capi.fast()
+    position, ws, ws_bytes = cache.position_, None, 0
+    if position >= _ONE_LAUNCH_TOKENS or p.head_dim not in (64, 128, 256):
+        ws = _workspace(output.device, L.pluto_cached_attention_step_workspace_bytes(
+            p.query_heads, p.key_value_heads, p.head_dim, position + 1))
+        ws, ws_bytes = ws.data_ptr(), ws.numel()
+    check(L.pluto_cached_attention_step(
+        _stream(), q_gate.data_ptr(), k.data_ptr(), v.data_ptr(), _dt(q_gate), q_norm.data_ptr(), k_norm.data_ptr(),
+        cache.packed_layout(), position, output.data_ptr(), _dt(output), ws, ws_bytes, p.query_heads,
+        p.key_value_heads, p.head_dim, p.rotary_dim, p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16)))
+
+
+def _cached_probabilities(p, cache, q_gate, k, v, q_norm, k_norm, probabilities) -> None:
+    """The softmax row of the token the step just attended with, for the inspection hook: the query is
+    prepared once more (which rewrites the token's cache row with the same values)."""
+    L = _capi.fast()
+    device, position = probabilities.device, cache.position_
     D, Hq, Hkv = p.head_dim, p.query_heads, p.key_value_heads
     queries = torch.empty((Hq, D), dtype=torch.bfloat16 if p.round_to_bfloat16 else torch.float32,
                           device=device)
     positions = torch.tensor([position], dtype=torch.int32, device=device)
-    layout = cache.layout()
     check(L.pluto_qk_prepare(_stream(), _ptr(q_gate), _ptr(k), _ptr(v), _dt(q_gate), 2 * Hq * D,
                              2 * D, _ptr(q_norm), _ptr(k_norm), _ptr(positions), _ptr(queries),
-                             _dt(queries), C_byref(layout), 1, 1, Hq, Hkv, D, p.rotary_dim,
+                             _dt(queries), cache.packed_layout(), 1, 1, Hq, Hkv, D, p.rotary_dim,
                              p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16)))
     lens = positions + 1
-    nbytes = L.pluto_gqa_decode_workspace_bytes(1, Hq, Hkv, D, position + 1)
-    ws = _workspace(device, nbytes)
-    gate = q_gate.reshape(-1)[D:]
-    check(L.pluto_gqa_decode(_stream(), _ptr(queries), _dt(queries), _ptr(gate), _dt(q_gate),
-                             2 * Hq * D, 2 * D, C_byref(layout), _ptr(lens), position + 1,
-                             _ptr(output), _dt(output), None, _ptr(ws), ws.numel(), 1, Hq, Hkv, D,
-                             int(p.round_to_bfloat16)))
-    if probabilities is not None:
-        check(L.pluto_gqa_decode_probs(_stream(), _ptr(queries), _dt(queries), C_byref(layout),
-                                       _ptr(lens), _ptr(probabilities), 0, position + 1, 1, Hq, Hkv,
-                                       D))
-    cache.Advance()
+    check(L.pluto_gqa_decode_probs(_stream(), _ptr(queries), _dt(queries), cache.packed_layout(),
+                                   _ptr(lens), _ptr(probabilities), 0, position + 1, 1, Hq, Hkv, D))
 
 
 def C_byref(struct):
@@ -537,8 +574,8 @@ def gqa_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, seq_
     B, Hq, D = q.shape
     pages, psize, Hkv, _ = k_pool.shape
     page_size = psize if page_size is None else page_size
-    layout = kv_layout(k_pool, v_pool, block_table, page_size, k_pool.stride(0), k_pool.stride(1))
-    L = _capi.lib()
+    layout = _pack_cache(k_pool, v_pool, block_table, page_size, k_pool.stride(0), k_pool.stride(1))
+    L = _capi.fast()
     if out is None:
         out = torch.empty_like(q)
     nbytes = L.pluto_gqa_decode_workspace_bytes(B, Hq, Hkv, D, max_seq_len)
@@ -548,7 +585,7 @@ def gqa_decode(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, seq_
     if gate is not None:
         gts, ghs = gate.stride(0), gate.stride(1)
     check(L.pluto_gqa_decode(_stream(), _ptr(q), _dt(q), _ptr(gate),
-                             _dt(gate) if gate is not None else 0, gts, ghs, C_byref(layout),
+                             _dt(gate) if gate is not None else 0, gts, ghs, layout,
                              _ptr(seq_lens), max_seq_len, _ptr(out), _dt(out), _ptr(lse), _ptr(ws),
                              ws.numel(), B, Hq, Hkv, D, int(round_to_bfloat16)))
     return (out, lse) if want_lse else out
@@ -580,10 +617,9 @@ class DeltaNetState:
         self.convolution_state_ = torch.empty((1, self.channels_, p.conv_kernel_dim), **f32)
         self.recurrent_state_ = torch.empty((1, p.value_heads, p.key_head_dim, p.value_head_dim),
                                             **f32)
-        self.convolved_qkv_ = torch.empty((self.channels_,), **f32)
-        self.core_output_ = torch.empty((p.value_heads, p.value_head_dim), **f32)
-        self.g_ = torch.empty((p.value_heads,), **f32)
-        self.beta_ = torch.empty((p.value_heads,), **f32)
+        # convolved channels, gates and core output of the shapes that take four launches per step
+        self.scratch_ = torch.empty((_capi.fast().pluto_gdn_token_step_scratch_bytes(
+            p.key_heads, p.value_heads, p.key_head_dim, p.value_head_dim) // 4,), **f32)
 
     @staticmethod
     def Create(p: DeltaNetParameters, device="cuda") -> "DeltaNetState":
@@ -608,22 +644,14 @@ class DeltaNetState:
         for t in (qkv, z, a, b, conv_weight, a_log, dt_bias, norm_weight, output):
             if t is None:
                 raise _invalid("DeltaNet requires non-null device pointers")
-        p, L, rnd = self.parameters_, _capi.lib(), int(self.parameters_.round_to_bfloat16)
-        check(L.pluto_gdn_conv_silu(_stream(), _ptr(qkv), _ptr(conv_weight), _dt(qkv), 1, 1,
-                                    self.channels_, p.conv_kernel_dim, rnd,
-                                    _ptr(self.convolution_state_), _ptr(self.convolved_qkv_), 0))
-        check(L.pluto_gdn_gates(_stream(), _ptr(a), _ptr(b), _ptr(a_log), _ptr(dt_bias), _dt(a), 1,
-                                p.value_heads, rnd, _ptr(self.g_), _ptr(self.beta_)))
-        kq = p.key_heads * p.key_head_dim
-        conv = self.convolved_qkv_
-        check(L.pluto_gdn_step(_stream(), _ptr(conv[:kq]), _ptr(conv[kq:2 * kq]),
-                               _ptr(conv[2 * kq:]), 0, _ptr(self.g_), _ptr(self.beta_),
-                               _ptr(self.recurrent_state_), _ptr(self.core_output_), 0, 1,
-                               p.key_heads, p.value_heads, p.key_head_dim, p.value_head_dim, 1,
-                               1.0, rnd))
-        check(L.pluto_gdn_out_norm_gate(_stream(), _ptr(self.core_output_), 0, _ptr(z), _dt(z),
-                                        _ptr(norm_weight), p.value_heads, p.value_head_dim,
-                                        p.rms_norm_epsilon, rnd, 1, _ptr(output), _dt(output)))
+        p = self.parameters_
+        scratch = self.scratch_
+        check(_capi.fast().pluto_gdn_token_step(
+            _stream(), qkv.data_ptr(), _dt(qkv), z.data_ptr(), _dt(z), a.data_ptr(), b.data_ptr(), _dt(a),
+            conv_weight.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), norm_weight.data_ptr(),
+            self.convolution_state_.data_ptr(), self.recurrent_state_.data_ptr(), output.data_ptr(), _dt(output),
+            scratch.data_ptr(), 4 * scratch.numel(), p.key_heads, p.value_heads, p.key_head_dim, p.value_head_dim,
+            p.conv_kernel_dim, p.rms_norm_epsilon, int(p.round_to_bfloat16)))
 
 
 def gdn_prefill(q, k, v, g, beta, state, normalize_qk=True, q_scale=1.0, round_to_bfloat16=True,
@@ -637,7 +665,7 @@ def gdn_prefill(q, k, v, g, beta, state, normalize_qk=True, q_scale=1.0, round_t
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     if out is None:
         out = torch.empty_like(v)
-    L = _capi.lib()
+    L = _capi.fast()
     ws_ptr, ws_bytes = None, 0
     if chunked is None or chunked:
         need = L.pluto_gdn_prefill_workspace_bytes(B, T, Hk, Hv, dk, dv, _dt(v))
@@ -661,7 +689,7 @@ def gdn_step(q, k, v, g, beta, state, normalize_qk=True, q_scale=1.0, round_to_b
     Hv, dv = v.shape[1], v.shape[2]
     if out is None:
         out = torch.empty_like(v)
-    check(_capi.lib().pluto_gdn_step(_stream(), _ptr(q), _ptr(k), _ptr(v), _dt(v), _ptr(g),
+    check(_capi.fast().pluto_gdn_step(_stream(), _ptr(q), _ptr(k), _ptr(v), _dt(v), _ptr(g),
                                      _ptr(beta), _ptr(state), _ptr(out), _dt(out), B, Hk, Hv, dk,
                                      dv, int(normalize_qk), float(q_scale), int(round_to_bfloat16)))
     return out
@@ -681,13 +709,13 @@ def gqa_decode_noalloc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
     scratch than the area holds."""
     B, Hq, D = q.shape
     _, psize, Hkv, _ = k_pool.shape
-    layout = kv_layout(k_pool, v_pool, block_table, psize, k_pool.stride(0), k_pool.stride(1))
+    layout = _pack_cache(k_pool, v_pool, block_table, psize, k_pool.stride(0), k_pool.stride(1))
     gts = ghs = 0
     if gate is not None:
         gts, ghs = gate.stride(0), gate.stride(1)
-    check(_capi.lib().pluto_gqa_decode_noalloc(
+    check(_capi.fast().pluto_gqa_decode_noalloc(
         _stream(), _ptr(q), _dt(q), _ptr(gate), _dt(gate) if gate is not None else 0, gts, ghs,
-        C_byref(layout), _ptr(seq_lens), max_seq_len, _ptr(out), _dt(out), _ptr(lse), B, Hq, Hkv, D,
+        layout, _ptr(seq_lens), max_seq_len, _ptr(out), _dt(out), _ptr(lse), B, Hq, Hkv, D,
         int(round_to_bfloat16)))
     return out
 
@@ -798,24 +826,24 @@ class QwenAttentionLayer(Layer):
 
     def _cached_forward(self, inputs, hooks) -> FwdResult:
         # src/llm/layers/qwen_attention.cc:370-412, minus the bf16<->fp32 cast launches
-        p = self.parameters_
+        p, cache = self.parameters_, self.cache_
         width = p.query_heads * p.head_dim
         kv = p.key_value_heads * p.head_dim
-        _validate_bf16_inputs(inputs, [2 * width, kv, kv], "QwenAttentionLayer")
-        if self.cache_.position() >= self.cache_.capacity():
+        _validate_bf16_inputs(inputs, (2 * width, kv, kv), "QwenAttentionLayer")
+        if cache.position_ >= cache.capacity_:
             raise _resource_exhausted("full-attention cache capacity reached")
-        output = torch.empty((1, width), dtype=torch.bfloat16, device=inputs[0].device)
-        length = self.cache_.position() + 1
-        inspect = hooks is not None and hooks.attention_probabilities_hook is not None
-        probabilities = torch.empty((p.query_heads, length), dtype=torch.float32,
-                                    device=inputs[0].device) if inspect else None
-        CachedAttentionStep(p, self.cache_, inputs[0].view(p.query_heads, 2, p.head_dim),
-                            inputs[1].view(p.key_value_heads, p.head_dim),
-                            inputs[2].view(p.key_value_heads, p.head_dim), self.weights_[0],
-                            self.weights_[1], output.view(p.query_heads, p.head_dim), probabilities)
-        if inspect:
-            hooks.attention_probabilities_hook(
-                self.name(), ActivationType(DataType.FP32, (1, p.query_heads, 1, length)), probabilities)
+        inputs = [x if x.is_contiguous() else x.contiguous() for x in inputs]
+        output = inputs[0].new_empty((1, width))
+        if hooks is None or hooks.attention_probabilities_hook is None:
+            _cached_step(p, cache, inputs[0], inputs[1], inputs[2], self.weights_[0], self.weights_[1], output)
+            cache.Advance()
+            return FwdResult([output], BackwardState())
+        length = cache.position_ + 1
+        probabilities = torch.empty((p.query_heads, length), dtype=torch.float32, device=inputs[0].device)
+        CachedAttentionStep(p, cache, inputs[0], inputs[1], inputs[2], self.weights_[0], self.weights_[1], output,
+                            probabilities)
+        hooks.attention_probabilities_hook(
+            self.name(), ActivationType(DataType.FP32, (1, p.query_heads, 1, length)), probabilities)
         return FwdResult([output], BackwardState())
 
     def _sequence_forward(self, inputs, hooks) -> FwdResult:
@@ -825,15 +853,15 @@ class QwenAttentionLayer(Layer):
         _validate_bf16_inputs(inputs, [2 * t * hq * d, t * hkv * d, t * hkv * d], "QwenAttentionLayer")
         if not p.round_to_bfloat16:
             raise _unimplemented("sequence Qwen attention without bf16 rounding is not built")
-        L = _capi.lib()
+        L = _capi.fast()
         device = inputs[0].device
         q = torch.empty((1, t, hq, d), dtype=torch.bfloat16, device=device)
         k = torch.empty((1, t, hkv, d), dtype=torch.bfloat16, device=device)
         v = torch.empty_like(k)
-        layout = kv_layout(k, v, None, t, t * hkv * d, hkv * d)
+        layout = _pack_cache(k, v, None, t, t * hkv * d, hkv * d)
         check(L.pluto_qk_prepare(_stream(), _ptr(inputs[0]), _ptr(inputs[1]), _ptr(inputs[2]), 1,
                                  2 * hq * d, 2 * d, _ptr(self.weights_[0]), _ptr(self.weights_[1]),
-                                 None, _ptr(q), 1, C_byref(layout), 1, t, hq, hkv, d, p.rotary_dim,
+                                 None, _ptr(q), 1, layout, 1, t, hq, hkv, d, p.rotary_dim,
                                  p.rms_norm_epsilon, p.rope_theta, 1))
         qg = inputs[0].view(1, t, hq, 2, d)
         result = gqa_prefill(q, k, v, gate=qg[:, :, :, 1], round_to_bfloat16=True, want_core=True,
@@ -844,8 +872,8 @@ class QwenAttentionLayer(Layer):
             probabilities = torch.zeros((hq, t, t), dtype=torch.float32, device=device)
             rows = torch.arange(1, t + 1, dtype=torch.int32, device=device)
             table = torch.zeros((t, 1), dtype=torch.int32, device=device)
-            paged = kv_layout(k, v, table, t, t * hkv * d, hkv * d)
-            check(L.pluto_gqa_decode_probs(_stream(), _ptr(q), 1, C_byref(paged), _ptr(rows),
+            paged = _pack_cache(k, v, table, t, t * hkv * d, hkv * d)
+            check(L.pluto_gqa_decode_probs(_stream(), _ptr(q), 1, paged, _ptr(rows),
                                            _ptr(probabilities), t, t * t, t, hq, hkv, d))
             hooks.attention_probabilities_hook(
                 self.name(), ActivationType(DataType.FP32, (1, hq, t, t)), probabilities)
@@ -868,7 +896,7 @@ class QwenAttentionLayer(Layer):
         if dy is None or not dy.is_cuda or dy.dtype != torch.float32 or dy.numel() != t * hq * d:
             raise _invalid("sequence attention buffer has an invalid size or Executor")
         qg_in, k_in, _, q, k, _, core, maxima, normalizers, v = state.intermediates
-        L = _capi.lib()
+        L = _capi.fast()
         device = dy.device
         f32 = dict(dtype=torch.float32, device=device)
         dqg = torch.empty((t, hq, 2, d), **f32)
@@ -947,10 +975,9 @@ class DeltaNetLayer(Layer):
         width = p.value_heads * p.value_head_dim
         channels = 2 * p.key_heads * p.key_head_dim + width
         _validate_bf16_inputs(inputs, [channels, width, p.value_heads, p.value_heads], "DeltaNetLayer")
-        output = torch.empty((1, width), dtype=torch.bfloat16, device=inputs[0].device)
-        self.cache_.Step(inputs[0].view(-1), inputs[1].view(p.value_heads, p.value_head_dim),
-                         inputs[2].view(-1), inputs[3].view(-1), *self.weights_,
-                         output.view(p.value_heads, p.value_head_dim))
+        inputs = [x if x.is_contiguous() else x.contiguous() for x in inputs]
+        output = inputs[0].new_empty((1, width))
+        self.cache_.Step(*inputs, *self.weights_, output)
         return FwdResult([output], BackwardState())
 
     def bwd_impl(self, output_gradients, state, hooks):
@@ -1013,7 +1040,7 @@ class SequenceDeltaNetLayer(Layer):
             raise _invalid("DeltaNet expects four inputs on its Executor")
         _validate_bf16_inputs(inputs, [t * channels, t * width, t * p.value_heads, t * p.value_heads],
                               "SequenceDeltaNetLayer")
-        L, rnd = _capi.lib(), int(p.round_to_bfloat16)
+        L, rnd = _capi.fast(), int(p.round_to_bfloat16)
         device = inputs[0].device
         if not p.round_to_bfloat16:
             raise _unimplemented("sequence delta-net without bf16 rounding is not built")
@@ -1062,7 +1089,7 @@ class SequenceDeltaNetLayer(Layer):
         if dy is None or not dy.is_cuda or dy.dtype != torch.float32 or dy.numel() != t * width:
             raise _invalid("SequenceDeltaNetLayer requires batch-one buffers of the declared shape")
         qkv_in, z, a, b, post, core, _ = state.intermediates
-        L, rnd = _capi.lib(), int(p.round_to_bfloat16)
+        L, rnd = _capi.fast(), int(p.round_to_bfloat16)
         device = dy.device
         f32 = dict(dtype=torch.float32, device=device)
         conv_p, a_log_p, dt_bias_p, norm_p = self.parameters_owned_
@@ -1184,7 +1211,7 @@ class FullyConnectedLayer(Layer):
         tokens = inputs[0].numel() // self.input_dim_
         output = torch.empty((tokens, self.output_dim_), dtype=torch.bfloat16, device=inputs[0].device)
         scales = self.weights_[1] if len(self.weights_) == 2 else None
-        check(_capi.lib().pluto_linear_imported_fwd(
+        check(_capi.fast().pluto_linear_imported_fwd(
             _stream(), _ptr(self.weights_[0]), self.imported_storage_.value, _ptr(scales),
             _ptr(inputs[0]), _ptr(output), tokens, self.input_dim_, self.output_dim_))
         return FwdResult([output], BackwardState())
@@ -1260,7 +1287,7 @@ class DenseLayer(Layer):
                                * standard_deviation)
 
     def _workspace(self, rows, device):
-        need = _capi.lib().pluto_dense_workspace_bytes(rows, self.input_dim_, self.output_dim_)
+        need = _capi.fast().pluto_dense_workspace_bytes(rows, self.input_dim_, self.output_dim_)
         ws = torch.empty((need + 256,), dtype=torch.uint8, device=device)
         ptr = (ws.data_ptr() + 255) // 256 * 256
         return ws, ptr, need
@@ -1272,7 +1299,7 @@ class DenseLayer(Layer):
         dtype = activation_torch_dtype(self.output_type_)
         output = torch.empty((rows, self.output_dim_), dtype=dtype, device=inputs[0].device)
         ws, ptr, need = self._workspace(rows, inputs[0].device)
-        check(_capi.lib().pluto_dense_fwd(
+        check(_capi.fast().pluto_dense_fwd(
             _stream(), _ptr(inputs[0]), 1 if self.output_type_ == DataType.BF16 else 0,
             _ptr(self.weights_[0]), _ptr(self.weights_[1]), _ptr(output), rows, self.input_dim_,
             self.output_dim_, ptr, need))
@@ -1290,7 +1317,7 @@ class DenseLayer(Layer):
         _validate_buffer(x, rows * self.input_dim_ * element, "dense saved input")
         dx = torch.empty((rows, self.input_dim_), dtype=torch.float32, device=dy.device)
         ws, ptr, need = self._workspace(rows, dy.device)
-        check(_capi.lib().pluto_dense_bwd(
+        check(_capi.fast().pluto_dense_bwd(
             _stream(), _ptr(x), 1 if self.output_type_ == DataType.BF16 else 0, _ptr(self.weights_[0]),
             _ptr(dy), _ptr(dx), _ptr(self.gradients_[0]), _ptr(self.gradients_[1]), rows,
             self.input_dim_, self.output_dim_, ptr, need))
@@ -1319,7 +1346,7 @@ def DequantizeMatrix(input: torch.Tensor, storage: MatrixStorage, scales: Option
     if storage == MatrixStorage.kBFloat16:
         return input
     output = torch.empty((rows, cols), dtype=torch.bfloat16, device=input.device)
-    check(_capi.lib().pluto_dequantize_matrix(_stream(), _ptr(input), storage.value, _ptr(scales),
+    check(_capi.fast().pluto_dequantize_matrix(_stream(), _ptr(input), storage.value, _ptr(scales),
                                               _ptr(output), rows, cols))
     return output
 
@@ -1371,7 +1398,7 @@ class BlockLinearLayer(Layer):
             raise _invalid("block training requires the owning executor, exact dimensions and batch size one")
 
     def _workspace(self, device):
-        need = _capi.lib().pluto_block_linear_workspace_bytes(self.sequence_length_, self.input_dim_,
+        need = _capi.fast().pluto_block_linear_workspace_bytes(self.sequence_length_, self.input_dim_,
                                                               self.output_dim_)
         ws = torch.empty((need + 256,), dtype=torch.uint8, device=device)
         return ws, (ws.data_ptr() + 255) // 256 * 256, need
@@ -1384,7 +1411,7 @@ class BlockLinearLayer(Layer):
         output = torch.empty((t, self.output_dim_), device=inputs[0].device,
                              dtype=torch.float32 if self.output_float32_ else torch.bfloat16)
         ws, ptr, need = self._workspace(inputs[0].device)
-        check(_capi.lib().pluto_block_linear_fwd(
+        check(_capi.fast().pluto_block_linear_fwd(
             _stream(), _ptr(self.weights_[0]), _ptr(inputs[0]), _ptr(output),
             0 if self.output_float32_ else 1, t, self.input_dim_, self.output_dim_, ptr, need))
         return FwdResult([output], BackwardState(intermediates=[inputs[0]]))
@@ -1398,7 +1425,7 @@ class BlockLinearLayer(Layer):
         self._check(state.intermediates[0], t * self.input_dim_, 2)
         dx = torch.empty((t, self.input_dim_), dtype=torch.float32, device=dy.device)
         ws, ptr, need = self._workspace(dy.device)
-        check(_capi.lib().pluto_block_linear_bwd(
+        check(_capi.fast().pluto_block_linear_bwd(
             _stream(), _ptr(self.weights_[0]), _ptr(state.intermediates[0]), _ptr(dy), _ptr(dx),
             _ptr(self.parameter_.gradient()), t, self.input_dim_, self.output_dim_, ptr, need))
         return [dx]

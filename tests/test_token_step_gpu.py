@@ -1,0 +1,104 @@
+"""The one-launch token steps (token_step.cu) against the launches they replace, through the C ABI:
+contexts of one row, either side of a warp's turn and the longest the single launch takes (then the
+first it does not), and every shape rule of the delta-net step."""
+import pytest
+import torch
+
+from pluto_b200 import _capi
+from pluto_b200.layers import (CachedAttentionStep, DeltaNetParameters, DeltaNetState, FullAttentionParameters,
+                               KeyValueCache, gqa_decode)
+
+pytestmark = pytest.mark.gpu
+
+
+def stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("heads,dim,rotary", [((24, 4), 256, 64), ((5, 1), 128, 128), ((3, 3), 64, 32)])
+@pytest.mark.parametrize("cache_dtype,io_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("rounded", [True, False])
+def test_cached_step_matches_prepare_and_decode(heads, dim, rotary, cache_dtype, io_dtype, rounded):
+    hq, hkv = heads
+    p = FullAttentionParameters(query_heads=hq, key_value_heads=hkv, head_dim=dim, rotary_dim=rotary, capacity=1030,
+                                round_to_bfloat16=rounded)
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    keys, values = rnd(1030, hkv, dim).bfloat16(), rnd(1030, hkv, dim).bfloat16()
+    wq, wk = rnd(dim) * 0.1, rnd(dim) * 0.1
+    L = _capi.fast()
+    for position in (0, 1, 15, 16, 17, 500, 1023, 1024, 1029):
+        qg, k, v = rnd(hq, 2, dim).to(io_dtype), rnd(hkv, dim).to(io_dtype), rnd(hkv, dim).to(io_dtype)
+        caches = []
+        for _ in range(2):
+            cache = KeyValueCache.Create(1030, hkv, dim, cache_dtype)
+            cache.keys().copy_(keys)
+            cache.values().copy_(values)
+            cache.position_ = position
+            caches.append(cache)
+        out = torch.empty(hq, dim, device="cuda", dtype=io_dtype)
+        CachedAttentionStep(p, caches[0], qg, k, v, wq, wk, out)
+        assert caches[0].position() == position + 1
+        # the separate entry points
+        queries = torch.empty(1, hq, dim, device="cuda", dtype=torch.bfloat16 if rounded else torch.float32)
+        at = torch.tensor([position], dtype=torch.int32, device="cuda")
+        code = 1 if io_dtype == torch.bfloat16 else 0
+        _capi.check(L.pluto_qk_prepare(stream(), qg.data_ptr(), k.data_ptr(), v.data_ptr(), code, 2 * hq * dim, 2 * dim,
+                                       wq.data_ptr(), wk.data_ptr(), at.data_ptr(), queries.data_ptr(),
+                                       1 if rounded else 0, caches[1].packed_layout(), 1, 1, hq, hkv, dim, rotary,
+                                       p.rms_norm_epsilon, p.rope_theta, int(rounded)))
+        want = gqa_decode(queries, caches[1].keys()[None], caches[1].values()[None], at + 1, position + 1,
+                          gate=qg[None, :, 1], round_to_bfloat16=rounded,
+                          out=torch.empty(1, hq, dim, device="cuda", dtype=io_dtype))[0]
+        assert torch.equal(caches[0].values(), caches[1].values())
+        if rounded:
+            assert torch.equal(caches[0].keys(), caches[1].keys())
+        else:   # the unrounded rotation may or may not contract into an fma: one rounding of one product
+            assert ((caches[0].keys().float() - caches[1].keys().float()).abs() <= 2 ** -7 * caches[1].keys().float().abs() + 1e-6).all()
+        # one rounding of the output type apart: its ties can fall either way; the decode kernels carry P
+        # to 2^-17, so unrounded fp32 results agree to 1e-5 of values of order one
+        bound = (2 ** -7 if rounded or io_dtype == torch.bfloat16 else 1e-5) * want.float().abs() + 2e-5
+        assert ((out.float() - want.float()).abs() <= bound).all(), position
+    assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("key_heads,value_heads,dk,dv,taps", [(2, 6, 128, 128, 4), (3, 3, 128, 128, 1), (1, 8, 128, 128, 3),
+                                                              (1, 9, 128, 128, 4), (2, 4, 64, 128, 4), (2, 2, 128, 96, 4),
+                                                              (1, 2, 128, 128, 5)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rounded", [True, False])
+def test_delta_step_matches_its_four_launches(key_heads, value_heads, dk, dv, taps, dtype, rounded):
+    p = DeltaNetParameters(key_heads=key_heads, value_heads=value_heads, key_head_dim=dk, value_head_dim=dv,
+                           conv_kernel_dim=taps, round_to_bfloat16=rounded)
+    gen = torch.Generator(device="cuda").manual_seed(value_heads * 7 + taps)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    kq = key_heads * dk
+    channels = 2 * kq + value_heads * dv
+    conv, a_log, dt_bias, norm = rnd(channels, taps), rnd(value_heads), rnd(value_heads), rnd(dv)
+    state = DeltaNetState.Create(p)
+    window = torch.zeros(channels, taps, device="cuda")
+    S = torch.zeros(1, value_heads, dk, dv, device="cuda")
+    L, code, rnd_flag = _capi.fast(), 1 if dtype == torch.bfloat16 else 0, int(rounded)
+    f32 = dict(device="cuda", dtype=torch.float32)
+    for _ in range(6):
+        qkv, z, a, b = rnd(channels).to(dtype), rnd(value_heads, dv).to(dtype), rnd(value_heads).to(dtype), rnd(value_heads).to(dtype)
+        out = torch.empty(value_heads, dv, device="cuda", dtype=dtype)
+        state.Step(qkv, z, a, b, conv, a_log, dt_bias, norm, out)
+        post, g, beta = torch.empty(channels, **f32), torch.empty(value_heads, **f32), torch.empty(value_heads, **f32)
+        core, want = torch.empty(value_heads, dv, **f32), torch.empty_like(out)
+        _capi.check(L.pluto_gdn_conv_silu(stream(), qkv.data_ptr(), conv.data_ptr(), code, 1, 1, channels, taps, rnd_flag,
+                                          window.data_ptr(), post.data_ptr(), 0))
+        _capi.check(L.pluto_gdn_gates(stream(), a.data_ptr(), b.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), code, 1,
+                                      value_heads, rnd_flag, g.data_ptr(), beta.data_ptr()))
+        _capi.check(L.pluto_gdn_step(stream(), post.data_ptr(), post[kq:].data_ptr(), post[2 * kq:].data_ptr(), 0,
+                                     g.data_ptr(), beta.data_ptr(), S.data_ptr(), core.data_ptr(), 0, 1, key_heads,
+                                     value_heads, dk, dv, 1, 1.0, rnd_flag))
+        _capi.check(L.pluto_gdn_out_norm_gate(stream(), core.data_ptr(), 0, z.data_ptr(), code, norm.data_ptr(), value_heads,
+                                              dv, p.rms_norm_epsilon, rnd_flag, 1, want.data_ptr(), code))
+        assert torch.equal(state.convolution_state_.view_as(window), window)
+        # fp32 sums of 128 terms in another order: 128 * 2^-24 = 8e-6 of the largest entry; outputs one
+        # rounding (core, then three products) of their type apart
+        assert (state.recurrent_state_ - S).abs().max() <= 1e-5 * S.abs().max()
+        bound = (2 ** -6 if rounded or code else 2e-5) * want.float().abs() + 2e-5 * want.float().abs().max()
+        assert ((out.float() - want.float()).abs() <= bound).all()
+    assert _capi.kernel_status() == 0
