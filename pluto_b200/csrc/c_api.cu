@@ -393,6 +393,7 @@ int fill_decode(pluto::DecodeArgs* a, const void* q, int q_dtype, const pluto_kv
   a->batch = batch; a->q_heads = q_heads; a->kv_heads = kv_heads; a->head_dim = head_dim;
   a->split_tokens = decode_split_tokens(batch, kv_heads, max_seq_len);
   a->splits = pluto::decode_chunk_count(max_seq_len, a->split_tokens);
+  a->max_length = max_seq_len;
   if (a->splits > 65535) return fail(PLUTO_E_INVALID, "max_seq_len exceeds what one decode launch can split");
   a->scale = 1.0f / sqrtf(static_cast<float>(head_dim));
   a->status = pluto::kernel_status_word();

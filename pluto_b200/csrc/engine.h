@@ -168,6 +168,7 @@ struct DecodeArgs {
   float* partial_acc;       // workspace [batch, q_heads, splits, head_dim] (second section)
   int batch, q_heads, kv_heads, head_dim;
   int splits, split_tokens;
+  int max_length;           // the caller's bound on seq_lens
   float scale;
   int round;
   uint32_t* status;

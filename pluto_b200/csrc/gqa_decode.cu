@@ -4,10 +4,11 @@
 // (src/llm/layers/util/cached_attention_ops.cc:83-126, :131-178), which run one program per query
 // head (24-40 CTAs), re-read each KV head once per query head and keep the cache in fp32.  Here:
 //   * the cache is read exactly once: all query heads of a KV head are the rows of one MMA tile;
-//   * the sequence is split into fixed chunks across CTAs (split-KV); every CTA produces a
-//     partial (max, sum, accumulator), the four consumer warps of a CTA merge through shared
-//     memory, and a second kernel merges the chunks in a fixed order (deterministic, no atomics,
-//     no inter-CTA waits);
+//   * the sequence is split across CTAs (split-KV); every CTA produces a partial (max, sum,
+//     accumulator), the token groups of a CTA merge through shared memory.  Small problems are cut
+//     into at most sixteen parts per sequence that form a cluster and merge through distributed
+//     shared memory (one launch); large ones into fixed chunks that a second kernel merges.  The
+//     order is fixed either way (deterministic, no atomics);
 //   * K/V tiles travel global -> shared as tiled TMA loads (no multicast) over a 4-D map of the
 //     page pool (column, kv head, token in page, page): one elected thread issues a handful of
 //     box copies per 64-token stage into a 3-stage ring guarded by mbarriers, 128-byte swizzled
@@ -18,7 +19,7 @@
 // The cache is a page pool: token t of sequence b lives in page block_table[b][t / page_size]
 // (or page b when there is no table: one contiguous region per sequence).
 //
-// A plain fp32 kernel covers every other case (fp32 cache, head widths other than 64/128,
+// A plain fp32 kernel covers every other case (fp32 cache, head widths other than 64/128/256,
 // unrounded operands) with the same split/merge structure.
 #include "common.cuh"
 #include "engine.h"
@@ -26,10 +27,16 @@
 namespace pluto {
 namespace {
 
-constexpr int kTile = 64;          // tokens per pipeline stage
 constexpr int kDecodeStages = 3;
-constexpr int kConsumerWarps = 4;  // 16 tokens of every tile each
-constexpr int kDecodeThreads = (kConsumerWarps + 1) * 32;
+constexpr int kMaxClusterParts = 16;
+// Tokens per pipeline stage: 32 KB of K and V at head widths 128 and 256 (16 KB at 64), so that two
+// CTAs share an SM and one's set-up, first loads and output run under the other's stream (one CTA per
+// SM with 64-token stages at head width 256 took 238 us where this takes 142, at 60 sequences of up
+// to 4000 tokens, 4 KV heads).
+template <int D>
+constexpr int kTile = D == 256 ? 32 : 64;
+template <int D>
+constexpr int kTokenWarps = kTile<D> / 16;   // 16 tokens of every tile each
 
 // Sequence length as the kernels use it: the device value clamped into what the host sized the
 // grid and the workspace for, [0, decode_chunk_capacity(splits, split_tokens)].  A value outside is a caller error; it
@@ -76,7 +83,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                          uint32_t b1) {
-  asm volatile(
+  // (not volatile: the order of independent products is the compiler's to choose)
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
       "{%8, %9}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -88,49 +96,94 @@ struct DecodeBarriers {
   uint64_t empty[kDecodeStages];
 };
 
-// grid (kv_heads, batch, splits), chunks in decreasing index order.  Partials: acc [B, Hq, splits, D], ml [B, Hq, splits, 2].
+// Head width 256: two warps share 16 tokens, each accumulating half of the channels (one warp's
+// accumulators and query fragments would take 192 registers).
 template <int D>
+constexpr int kChannelParts = D == 256 ? 2 : 1;
+constexpr int kDecodeThreads = (4 + 1) * 32;   // four consumer warps at every width, one producer
+template <int D>
+constexpr int kDecodeStageBytes = 2 * kTile<D> * D * 2;
+
+// The reference's output stage (cached_attention_ops.cc:120-125): R(R(acc / l) * R(sigmoid(gate))).
+__device__ __forceinline__ void store_output(const DecodeArgs& a, int b, int head, int d, float value) {
+  if (a.round) value = bf16_round(value);
+  if (a.gate) {
+    const size_t g = static_cast<size_t>(b) * a.gate_token + static_cast<size_t>(head) * a.gate_head + d;
+    const float x = a.gate_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[g])
+                                   : static_cast<const float*>(a.gate)[g];
+    float sigmoid = 1.0f / (1.0f + expf(-x));
+    if (a.round) sigmoid = bf16_round(sigmoid);
+    value *= sigmoid;
+    if (a.round) value = bf16_round(value);
+  }
+  const size_t idx = (static_cast<size_t>(b) * a.q_heads + head) * a.head_dim + d;
+  if (a.out_is_bf16) static_cast<__nv_bfloat16*>(a.out)[idx] = __float2bfloat16_rn(value);
+  else static_cast<float*>(a.out)[idx] = value;
+}
+
+// kCluster false: grid (kv_heads, batch, splits), chunks in decreasing index order; partials
+//   acc [B, Hq, splits, D], ml [B, Hq, splits, 2] for the merge kernel.
+// kCluster true: grid (kv_heads, batch, parts), the parts of a (sequence, KV head) are one cluster and
+//   cut the sequence's own length evenly; their partials meet in distributed shared memory and the
+//   output leaves from here, so the call is one launch and needs no scratch.
+template <int D, bool kCluster>
 __global__ void __launch_bounds__(kDecodeThreads, 2)
 gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               DecodeArgs a) {
+  constexpr int kTile = pluto::kTile<D>, kTokenWarps = pluto::kTokenWarps<D>;
   constexpr int kHalves = D / 64;                 // 64-column (128-byte) swizzled slabs per row
   constexpr int kHalfBytes = kTile * 128;         // one slab of a tile
   constexpr int kTileBytes = kHalves * kHalfBytes;
   constexpr int kStageBytes = 2 * kTileBytes;     // K tile then V tile
+  constexpr int kParts = kChannelParts<D>, kWarps = kTokenWarps * kParts;
+  static_assert((kWarps + 1) * 32 == kDecodeThreads, "warps");
+  constexpr int kOwnBlocks = D / 16 / kParts;     // 16-channel blocks of the accumulator a warp owns
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   DecodeBarriers* bar = reinterpret_cast<DecodeBarriers*>(smem + kDecodeStages * kStageBytes);
 
-  pdl_launch_dependents();   // the merge may be placed as SMs free up; it waits for this grid itself
-  // chunks in decreasing index order, (KV head, sequence) fastest: the four short chunks of every
-  // sequence are the last CTAs of the launch
-  const int split = gridDim.z - 1 - blockIdx.z, kv_head = blockIdx.x, b = blockIdx.y;
-  const int length = bounded_length(a, b, 36);
-  const int begin = decode_chunk_begin(split, a.split_tokens);
-  if (begin >= length) return;  // whole CTA leaves before touching any barrier
-  const int end = min(length, begin + decode_chunk_tokens(split, a.split_tokens));
-  const int tiles = (end - begin + kTile - 1) / kTile;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int group = a.q_heads / a.kv_heads;
-
+  // Launched with programmatic stream serialisation: the set-up of this grid overlaps the end of the
+  // one before it, whose results (query, lengths, cache) are read only after the wait.
   if (threadIdx.x == 0) {
     for (int s = 0; s < kDecodeStages; ++s) {
       mbar_init(&bar->full[s], 1);
-      mbar_init(&bar->empty[s], kConsumerWarps);
+      mbar_init(&bar->empty[s], kWarps);
     }
     mbar_fence_init();
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
   }
+  pdl_wait();
+  pdl_launch_dependents();   // the merge (or the next call) may be placed as SMs free up
+
+  const int kv_head = blockIdx.x, b = blockIdx.y;
+  const int length = bounded_length(a, b, 36);
+  int begin, end, split = 0;
+  if (kCluster) {
+    const int parts = gridDim.z, chunk = ((length + parts - 1) / parts + kTile - 1) / kTile * kTile;
+    begin = min(length, static_cast<int>(blockIdx.z) * chunk);
+    end = min(length, begin + chunk);
+  } else {
+    // chunks in decreasing index order, (KV head, sequence) fastest: the four short chunks of every
+    // sequence are the last CTAs of the launch
+    split = gridDim.z - 1 - blockIdx.z;
+    begin = decode_chunk_begin(split, a.split_tokens);
+    if (begin >= length) return;  // whole CTA leaves before touching any barrier
+    end = min(length, begin + decode_chunk_tokens(split, a.split_tokens));
+  }
+  const int tiles = (end - begin + kTile - 1) / kTile;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int group = a.q_heads / a.kv_heads;
   __syncthreads();
 
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
-  float o[D / 8][4];
+  float o[2 * kOwnBlocks][4];
+  const int token_warp = warp % kTokenWarps, part = warp / kTokenWarps;
 
-  if (warp == kConsumerWarps) {
+  if (warp == kWarps) {
     // ---------------------------------------------------------------- producer warp
     if (lane == 0) {
-      tma_prefetch_desc(&map_k);
-      tma_prefetch_desc(&map_v);
       bool ok = true;
       const int rows = a.box_rows;  // tokens per box: divides both the tile and the page size
       for (int it = 0; it < tiles && ok; ++it) {
@@ -166,30 +219,33 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
     // A fragments of Q: rows = query heads of this KV head (rows >= group are zero).
     uint32_t qf[D / 16][4];
     {
-      const int r0 = lane / 4, r1 = r0 + 8;
+      const int r0 = lane / 4;
       const size_t head0 = static_cast<size_t>(b) * a.q_heads + static_cast<size_t>(kv_head) * group;
+      const bool pairs = a.q_is_bf16 && (reinterpret_cast<uintptr_t>(a.q) & 3u) == 0;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int col = ks * 16 + half * 8 + (lane % 4) * 2;
-          float x0 = 0.f, x1 = 0.f, y0 = 0.f, y1 = 0.f;
-          if (a.q_is_bf16) {
-            const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(a.q);
-            if (r0 < group) { x0 = __bfloat162float(q[(head0 + r0) * D + col]); x1 = __bfloat162float(q[(head0 + r0) * D + col + 1]); }
-            if (r1 < group) { y0 = __bfloat162float(q[(head0 + r1) * D + col]); y1 = __bfloat162float(q[(head0 + r1) * D + col + 1]); }
-          } else {
-            const float* q = static_cast<const float*>(a.q);
-            if (r0 < group) { x0 = q[(head0 + r0) * D + col]; x1 = q[(head0 + r0) * D + col + 1]; }
-            if (r1 < group) { y0 = q[(head0 + r1) * D + col]; y1 = q[(head0 + r1) * D + col + 1]; }
+        for (int i = 0; i < 4; ++i) {   // rows r0, r0 + 8; columns 0-7, 8-15 of the step
+          const int r = r0 + (i & 1) * 8, col = ks * 16 + (i >> 1) * 8 + (lane % 4) * 2;
+          uint32_t packed = 0u;
+          if (r < group) {
+            const size_t at = (head0 + r) * D + col;
+            if (pairs) {
+              packed = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(a.q) + at);
+            } else if (a.q_is_bf16) {
+              const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(a.q) + at;
+              packed = pack_bf16(__bfloat162float(q[0]), __bfloat162float(q[1]));
+            } else {
+              const float* q = static_cast<const float*>(a.q) + at;
+              packed = pack_bf16(q[0], q[1]);
+            }
           }
-          qf[ks][half * 2 + 0] = pack_bf16(x0, x1);
-          qf[ks][half * 2 + 1] = pack_bf16(y0, y1);
+          qf[ks][i] = packed;
         }
       }
     }
 #pragma unroll
-    for (int nb = 0; nb < D / 8; ++nb)
+    for (int nb = 0; nb < 2 * kOwnBlocks; ++nb)
 #pragma unroll
       for (int i = 0; i < 4; ++i) o[nb][i] = 0.0f;
     const float scale_log2 = a.scale * 1.4426950408889634f;
@@ -201,41 +257,43 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
       const uint32_t k_tile = smem_u32(smem + st * kStageBytes);
       const uint32_t v_tile = k_tile + kTileBytes;
       const int live = end - (begin + it * kTile);  // live tokens in this tile (may exceed kTile)
-      if (live < (warp + 1) * 16) {
+      if (live < (token_warp + 1) * 16) {
         // Rows past the sequence end hold whatever the page (or an earlier stage) held; their
         // probabilities are zero, but 0 * NaN would poison P V, so this warp clears its own dead
-        // V rows first.  Only the last tile of a sequence takes this path.
-        for (int r = max(live, warp * 16); r < (warp + 1) * 16; ++r)
-          for (int c = lane; c < kHalves * 8; c += 32)
-            sts_b32x4(smem_u32(smem) + st * kStageBytes + kTileBytes + (c / 8) * kHalfBytes + r * 128 +
-                          (c % 8) * 16, 0u, 0u, 0u, 0u);
+        // V rows (its channels of them) first.  Only the last tile of a sequence takes this path.
+        for (int r = max(live, token_warp * 16); r < (token_warp + 1) * 16; ++r)
+          for (int c = part * kHalves * 8 / kParts + lane; c < (part + 1) * kHalves * 8 / kParts; c += 32)
+            sts_b32x4(v_tile + (c / 8) * kHalfBytes + r * 128 + (c % 8) * 16, 0u, 0u, 0u, 0u);
         fence_proxy_async();
         __syncwarp();
       }
       // ---- S = Q K^T for this warp's 16 tokens: two n-blocks of 8 tokens
+      // (two accumulators each, for the even and the odd steps: the chain of dependent products is what
+      // a tile waits for)
       float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float s_odd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
+      for (int kp = 0; kp < D / 32; ++kp) {
 #pragma unroll
-        for (int kp = 0; kp < D / 32; ++kp) {
+        for (int nb = 0; nb < 2; ++nb) {
           uint32_t kf[4];
           // element (row, col) of a tile sits in slab col/64 at row*128 + ((col%64)/8 ^ row%8)*16
-          const int row = warp * 16 + nb * 8 + lane % 8;
+          const int row = token_warp * 16 + nb * 8 + lane % 8;
           const int chunk = (kp * 4 + lane / 8) % 8;
           ldmatrix_x4(kf, k_tile + (kp / 2) * kHalfBytes + row * 128 + ((chunk ^ (row % 8)) * 16));
           mma_bf16(s[nb], qf[2 * kp], kf[0], kf[1]);
-          mma_bf16(s[nb], qf[2 * kp + 1], kf[2], kf[3]);
+          mma_bf16(s_odd[nb], qf[2 * kp + 1], kf[2], kf[3]);
         }
       }
       // ---- online softmax (rows lane/4 and lane/4+8; columns = tokens)
-      const int token0 = begin + it * kTile + warp * 16 + (lane % 4) * 2;
+      const int token0 = begin + it * kTile + token_warp * 16 + (lane % 4) * 2;
       float tile_max[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int token = token0 + nb * 8 + (i & 1);
-          s[nb][i] = token < end ? s[nb][i] * scale_log2 : -INFINITY;
+          s[nb][i] = token < end ? (s[nb][i] + s_odd[nb][i]) * scale_log2 : -INFINITY;
           tile_max[i >> 1] = fmaxf(tile_max[i >> 1], s[nb][i]);
         }
       // P is split into a bf16 high part and a bf16 remainder so that P V keeps ~16 mantissa
@@ -261,22 +319,27 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
         pl[r] = pack_bf16(p00 - bf16_lo(pf[r]), p01 - bf16_hi(pf[r]));
         pl[2 + r] = pack_bf16(p10 - bf16_lo(pf[2 + r]), p11 - bf16_hi(pf[2 + r]));
 #pragma unroll
-        for (int nb = 0; nb < D / 8; ++nb) {
+        for (int nb = 0; nb < 2 * kOwnBlocks; ++nb) {
           o[nb][2 * r] *= correction;
           o[nb][2 * r + 1] *= correction;
         }
       }
-      // ---- O += P V
+      // ---- O += P V over this warp's channels; the high-part products of two blocks before their
+      // remainders, so that no product waits for the one just issued
 #pragma unroll
-      for (int np = 0; np < D / 16; ++np) {
-        uint32_t vf[4];
-        const int row = warp * 16 + ((lane / 8) & 1) * 8 + lane % 8;
-        const int chunk = (np * 2 + lane / 16) % 8;
-        ldmatrix_x4_trans(vf, v_tile + (np / 4) * kHalfBytes + row * 128 + ((chunk ^ (row % 8)) * 16));
-        mma_bf16(o[2 * np], pf, vf[0], vf[1]);
-        mma_bf16(o[2 * np], pl, vf[0], vf[1]);
-        mma_bf16(o[2 * np + 1], pf, vf[2], vf[3]);
-        mma_bf16(o[2 * np + 1], pl, vf[2], vf[3]);
+      for (int np = 0; np < kOwnBlocks; np += 2) {
+        uint32_t vf[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int block = part * kOwnBlocks + np + u;
+          const int row = token_warp * 16 + ((lane / 8) & 1) * 8 + lane % 8;
+          const int chunk = (block * 2 + lane / 16) % 8;
+          ldmatrix_x4_trans(vf[u], v_tile + (block / 4) * kHalfBytes + row * 128 + ((chunk ^ (row % 8)) * 16));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mma_bf16(o[2 * np + u], pf, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mma_bf16(o[2 * np + u], pl, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar->empty[st]);
@@ -284,51 +347,97 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   }
   __syncthreads();  // every stage consumed, every copy landed: the ring can be reused as scratch
 
-  // ---- merge the four warps' partial softmax states through shared memory (ld.shared / st.shared
-  // by address: `smem` went through alignment arithmetic and is a generic pointer to the compiler)
-  const uint32_t scratch = smem_u32(smem);                               // fp32 [warps][16][D]
-  const uint32_t scratch_ml = scratch + kConsumerWarps * 16 * D * 4;     // fp32 [warps][16][2]
-  if (warp < kConsumerWarps) {
+  // ---- merge the token groups' partial softmax states through shared memory (ld.shared / st.shared
+  // by address: `smem` went through alignment arithmetic and is a generic pointer).  Rows are 8 floats
+  // longer than the head, so that the pair stores of half a warp (4 rows x 4 pairs) hit all banks once.
+  constexpr int kRow = D + 8;
+  const uint32_t scratch = smem_u32(smem);                               // fp32 [token groups][16][kRow]
+  const uint32_t scratch_ml = scratch + kTokenWarps * 16 * kRow * 4;     // fp32 [token groups][16][2]
+  const uint32_t merged = scratch + kDecodeStages * kStageBytes / 2;     // fp32 [16][D], [16][2], [parts][16][2]
+  const uint32_t merged_ml = merged + 16 * D * 4, all_ml = merged_ml + 16 * 8;
+  static_assert(kTokenWarps * 16 * (kRow + 2) * 4 <= kDecodeStages * kStageBytes / 2 &&
+                    16 * (D + 2 + 2 * kMaxClusterParts) * 4 <= kDecodeStages * kStageBytes / 2, "merge scratch");
+  if (warp < kWarps) {
     const int r0 = lane / 4;
 #pragma unroll
-    for (int nb = 0; nb < D / 8; ++nb) {
-      const int col = nb * 8 + (lane % 4) * 2;
-      sts_f32(scratch + ((warp * 16 + r0) * D + col) * 4, o[nb][0]);
-      sts_f32(scratch + ((warp * 16 + r0) * D + col + 1) * 4, o[nb][1]);
-      sts_f32(scratch + ((warp * 16 + r0 + 8) * D + col) * 4, o[nb][2]);
-      sts_f32(scratch + ((warp * 16 + r0 + 8) * D + col + 1) * 4, o[nb][3]);
-    }
-    if (lane % 4 == 0) {
-      sts_f32(scratch_ml + ((warp * 16 + r0) * 2) * 4, m_run[0]);
-      sts_f32(scratch_ml + ((warp * 16 + r0) * 2 + 1) * 4, l_run[0]);
-      sts_f32(scratch_ml + ((warp * 16 + r0 + 8) * 2) * 4, m_run[1]);
-      sts_f32(scratch_ml + ((warp * 16 + r0 + 8) * 2 + 1) * 4, l_run[1]);
+    for (int half = 0; half < 2; ++half) {
+      const int r = r0 + half * 8;
+      if (r >= group) continue;   // rows without a query head
+      const uint32_t row = scratch + ((token_warp * 16 + r) * kRow + part * (D / kParts) + (lane % 4) * 2) * 4;
+#pragma unroll
+      for (int nb = 0; nb < 2 * kOwnBlocks; ++nb)
+        sts_b64(row + nb * 32, f2_pack(o[nb][2 * half], o[nb][2 * half + 1]));
+      if (lane % 4 == 0 && part == 0)
+        sts_b64(scratch_ml + (token_warp * 16 + r) * 8, f2_pack(m_run[half], l_run[half]));
     }
   }
   __syncthreads();
   for (int idx = threadIdx.x; idx < group * D; idx += kDecodeThreads) {
     const int r = idx / D, d = idx % D;
-    float m_w[kConsumerWarps], m_tot = -INFINITY;
+    float m_w[kTokenWarps], m_tot = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < kConsumerWarps; ++w) {
+    for (int w = 0; w < kTokenWarps; ++w) {
       m_w[w] = lds_f32(scratch_ml + ((w * 16 + r) * 2) * 4);
       m_tot = fmaxf(m_tot, m_w[w]);
     }
+    const float m_safe = m_tot == -INFINITY ? 0.0f : m_tot;   // a cluster part without tokens
     float acc = 0.0f, l_tot = 0.0f;
 #pragma unroll
-    for (int w = 0; w < kConsumerWarps; ++w) {
-      const float f = fast_exp2(m_w[w] - m_tot);
-      acc += lds_f32(scratch + ((w * 16 + r) * D + d) * 4) * f;
+    for (int w = 0; w < kTokenWarps; ++w) {
+      const float f = fast_exp2(m_w[w] - m_safe);
+      acc += lds_f32(scratch + ((w * 16 + r) * kRow + d) * 4) * f;
       l_tot += lds_f32(scratch_ml + ((w * 16 + r) * 2 + 1) * 4) * f;
     }
-    const size_t head = static_cast<size_t>(b) * a.q_heads + static_cast<size_t>(kv_head) * group + r;
-    const size_t slot = head * a.splits + split;
-    a.partial_acc[slot * D + d] = acc;
-    if (d == 0) {
-      a.partial_ml[slot * 2] = m_tot;
-      a.partial_ml[slot * 2 + 1] = l_tot;
+    if (kCluster) {
+      sts_f32(merged + idx * 4, acc);
+      if (d == 0) {
+        sts_f32(merged_ml + r * 8, m_tot);
+        sts_f32(merged_ml + r * 8 + 4, l_tot);
+      }
+    } else {
+      const size_t head = static_cast<size_t>(b) * a.q_heads + static_cast<size_t>(kv_head) * group + r;
+      const size_t slot = head * a.splits + split;
+      a.partial_acc[slot * D + d] = acc;
+      if (d == 0) {
+        a.partial_ml[slot * 2] = m_tot;
+        a.partial_ml[slot * 2 + 1] = l_tot;
+      }
     }
   }
+  if (!kCluster) return;
+
+  // ---- the parts' states, in part order; the cluster shares the group's outputs out
+  const int parts = gridDim.z;
+  cluster_sync();
+  for (int i = threadIdx.x; i < parts * group * 2; i += kDecodeThreads) {
+    const int z = i / (group * 2), at = i % (group * 2);
+    sts_f32(all_ml + (z * 32 + at) * 4, lds_cluster_f32(merged_ml + at * 4, z));
+  }
+  __syncthreads();
+  for (int idx = blockIdx.z * kDecodeThreads + threadIdx.x; idx < group * D; idx += parts * kDecodeThreads) {
+    const int r = idx / D, d = idx % D, head = kv_head * group + r;
+    float x[kMaxClusterParts], m_tot = -INFINITY;
+#pragma unroll
+    for (int z = 0; z < kMaxClusterParts; ++z)
+      if (z < parts) {
+        x[z] = lds_cluster_f32(merged + idx * 4, z);
+        m_tot = fmaxf(m_tot, lds_f32(all_ml + (z * 32 + r * 2) * 4));
+      }
+    float acc = 0.0f, l = 0.0f;
+#pragma unroll
+    for (int z = 0; z < kMaxClusterParts; ++z)
+      if (z < parts) {
+        const float m = lds_f32(all_ml + (z * 32 + r * 2) * 4);
+        const float w = m == -INFINITY ? 0.0f : fast_exp2(m - m_tot);
+        acc = fmaf(x[z], w, acc);
+        l = fmaf(lds_f32(all_ml + (z * 32 + r * 2 + 1) * 4), w, l);
+      }
+    // (a length of zero is a caller error: zeros, not 0 / 0)
+    store_output(a, b, head, d, length > 0 ? acc / l : 0.0f);
+    if (d == 0 && a.lse)
+      a.lse[static_cast<size_t>(b) * a.q_heads + head] = length > 0 ? m_tot * 0.6931471805599453f + logf(l) : -INFINITY;
+  }
+  cluster_sync();   // the peers' shared memory is read until here
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -336,6 +445,7 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
 // token row in flight, each lane owning head_dim/32 (<= 8) channels.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) gqa_decode_generic(DecodeArgs a) {
+  pdl_wait();
   pdl_launch_dependents();
   const int split = gridDim.z - 1 - blockIdx.z, head = blockIdx.x, b = blockIdx.y;
   const int length = bounded_length(a, b, 37);
@@ -419,6 +529,7 @@ constexpr int kMergeSplits = 1024;   // chunk weights held in shared memory per 
 
 __global__ void __launch_bounds__(kMergeThreads) gqa_decode_merge(DecodeArgs a) {
   pdl_wait();   // the chunk kernel's partials are complete and visible from here on
+  pdl_launch_dependents();
   const int head = blockIdx.x, b = blockIdx.y, D = a.head_dim;
   const int length = bounded_length(a, b, 38);
   const int splits = decode_chunk_count(length, a.split_tokens);   // <= a.splits
@@ -480,21 +591,7 @@ __global__ void __launch_bounds__(kMergeThreads) gqa_decode_merge(DecodeArgs a) 
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
     const int d = threadIdx.x + c * kMergeThreads;
-    if (d >= D) continue;
-    float value = acc[c] / l_tot;
-    if (a.round) value = bf16_round(value);
-    if (a.gate) {
-      const size_t g = static_cast<size_t>(b) * a.gate_token + static_cast<size_t>(head) * a.gate_head + d;
-      const float x = a.gate_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[g])
-                                     : static_cast<const float*>(a.gate)[g];
-      float sigmoid = 1.0f / (1.0f + expf(-x));
-      if (a.round) sigmoid = bf16_round(sigmoid);
-      value *= sigmoid;
-      if (a.round) value = bf16_round(value);
-    }
-    const size_t idx = (static_cast<size_t>(b) * a.q_heads + head) * D + d;
-    if (a.out_is_bf16) static_cast<__nv_bfloat16*>(a.out)[idx] = __float2bfloat16_rn(value);
-    else static_cast<float*>(a.out)[idx] = value;
+    if (d < D) store_output(a, b, head, d, acc[c] / l_tot);
   }
   if (threadIdx.x == 0 && a.lse) {
     // natural-log sum-exp of the scaled scores
@@ -549,7 +646,7 @@ __global__ void __launch_bounds__(256) gqa_decode_probs(DecodeArgs a, float* pro
 
 template <int D>
 constexpr size_t decode_smem() {
-  return 1024 + kDecodeStages * 2 * kTile * D * 2 + sizeof(DecodeBarriers);
+  return 1024 + kDecodeStages * kDecodeStageBytes<D> + sizeof(DecodeBarriers);
 }
 
 // 4-D map of a bf16 page pool: (column, kv head, token in page, page); box = 64 columns x
@@ -585,53 +682,87 @@ bool make_pool_map(CUtensorMap* map, const void* base, const DecodeArgs& a, int 
 bool gqa_decode_uses_tensor_cores(const DecodeArgs& a) {
   const int group = a.q_heads / a.kv_heads;
   const int pages = a.block_table ? a.num_pages : a.batch;
-  return a.k_bases == nullptr && a.kv_is_bf16 && (a.head_dim == 64 || a.head_dim == 128) && group <= 16 &&
+  return a.k_bases == nullptr && a.kv_is_bf16 && (a.head_dim == 64 || a.head_dim == 128 || a.head_dim == 256) && group <= 16 &&
          (a.round || a.q_is_bf16) && a.token_stride % 8 == 0 && a.page_stride % 8 == 0 &&
-         a.page_size % 16 == 0 && pages > 0 &&
+         (a.block_table == nullptr || a.page_size % 16 == 0) && pages > 0 &&
          (reinterpret_cast<uintptr_t>(a.k_base) & 15u) == 0 &&
          (reinterpret_cast<uintptr_t>(a.v_base) & 15u) == 0;
 }
 
+namespace {
+
+template <typename... Params>
+cudaError_t launch_decode(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                          int cluster_z, const Params&... params) {
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = attributes[1].val.clusterDim.y = 1;
+  attributes[1].val.clusterDim.z = static_cast<unsigned>(cluster_z);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = attributes;
+  config.numAttrs = cluster_z > 0 ? 2 : 1;
+  return cudaLaunchKernelEx(&config, kernel, params...);
+}
+
+template <int D>
+cudaError_t launch_tc(cudaStream_t stream, const CUtensorMap& map_k, const CUtensorMap& map_v, const DecodeArgs& a,
+                      int parts) {
+  auto kernel = parts > 0 ? gqa_decode_tc<D, true> : gqa_decode_tc<D, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(decode_smem<D>()));
+  if (e == cudaSuccess && parts > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  return launch_decode(kernel, dim3(a.kv_heads, a.batch, parts > 0 ? parts : a.splits), kDecodeThreads,
+                       decode_smem<D>(), stream, parts, map_k, map_v, a);
+}
+
+// Parts per (sequence, KV head) of the one-launch form, 0 for chunks + merge kernel.
+// One launch while the caches it may read hold at most 256 MB (about 40 us of HBM): as many parts as keep
+// the grid near the 296 CTAs that are resident at once (up to 400: the ragged lengths leave gaps) and
+// a part above 32 tokens; 16 parts are beyond the portable cluster size and opted into.  Measured, best
+// one-launch form against chunks + merge: 8 units (sequence x KV head) of up to 30000 tokens 33 against
+// 44 us, 16 of 3000 (width 256) 18 / 20, 128 of 2000 22 / 27, 480 of 500 27 / 34.  Above, the merge is a
+// few per cent and whole-chip balance counts: 240 units of 4000 tokens (width 256) 143 against 113 us,
+// 64 of 20000 171 / 144, 720 of 8000 (width 64) 175 / 138.
+int cluster_parts(const DecodeArgs& a) {
+  const long long units = static_cast<long long>(a.batch) * a.kv_heads;
+  if (units * a.max_length * a.head_dim * 4 > 256LL << 20) return 0;
+  int z = 1;
+  while (z < kMaxClusterParts && units * z * 2 <= 400 && a.max_length >= z * 2 * 32) z *= 2;
+  return z;
+}
+
+}  // namespace
+
 cudaError_t gqa_decode(cudaStream_t stream, const DecodeArgs& args) {
   DecodeArgs a = args;
+  cudaError_t e;
   if (gqa_decode_uses_tensor_cores(a)) {
-    const dim3 grid(a.kv_heads, a.batch, a.splits);
-    cudaError_t e;
-    a.box_rows = a.page_size % kTile == 0 ? kTile : 16;
+    // (without a block table a box past the end of its sequence's region reads zeros: any size goes)
+    const int tile = a.head_dim == 256 ? kTile<256> : kTile<128>;
+    a.box_rows = a.block_table == nullptr || a.page_size % tile == 0 ? tile : 16;
     const int pages = a.block_table ? a.num_pages : a.batch;
     CUtensorMap map_k, map_v;
     if (!make_pool_map(&map_k, a.k_base, a, pages) || !make_pool_map(&map_v, a.v_base, a, pages))
       return cudaErrorInvalidValue;
-    if (a.head_dim == 128) {
-      e = cudaFuncSetAttribute(gqa_decode_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(decode_smem<128>()));
-      if (e != cudaSuccess) return e;
-      gqa_decode_tc<128><<<grid, kDecodeThreads, decode_smem<128>(), stream>>>(map_k, map_v, a);
-    } else {
-      e = cudaFuncSetAttribute(gqa_decode_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(decode_smem<64>()));
-      if (e != cudaSuccess) return e;
-      gqa_decode_tc<64><<<grid, kDecodeThreads, decode_smem<64>(), stream>>>(map_k, map_v, a);
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    const int parts = cluster_parts(a);
+    e = a.head_dim == 256 ? launch_tc<256>(stream, map_k, map_v, a, parts)
+        : a.head_dim == 128 ? launch_tc<128>(stream, map_k, map_v, a, parts)
+                            : launch_tc<64>(stream, map_k, map_v, a, parts);
+    if (e != cudaSuccess || parts > 0) return e;
   } else {
-    gqa_decode_generic<<<dim3(a.q_heads, a.batch, a.splits), 128, 0, stream>>>(a);
-    cudaError_t e = cudaGetLastError();
+    e = launch_decode(gqa_decode_generic, dim3(a.q_heads, a.batch, a.splits), 128, 0, stream, 0, a);
     if (e != cudaSuccess) return e;
   }
-  // The merge is launched with programmatic stream serialisation: its CTAs are placed while the
-  // chunk kernel's last CTAs still run, and wait for that grid before they read a partial.
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(a.q_heads, a.batch);
-  config.blockDim = dim3(kMergeThreads);
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, gqa_decode_merge, a);
+  // The merge's CTAs are placed while the chunk kernel's last CTAs still run, and wait for that grid
+  // before they read a partial.
+  return launch_decode(gqa_decode_merge, dim3(a.q_heads, a.batch), kMergeThreads, 0, stream, 0, a);
 }
 
 cudaError_t gqa_decode_probabilities(cudaStream_t stream, const DecodeArgs& a, float* probs,

@@ -75,7 +75,26 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
   const int length = a.position + 1, half = a.rotary / 2;
   const size_t row0 = static_cast<size_t>(kv_head) * D + c0;
 
-  // the gate of this thread's output channel, requested before anything waits
+  // What no kernel of a decoding stream writes may be read before the wait; everything else after it.
+  float w_norm[kPer];
+  if (warp < 2) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) w_norm[i] = 1.0f + (warp == 0 ? a.q_norm : a.k_norm)[c0 + i];
+  }
+  pdl_wait();
+  pdl_launch_dependents();   // the next launch sets itself up meanwhile and waits for this grid in turn
+  // The first rows of the cache and the gate of this thread's output channel are requested before
+  // anything waits: at short contexts the kernel is a chain of memory round trips.
+  constexpr int kAhead = 2;
+  float k_ahead[kAhead][kPer], v_ahead[kAhead][kPer];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int t = warp + u * kStepWarps;
+    if (t < a.position) {
+      load_row<kPer, KV_BF16>(a.k_cache, static_cast<size_t>(t) * a.token_stride + row0, k_ahead[u]);
+      load_row<kPer, KV_BF16>(a.v_cache, static_cast<size_t>(t) * a.token_stride + row0, v_ahead[u]);
+    }
+  }
   float gate = 0.0f;
   if (threadIdx.x < D) gate = load_any(a.q_gate, static_cast<size_t>(head) * 2 * D + D + threadIdx.x, a.in_is_bf16);
   if (static_cast<int>(threadIdx.x) < half) {
@@ -89,7 +108,6 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
   if (warp < 2) {
     const void* in = warp == 0 ? a.q_gate : a.k;
     const size_t in0 = warp == 0 ? static_cast<size_t>(head) * 2 * D : static_cast<size_t>(kv_head) * D;
-    const float* norm = warp == 0 ? a.q_norm : a.k_norm;
     float sq = 0.0f;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) n[i] = load_any(in, in0 + c0 + i, a.in_is_bf16);
@@ -105,7 +123,7 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
     const float inverse = rsqrtf(warp_sum(sq) / static_cast<float>(D) + a.epsilon);
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      n[i] = rnd(n[i] * inverse * (1.0f + norm[c0 + i]), a.round);
+      n[i] = rnd(n[i] * inverse * w_norm[i], a.round);
       vec[warp][c0 + i] = n[i];
     }
   } else if (warp == 2) {
@@ -145,15 +163,22 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
 #pragma unroll
   for (int i = 0; i < kPer; ++i) q[i] = vec[0][c0 + i];
   float top = -INFINITY;
-#pragma unroll 4
-  for (int t = warp; t < a.position; t += kStepWarps) {
-    float k[kPer], dot = 0.0f;
-    load_row<kPer, KV_BF16>(a.k_cache, static_cast<size_t>(t) * a.token_stride + row0, k);
+  auto attend = [&](int t, const float (&k)[kPer]) {
+    float dot = 0.0f;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) dot = fmaf(k[i], q[i], dot);
     dot = warp_sum(dot) * a.scale;
     if (lane == 0) score[t] = dot;
     top = fmaxf(top, dot);
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (warp + u * kStepWarps < a.position) attend(warp + u * kStepWarps, k_ahead[u]);
+#pragma unroll 8
+  for (int t = warp + kAhead * kStepWarps; t < a.position; t += kStepWarps) {
+    float k[kPer];
+    load_row<kPer, KV_BF16>(a.k_cache, static_cast<size_t>(t) * a.token_stride + row0, k);
+    attend(t, k);
   }
   if (warp == a.position % kStepWarps) {   // the new token, as the cache holds it
     float dot = 0.0f;
@@ -181,8 +206,15 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
   float acc[kPer];
 #pragma unroll
   for (int i = 0; i < kPer; ++i) acc[i] = 0.0f;
-#pragma unroll 4
-  for (int t = warp; t < a.position; t += kStepWarps) {
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (warp + u * kStepWarps < a.position) {
+      const float p = score[warp + u * kStepWarps];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) acc[i] = fmaf(p, v_ahead[u][i], acc[i]);
+    }
+#pragma unroll 8
+  for (int t = warp + kAhead * kStepWarps; t < a.position; t += kStepWarps) {
     float v[kPer];
     load_row<kPer, KV_BF16>(a.v_cache, static_cast<size_t>(t) * a.token_stride + row0, v);
     const float p = score[t];
@@ -226,18 +258,27 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
   __shared__ float4 column[16][kDim / 4];  // per-warp column sums
   __shared__ float delta_s[kDim], gates[2], red[4];
 
+  // weights before the wait, everything that a kernel of the stream writes after it
+  const int part = tid / kDim, i = tid % kDim;   // threads 0..383: one channel of q, k, v each
+  const int channel = part == 2 ? 2 * a.key_heads * kDim + h * kDim + i : (part * a.key_heads + kh) * kDim + i;
+  float w[kMaxTaps], norm = 0.0f;
+  if (tid < 3 * kDim) {
+#pragma unroll
+    for (int tap = 0; tap < kMaxTaps; ++tap)
+      w[tap] = tap < a.width ? a.conv_weight[static_cast<size_t>(channel) * a.width + tap] : 0.0f;
+    if (part == 0) norm = a.norm_weight[i];
+  }
+  pdl_wait();
+  pdl_launch_dependents();
   float4 S[8];
   float* state = a.state + static_cast<size_t>(h) * kDim * kDim + warp * 8 * kDim + lane * 4;
 #pragma unroll
   for (int r = 0; r < 8; ++r) S[r] = *reinterpret_cast<const float4*>(state + r * kDim);
 
-  const int part = tid / kDim, i = tid % kDim;   // threads 0..383: one channel of q, k, v each
-  const int channel = part == 2 ? 2 * a.key_heads * kDim + h * kDim + i : (part * a.key_heads + kh) * kDim + i;
   float window[kMaxTaps];
-  float z = 0.0f, norm = 0.0f;
+  float z = 0.0f;
   if (tid < 3 * kDim) {
     const float* own = a.conv_state + static_cast<size_t>(channel) * a.width;
-    const float* w = a.conv_weight + static_cast<size_t>(channel) * a.width;
     float sum = 0.0f;
 #pragma unroll
     for (int tap = 0; tap < kMaxTaps; ++tap) {
@@ -252,7 +293,6 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
     qkv[part][i] = rnd(sum / (1.0f + expf(-sum)), a.round);
     if (part == 0) {   // the threads that finish the row
       z = load_any(a.z, static_cast<size_t>(h) * kDim + i, a.z_is_bf16);
-      norm = a.norm_weight[i];
     }
   } else if (tid == 3 * kDim) {
     const float alpha = load_any(a.a_in, h, a.ab_is_bf16) + a.dt_bias[h];
@@ -343,8 +383,16 @@ cudaError_t cached_step(cudaStream_t stream, const CachedStepArgs& a) {
   static const Kernel kernels[3][2] = {{cached_step_kernel<2, false>, cached_step_kernel<2, true>},
                                        {cached_step_kernel<4, false>, cached_step_kernel<4, true>},
                                        {cached_step_kernel<8, false>, cached_step_kernel<8, true>}};
-  kernels[a.head_dim / 128][a.kv_is_bf16 ? 1 : 0]<<<a.q_heads, kStepWarps * 32, 0, stream>>>(a);
-  return cudaGetLastError();
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(a.q_heads);
+  config.blockDim = dim3(kStepWarps * 32);
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernels[a.head_dim / 128][a.kv_is_bf16 ? 1 : 0], a);
 }
 
 bool gdn_token_supported(int key_heads, int value_heads, int key_dim, int value_dim, int width) {
@@ -352,16 +400,18 @@ bool gdn_token_supported(int key_heads, int value_heads, int key_dim, int value_
 }
 
 cudaError_t gdn_token(cudaStream_t stream, const GdnTokenArgs& a) {
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = static_cast<unsigned>(a.value_heads / a.key_heads);
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = static_cast<unsigned>(a.value_heads / a.key_heads);
+  attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(a.value_heads);
   config.blockDim = dim3(kTokenThreads);
   config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
   return cudaLaunchKernelEx(&config, gdn_token_kernel, a);
 }
 

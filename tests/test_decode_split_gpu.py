@@ -1,0 +1,59 @@
+"""Tensor-core decode in its two forms (parts of a cluster; chunks + merge kernel) and at all three
+head widths against float64, with lengths at the edges of the 64-token tiles and of the parts: one
+token, fewer tokens than parts, and part boundaries."""
+import math
+
+import pytest
+import torch
+
+from pluto_b200 import _capi
+from pluto_b200.layers import gqa_decode
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch,hq,hkv,dim,longest", [
+    # 256 MB of cache at most: one launch, 1 to 16 parts; more: chunks and the merge kernel
+    (1, 24, 4, 256, 1), (5, 24, 4, 256, 130), (2, 24, 4, 256, 4096), (40, 8, 4, 256, 300), (17, 24, 4, 256, 4000),
+    (1, 40, 8, 128, 64), (4, 40, 8, 128, 65), (7, 5, 1, 128, 2000), (40, 8, 8, 128, 500), (9, 40, 8, 128, 8200),
+    (1, 12, 12, 64, 63), (30, 12, 12, 64, 129), (6, 12, 12, 64, 1025), (1, 16, 1, 64, 8200), (12, 12, 12, 64, 8200)])
+@pytest.mark.parametrize("page", [0, 16, 64])
+def test_decode_matches_float64(batch, hq, hkv, dim, longest, page):
+    gen = torch.Generator(device="cuda").manual_seed(longest + dim)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    capacity = (longest + 63) // 64 * 64
+    k, v = rnd(batch, capacity, hkv, dim).bfloat16(), rnd(batch, capacity, hkv, dim).bfloat16()
+    q, gate = rnd(batch, hq, dim).bfloat16(), rnd(batch, hq, dim).bfloat16()
+    lens = torch.randint(1, longest + 1, (batch,), device="cuda", generator=gen, dtype=torch.int32)
+    lens[0] = longest
+    edges = [x for x in (1, 63, 64, 65, longest // 2, longest - 1) if 1 <= x <= longest]
+    for i, x in enumerate(edges[:batch - 1]):
+        lens[1 + i] = x
+    # rows past a sequence's end must not matter, whatever they hold
+    dead = torch.arange(capacity, device="cuda")[None, :] >= lens[:, None]
+    k[dead] = float("nan")
+    v[dead] = float("inf")
+    group = hq // hkv
+    kk = k.double().repeat_interleave(group, 2).masked_fill(dead[:, :, None, None], 0)
+    vv = v.double().repeat_interleave(group, 2).masked_fill(dead[:, :, None, None], 0)
+    s = torch.einsum("bhd,bthd->bht", q.double(), kk) / math.sqrt(dim)
+    s = s.masked_fill(dead[:, None, :], -math.inf)
+    want = torch.einsum("bht,bthd->bhd", torch.softmax(s, -1), vv)
+    table, pool_k, pool_v = None, k, v
+    if page:
+        blocks = capacity // page
+        table = torch.randperm(batch * blocks, device="cuda", generator=gen).to(torch.int32).view(batch, blocks)
+        pool_k, pool_v = (torch.empty(batch * blocks, page, hkv, dim, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        pool_k[table.reshape(-1).long()] = k.view(-1, page, hkv, dim)
+        pool_v[table.reshape(-1).long()] = v.view(-1, page, hkv, dim)
+    out = torch.empty(batch, hq, dim, device="cuda")
+    got, lse = gqa_decode(q, pool_k, pool_v, lens, longest, block_table=table, round_to_bfloat16=False, out=out, want_lse=True)
+    # P carries 2^-17 relative error into a weighted mean of N(0, 1) values; fp32 sums of up to 8200 terms
+    assert (got.double() - want).abs().max().item() < 4e-5
+    assert (lse.double() - torch.logsumexp(s, -1)).abs().max().item() < 2e-5
+    gated = gqa_decode(q, pool_k, pool_v, lens, longest, block_table=table, gate=gate)
+    expected = want.bfloat16().double() * torch.sigmoid(gate.double()).bfloat16().double()
+    # the core and the product can each fall on either side of a tie: one bf16 ulp (at most 2^-7) apiece
+    assert ((gated.double() - expected).abs() <= 2 ** -6 * expected.abs() + 4e-5).all()
+    assert torch.equal(gated, gqa_decode(q, pool_k, pool_v, lens, longest, block_table=table, gate=gate))
+    assert _capi.kernel_status() == 0
