@@ -75,14 +75,13 @@ __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStep
   const int length = a.position + 1, half = a.rotary / 2;
   const size_t row0 = static_cast<size_t>(kv_head) * D + c0;
 
-  // What no kernel of a decoding stream writes may be read before the wait; everything else after it.
+  pdl_wait();   // every input, the weights too: the kernel before this one may have written them
+  pdl_launch_dependents();   // the next launch sets itself up meanwhile and waits for this grid in turn
   float w_norm[kPer];
   if (warp < 2) {
 #pragma unroll
     for (int i = 0; i < kPer; ++i) w_norm[i] = 1.0f + (warp == 0 ? a.q_norm : a.k_norm)[c0 + i];
   }
-  pdl_wait();
-  pdl_launch_dependents();   // the next launch sets itself up meanwhile and waits for this grid in turn
   // The first rows of the cache and the gate of this thread's output channel are requested before
   // anything waits: at short contexts the kernel is a chain of memory round trips.
   constexpr int kAhead = 2;
@@ -258,7 +257,8 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
   __shared__ float4 column[16][kDim / 4];  // per-warp column sums
   __shared__ float delta_s[kDim], gates[2], red[4];
 
-  // weights before the wait, everything that a kernel of the stream writes after it
+  pdl_wait();   // every input, the weights too: the kernel before this one may have written them
+  pdl_launch_dependents();
   const int part = tid / kDim, i = tid % kDim;   // threads 0..383: one channel of q, k, v each
   const int channel = part == 2 ? 2 * a.key_heads * kDim + h * kDim + i : (part * a.key_heads + kh) * kDim + i;
   float w[kMaxTaps], norm = 0.0f;
@@ -268,8 +268,6 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
       w[tap] = tap < a.width ? a.conv_weight[static_cast<size_t>(channel) * a.width + tap] : 0.0f;
     if (part == 0) norm = a.norm_weight[i];
   }
-  pdl_wait();
-  pdl_launch_dependents();
   float4 S[8];
   float* state = a.state + static_cast<size_t>(h) * kDim * kDim + warp * 8 * kDim + lane * 4;
 #pragma unroll
