@@ -118,7 +118,12 @@ int pluto_attn_bwd(pluto_stream_t stream, const void* qkv, const void* out, cons
   if (!normalizers) return fail(PLUTO_E_INVALID, "attention backward requires the saved normalizers");
   if (!d_out || !d_qkv || !deltas)
     return fail(PLUTO_E_INVALID, "attention backward requires non-null gradient pointers");
-  if (workspace != nullptr) {
+  // Head width 256 needs no workspace where the tensor-core kernels do not apply: a caller that sized
+  // its scratch for other layers, or whose tensors are not 16-byte aligned, gets the exact kernels.
+  const bool wide_ok = workspace_bytes >= pluto_attn_bwd_workspace_bytes(batch, seq, heads, head_dim, dtype) &&
+                       (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 && aligned16(qkv) && aligned16(d_qkv) &&
+                       aligned16(out) && aligned16(d_out);
+  if (workspace != nullptr && (head_dim != 256 || dtype != PLUTO_BF16 || wide_ok)) {
     const size_t need = pluto_attn_bwd_workspace_bytes(batch, seq, heads, head_dim, dtype);
     if (need == 0)
       return fail(PLUTO_E_INVALID, "attention backward has no tensor-core path for this shape; pass a null workspace");
@@ -254,8 +259,11 @@ int pluto_gqa_prefill_bwd(pluto_stream_t stream, const void* q, const void* k, c
       q_token_stride < (static_cast<size_t>(q_heads) - 1) * q_head_stride + head_dim)
     return fail(PLUTO_E_INVALID, "attention query strides overlap");
   const size_t D = head_dim, qd = static_cast<size_t>(q_heads) * D, kd = static_cast<size_t>(kv_heads) * D;
-  // bf16 tensors of head width 64/128 with a dense query run on tcgen05 when a workspace is given
-  if (workspace != nullptr && tensor_core_shape(head_dim, dtype) && q_head_stride == D &&
+  // bf16 tensors of head width 64/128/256 with a dense query run on tcgen05 when a workspace is given;
+  // at width 256 a workspace that is too small or gradients off a 16-byte boundary mean the exact kernels
+  const bool wide_ok = head_dim != 256 || (workspace_bytes >= bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim) &&
+                                           aligned16(dq) && aligned16(dk) && aligned16(dv));
+  if (workspace != nullptr && wide_ok && tensor_core_shape(head_dim, dtype) && q_head_stride == D &&
       q_token_stride % 8 == 0 && q_token_stride <= 0x7fffffffu && aligned16(q) && aligned16(k) &&
       aligned16(v) && aligned16(dc) && aligned16(workspace)) {
     if (workspace_bytes < bwd_tc_workspace_bytes(batch, seq, q_heads, head_dim))

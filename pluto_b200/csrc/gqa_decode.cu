@@ -679,7 +679,10 @@ bool make_pool_map(CUtensorMap* map, const void* base, const DecodeArgs& a, int 
 
 }  // namespace
 
+// (Head width 256 with fp32 results that nothing rounds keeps the plain kernel: the two bf16 parts of a
+// probability carry 16 bits, which a bf16 result cannot tell from 24 but an fp32 one can.)
 bool gqa_decode_uses_tensor_cores(const DecodeArgs& a) {
+  if (a.head_dim == 256 && !a.round && !a.out_is_bf16) return false;
   const int group = a.q_heads / a.kv_heads;
   const int pages = a.block_table ? a.num_pages : a.batch;
   return a.k_bases == nullptr && a.kv_is_bf16 && (a.head_dim == 64 || a.head_dim == 128 || a.head_dim == 256) && group <= 16 &&

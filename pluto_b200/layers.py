@@ -399,11 +399,13 @@ class KeyValueCache:
         self.position_ = 0  # contents are not cleared, as in the reference
 
     def packed_layout(self) -> bytes:
-        """struct pluto_kv_cache of this cache, for the vectorcall binding; the buffers never move."""
-        if self.packed_ is None:
+        """struct pluto_kv_cache of this cache, for the vectorcall binding; packed again when the buffers
+        have moved."""
+        where = (self.keys_.data_ptr(), self.values_.data_ptr(), self.keys_.dtype)
+        if self.packed_ is None or self.packed_[0] != where:
             row = self.key_value_heads_ * self.head_dim_
-            self.packed_ = _pack_cache(self.keys_, self.values_, None, self.capacity_, self.capacity_ * row, row)
-        return self.packed_
+            self.packed_ = where, _pack_cache(self.keys_, self.values_, None, self.capacity_, self.capacity_ * row, row)
+        return self.packed_[1]
 
     def layout(self) -> "_capi.KvCacheStruct":
         return kv_layout(self.keys_, self.values_, None, self.capacity_,
