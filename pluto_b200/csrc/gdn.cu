@@ -176,7 +176,7 @@ __global__ void gdn_gates_kernel(const void* a_in, const void* b_in, const float
 // sequence).  y_t = R(SiLU(R(sum_tap w[c][tap] * x[t + tap - width + 1]))) with inputs rounded
 // first; on return the state holds the last `width` inputs of this call (the reference's
 // shift register).  One thread per (batch, channel), sequential in t: windows wider than four
-// taps, channel counts that are not a multiple of four, and single tokens.
+// taps, channel counts that are not a multiple of four, single tokens, and output over the input.
 __global__ void gdn_conv_kernel(const void* input, const float* weight, int in_is_bf16, int batch,
                                 int tokens, int channels, int width, int round, float* state,
                                 void* output, int out_is_bf16) {
@@ -398,8 +398,12 @@ cudaError_t gdn_conv(cudaStream_t stream, const void* input, const float* weight
                      int batch, int tokens, int channels, int width, int round, float* state,
                      void* output, int out_is_bf16) {
   // four-tap windows and shorter over several tokens: cut along the tokens (a single token has
-  // nothing to cut, and grid.y / grid.z bound what one launch can hold)
-  if (width >= 2 && width <= 4 && tokens > 1 && channels % 4 == 0 && batch <= 65535 &&
+  // nothing to cut, and grid.y / grid.z bound what one launch can hold; in place, a segment's history
+  // would already be the segment before's output, so a thread then walks all tokens)
+  const size_t elements = static_cast<size_t>(batch) * tokens * channels;
+  const uintptr_t in0 = reinterpret_cast<uintptr_t>(input), out0 = reinterpret_cast<uintptr_t>(output);
+  const bool apart = in0 + elements * (in_is_bf16 ? 2 : 4) <= out0 || out0 + elements * (out_is_bf16 ? 2 : 4) <= in0;
+  if (apart && width >= 2 && width <= 4 && tokens > 1 && channels % 4 == 0 && batch <= 65535 &&
       (tokens + kConvSegment - 1) / kConvSegment <= 65535 && aligned_to(input, in_is_bf16 ? 8 : 16) &&
       aligned_to(output, out_is_bf16 ? 8 : 16)) {
     auto launch = width == 4 ? launch_conv_segments<4> : width == 3 ? launch_conv_segments<3> : launch_conv_segments<2>;
