@@ -138,6 +138,7 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   constexpr int kParts = kChannelParts<D>, kWarps = kTokenWarps * kParts;
   static_assert((kWarps + 1) * 32 == kDecodeThreads, "warps");
   constexpr int kOwnBlocks = D / 16 / kParts;     // 16-channel blocks of the accumulator a warp owns
+  constexpr bool kThirds = D == 256;              // P in three bf16 parts
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -296,36 +297,39 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           s[nb][i] = token < end ? (s[nb][i] + s_odd[nb][i]) * scale_log2 : -INFINITY;
           tile_max[i >> 1] = fmaxf(tile_max[i >> 1], s[nb][i]);
         }
-      // P is split into a bf16 high part and a bf16 remainder so that P V keeps ~16 mantissa
-      // bits: the result then tracks the fp32 reference to ~1e-5 instead of a bf16 ulp, and the
-      // extra MMAs are free in a bandwidth-bound kernel.
-      uint32_t pf[4], pl[4];
+      // P enters P V as a bf16 high part and a bf16 remainder, 16 bits, at head width 256 as a second
+      // remainder too, 24 bits; the extra MMAs are free in a bandwidth-bound kernel.
+      uint32_t pf[4], pl[4], pt[4];
+      float correction[2];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 1));
         tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 2));
         const float m_new = fmaxf(m_run[r], tile_max[r]);
         const float m_safe = m_new == -INFINITY ? 0.0f : m_new;
-        const float correction = fast_exp2(m_run[r] - m_safe);
+        correction[r] = fast_exp2(m_run[r] - m_safe);
         const float p00 = fast_exp2(s[0][2 * r] - m_safe), p01 = fast_exp2(s[0][2 * r + 1] - m_safe);
         const float p10 = fast_exp2(s[1][2 * r] - m_safe), p11 = fast_exp2(s[1][2 * r + 1] - m_safe);
         float sum = p00 + p01 + p10 + p11;
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        l_run[r] = l_run[r] * correction + sum;
+        l_run[r] = l_run[r] * correction[r] + sum;
         m_run[r] = m_new;
         pf[r] = pack_bf16(p00, p01);      // a0 / a1: tokens 0-7
         pf[2 + r] = pack_bf16(p10, p11);  // a2 / a3: tokens 8-15
-        pl[r] = pack_bf16(p00 - bf16_lo(pf[r]), p01 - bf16_hi(pf[r]));
-        pl[2 + r] = pack_bf16(p10 - bf16_lo(pf[2 + r]), p11 - bf16_hi(pf[2 + r]));
-#pragma unroll
-        for (int nb = 0; nb < 2 * kOwnBlocks; ++nb) {
-          o[nb][2 * r] *= correction;
-          o[nb][2 * r + 1] *= correction;
+        const float r00 = p00 - bf16_lo(pf[r]), r01 = p01 - bf16_hi(pf[r]);
+        const float r10 = p10 - bf16_lo(pf[2 + r]), r11 = p11 - bf16_hi(pf[2 + r]);
+        pl[r] = pack_bf16(r00, r01);
+        pl[2 + r] = pack_bf16(r10, r11);
+        if (kThirds) {
+          pt[r] = pack_bf16(r00 - bf16_lo(pl[r]), r01 - bf16_hi(pl[r]));
+          pt[2 + r] = pack_bf16(r10 - bf16_lo(pl[2 + r]), r11 - bf16_hi(pl[2 + r]));
         }
       }
-      // ---- O += P V over this warp's channels; the high-part products of two blocks before their
-      // remainders, so that no product waits for the one just issued
+      // ---- O = O * correction + P V over this warp's channels; the high-part products of two blocks
+      // before their remainders, so that no product waits for the one just issued.  Every tile starts
+      // from zero and is added in fp32: the tensor cores truncate when they accumulate, and over the
+      // hundreds of tiles of a long sequence that would add up.
 #pragma unroll
       for (int np = 0; np < kOwnBlocks; np += 2) {
         uint32_t vf[2][4];
@@ -336,10 +340,19 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           const int chunk = (block * 2 + lane / 16) % 8;
           ldmatrix_x4_trans(vf[u], v_tile + (block / 4) * kHalfBytes + row * 128 + ((chunk ^ (row % 8)) * 16));
         }
+        float pv[4][4] = {};
 #pragma unroll
-        for (int u = 0; u < 4; ++u) mma_bf16(o[2 * np + u], pf, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
+        for (int u = 0; u < 4; ++u) mma_bf16(pv[u], pf, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) mma_bf16(o[2 * np + u], pl, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
+        for (int u = 0; u < 4; ++u) mma_bf16(pv[u], pl, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
+        if (kThirds) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mma_bf16(pv[u], pt, vf[u / 2][(u & 1) * 2], vf[u / 2][(u & 1) * 2 + 1]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o[2 * np + u][i] = fmaf(o[2 * np + u][i], correction[i >> 1], pv[u][i]);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar->empty[st]);
