@@ -590,68 +590,76 @@ linear_gemv_mma(const void* __restrict__ weights, const float* __restrict__ scal
 }
 
 // ------------------------------------------------------------------------------------------------
-// FP8 weights, one to four tokens, cols % 256 == 0: the streaming ring feeding the tensor cores.
+// FP8 weights, up to eight tokens, cols % 256 == 0: the streaming ring feeding the tensor cores.
 // The FMA form above spends its time converting E4M3 to fp32 (its slope is 4.1 TB/s); an
-// m16n8k32 E4M3 MMA takes the codes as they are.  A slab is 4 (2, 1) weight rows in one contiguous
-// piece of memory, so the MMA is laid out around that: every row is cut into two halves of
-// cols / 2, the 8 columns of the B operand are the 8 (row, half) pieces, and the rows of the A
-// operand are the (token, half) pieces of the quantised activation.  D[(t, h)][(r, h')] is the
-// dot product of token t's half h with row r's half h'; only h == h' means anything, and
-// y[t][r] = D[(t,0)][(r,0)] + D[(t,1)][(r,1)].  Half of the tensor work is thrown away, which
-// costs nothing here.  Every piece sits in shared memory at a stride of its length + 64 bytes,
-// which makes the fragments' 16-byte loads conflict-free, and a lane loads 16 consecutive bytes
-// at 16 * (lane % 4) of a 64-byte block on both sides, so the K order inside a block is the same
-// permutation for A and B.  Scales: each 128-column group's four MMAs go into a fresh
-// accumulator that is added with (weight block scale x activation group scale).
+// m16n8k32 E4M3 MMA takes the codes as they are.  A slab is 8 / P weight rows in one contiguous
+// piece of memory (P = 2, 4 or 8: long rows leave room for fewer in the ring), so the MMA is laid out
+// around that: every row is cut into P pieces of cols / P, the 8 columns of the B operand are the 8
+// (row, piece) pairs, and the 16 rows of the A operand are (token, piece) pairs of the quantised
+// activation, 16 / P tokens at most.  D[(t, h)][(r, h')] is the dot product of token t's piece h with
+// row r's piece h'; only h == h' means anything, and y[t][r] = sum over h of D[(t,h)][(r,h)].  The rest
+// of the tensor work is thrown away, which costs nothing here.  Every piece sits in shared memory at a
+// stride of its length + 64 bytes, which makes the fragments' 16-byte loads conflict-free, and a lane
+// loads 16 consecutive bytes at 16 * (lane % 4) of a 64-byte block on both sides, so the K order inside
+// a block is the same permutation for A and B.  Scales: each 128-column group's four MMAs go into a
+// fresh accumulator that is added with (weight block scale x activation group scale).
 // ------------------------------------------------------------------------------------------------
 constexpr int kPiecePad = 64;
+constexpr int kStreamMmaTokens = 8;
 
 struct StreamMmaLayout {
-  int stages, slab_rows, half;               // half = cols / 2
+  int stages, slab_rows, pieces, length;     // pieces per row, bytes per piece
   size_t piece_stride, slab_bytes, xs_offset, xscale_offset, partial_offset, bar_offset, total;
 };
-inline StreamMmaLayout stream_mma_layout(int cols, int tokens) {
-  StreamMmaLayout l;
-  l.half = cols / 2;
-  l.piece_stride = static_cast<size_t>(l.half) + kPiecePad;
-  const size_t xs_bytes = 2 * static_cast<size_t>(tokens) * l.piece_stride;
-  const size_t xscale_bytes = static_cast<size_t>(tokens) * (cols / 128) * 4;
-  const size_t partial_bytes = 2 * kWarps * 4 * kRows * 4;   // [buffer][warp][token][row]
-  const size_t tail = 2 * kStreamMaxStages * 8 + 4 * kGroups;
-  const size_t fixed = xs_bytes + xscale_bytes + partial_bytes + tail;
-  l.stages = 0;
+// The most rows per slab whose ring holds a slot per group beside the activation and which give every
+// CTA two slabs (`ctas` of them); stages == 0: the shape does not qualify.
+inline StreamMmaLayout stream_mma_layout(int cols, int rows, int tokens, int ctas) {
+  StreamMmaLayout l = {};
   for (l.slab_rows = kRows; l.slab_rows >= 1; l.slab_rows /= 2) {
-    l.slab_bytes = (2 * l.slab_rows * l.piece_stride + 1023) / 1024 * 1024;
+    l.pieces = 8 / l.slab_rows;
+    l.length = cols / l.pieces;
+    if (cols % (128 * l.pieces) != 0 || tokens * l.pieces > 16 || rows < 2 * l.slab_rows * ctas) continue;
+    l.piece_stride = static_cast<size_t>(l.length) + kPiecePad;
+    const size_t xs_bytes = static_cast<size_t>(tokens) * l.pieces * l.piece_stride;
+    const size_t xscale_bytes = static_cast<size_t>(tokens) * (cols / 128) * 4;
+    const size_t partial_bytes = 2 * kWarps * kStreamMmaTokens * kRows * 4;   // [buffer][warp][token][row]
+    const size_t tail = 2 * kStreamMaxStages * 8 + 4 * kGroups;
+    const size_t fixed = xs_bytes + xscale_bytes + partial_bytes + tail + 8;
+    l.slab_bytes = (8 * l.piece_stride + 1023) / 1024 * 1024;
+    l.stages = 0;
     if (fixed < static_cast<size_t>(kStreamBudget))
       l.stages = static_cast<int>(std::min<size_t>(kStreamMaxStages, (kStreamBudget - fixed) / l.slab_bytes)) /
                  kGroups * kGroups;
-    if (l.stages > 0) break;
+    if (l.stages == 0) continue;
+    l.xs_offset = l.stages * l.slab_bytes;
+    l.xscale_offset = l.xs_offset + xs_bytes;
+    l.partial_offset = l.xscale_offset + xscale_bytes;
+    l.bar_offset = (l.partial_offset + partial_bytes + 7) / 8 * 8;
+    l.total = l.bar_offset + tail;
+    return l;
   }
-  if (l.stages == 0) l.slab_rows = kRows;
-  l.xs_offset = l.stages * l.slab_bytes;
-  l.xscale_offset = l.xs_offset + xs_bytes;
-  l.partial_offset = l.xscale_offset + xscale_bytes;
-  l.bar_offset = (l.partial_offset + partial_bytes + 7) / 8 * 8;
-  l.total = l.bar_offset + tail;
+  l.stages = 0;
   return l;
 }
 
+template <int P, bool second>   // second: tokens of the A rows 8 to 15 (tokens * P > 8)
 __global__ void __launch_bounds__(kThreads + 32, 2)
 linear_gemv_stream_e4m3(const uint8_t* __restrict__ weights, const float* __restrict__ scales,
                         const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int cols,
                         int rows, int tokens, StreamMmaLayout layout, uint32_t* status) {
+  constexpr int kSlabRows = 8 / P;
   extern __shared__ __align__(1024) uint8_t stream_smem[];
   uint8_t* ring = stream_smem;
-  uint8_t* xs = stream_smem + layout.xs_offset;                                   // [token][half][piece]
+  uint8_t* xs = stream_smem + layout.xs_offset;                                   // [token][piece]
   float* xscale = reinterpret_cast<float*>(stream_smem + layout.xscale_offset);   // [token][cols / 128]
   float* partial = reinterpret_cast<float*>(stream_smem + layout.partial_offset);
   uint64_t* full = reinterpret_cast<uint64_t*>(stream_smem + layout.bar_offset);
   uint64_t* empty = full + kStreamMaxStages;
   int* failed = reinterpret_cast<int*>(empty + kStreamMaxStages);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int stages = layout.stages, slab_rows = layout.slab_rows, half = layout.half;
+  const int stages = layout.stages, length = layout.length;
   const size_t stride = layout.piece_stride;
-  const int n_tasks = (rows + slab_rows - 1) / slab_rows;
+  const int n_tasks = (rows + kSlabRows - 1) / kSlabRows;
   const int groups128 = cols / 128;
 
   pdl_launch_dependents();
@@ -665,16 +673,16 @@ linear_gemv_stream_e4m3(const uint8_t* __restrict__ weights, const float* __rest
   }
   __syncthreads();
 
-  // slab n of this CTA = task blockIdx.x + n * gridDim.x; piece 2 r + h = half h of its row r
+  // slab n of this CTA = task blockIdx.x + n * gridDim.x; piece P r + h = piece h of its row r
   auto issue = [&](int n) {
     const int task = blockIdx.x + n * gridDim.x;
     const int st = n % stages;
-    const int rows_here = min(slab_rows, rows - task * slab_rows);
+    const int rows_here = min(kSlabRows, rows - task * kSlabRows);
     mbar_expect_tx(&full[st], static_cast<uint32_t>(rows_here) * cols);
-    const uint8_t* src = weights + static_cast<size_t>(task) * slab_rows * cols;
+    const uint8_t* src = weights + static_cast<size_t>(task) * kSlabRows * cols;
     uint8_t* dst = ring + st * layout.slab_bytes;
-    for (int piece = 0; piece < 2 * rows_here; ++piece)
-      bulk_load(dst + piece * stride, src + static_cast<size_t>(piece) * half, half, &full[st]);
+    for (int piece = 0; piece < P * rows_here; ++piece)
+      bulk_load(dst + piece * stride, src + static_cast<size_t>(piece) * length, length, &full[st]);
   };
   const int my_tasks = blockIdx.x < n_tasks ? (n_tasks - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
@@ -689,7 +697,7 @@ linear_gemv_stream_e4m3(const uint8_t* __restrict__ weights, const float* __rest
     return;
   }
 
-  // activation -> E4M3 codes per (token, half) piece + one scale per group of 128 (one warp a group)
+  // activation -> E4M3 codes per (token, piece) + one scale per group of 128 (one warp a group)
   pdl_wait();   // the previous kernel's output may be this activation
   {
     constexpr int kBatch = 5;   // groups whose 8-byte loads are in flight together
@@ -716,8 +724,8 @@ linear_gemv_stream_e4m3(const uint8_t* __restrict__ weights, const float* __rest
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           word |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(v[i] / divisor, __NV_SATFINITE, __NV_E4M3)) << (8 * i);
-        const int c = g * 128 + lane * 4, h = c / half;
-        *reinterpret_cast<uint32_t*>(xs + (2 * t + h) * stride + (c - h * half)) = word;
+        const int c = g * 128 + lane * 4, h = c / length;
+        *reinterpret_cast<uint32_t*>(xs + (P * t + h) * stride + (c - h * length)) = word;
         if (lane == 0) xscale[t * groups128 + g] = scale;
       }
     }
@@ -727,75 +735,97 @@ linear_gemv_stream_e4m3(const uint8_t* __restrict__ weights, const float* __rest
   const int group = warp / kGroupWarps, gwarp = warp % kGroupWarps;
   const int gthread = threadIdx.x % kGroupThreads;
   const int g = lane / 4, q = lane % 4;
-  // A row g = (token g / 2, half g % 2); B column g = piece g = (row g / 2, half g % 2);
-  // accumulator element i < 2 of this lane: A row g, B column 2 q + i = (row q, half i)
-  const int my_half = g & 1, my_token = g >> 1;
-  const bool a_valid = my_token < tokens;
+  // A rows g and g + 8 = (token g / P, piece g % P) and the same piece 8 / P tokens on; B column g =
+  // (row g / P, piece g % P).  Accumulator elements i and 2 + i of this lane: A rows g and g + 8, B
+  // column 2 q + i, whose piece matches this lane's in at most one i.
+  const int my_piece = g % P, token0 = g / P, token1 = token0 + 8 / P;
+  const bool match = my_piece / 2 == q % (P / 2);
+  const bool odd = my_piece & 1;
+  const int my_row = q / (P / 2);
   const uint8_t* a_ptr = xs + g * stride + q * 16;
-  const int half_groups = half / 128;
-  const float* my_xscale = xscale + min(my_token, tokens - 1) * groups128 + my_half * half_groups;
+  const bool valid0 = token0 < tokens, valid1 = token1 < tokens;
+  const int piece_groups = length / 128;
+  const float* xscale0 = xscale + min(token0, tokens - 1) * groups128 + my_piece * piece_groups;
+  const float* xscale1 = xscale + min(token1, tokens - 1) * groups128 + my_piece * piece_groups;
   for (int n = group, turn = 0; n < my_tasks; n += kGroups, ++turn) {
-    const int task = blockIdx.x + n * gridDim.x, row0 = task * slab_rows, st = n % stages;
-    const int rows_here = min(slab_rows, rows - row0);
+    const int task = blockIdx.x + n * gridDim.x, row0 = task * kSlabRows, st = n % stages;
+    const int rows_here = min(kSlabRows, rows - row0);
     // the rows of a slab lie in one 128-row scale block (1, 2 and 4 divide 128)
-    const float* wscale = scales + static_cast<size_t>(row0 / 128) * groups128 + my_half * half_groups;
-    float total = 0.0f;
+    const float* wscale = scales + static_cast<size_t>(row0 / 128) * groups128 + my_piece * piece_groups;
+    float total0 = 0.0f, total1 = 0.0f;
     const bool ok = mbar_wait(&full[st], (n / stages) & 1, status, 43);
     if (!ok) *reinterpret_cast<volatile int*>(failed + group) = 1;
     if (ok) {
-      // columns past the slab's pieces (slabs of fewer than 4 rows) re-read its last piece; their
-      // results are never stored
-      const uint8_t* b_ptr = ring + st * layout.slab_bytes + min(g, 2 * slab_rows - 1) * stride + q * 16;
-      for (int kg = gwarp; kg < half_groups; kg += kGroupWarps) {
+      // (a last slab with fewer rows leaves older pieces in its other columns; they are never stored)
+      const uint8_t* b_ptr = ring + st * layout.slab_bytes + g * stride + q * 16;
+      for (int kg = gwarp; kg < piece_groups; kg += kGroupWarps) {
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int block = 0; block < 2; ++block) {
           const uint4 b = *reinterpret_cast<const uint4*>(b_ptr + kg * 128 + block * 64);
-          uint4 a = make_uint4(0u, 0u, 0u, 0u);
-          if (a_valid) a = *reinterpret_cast<const uint4*>(a_ptr + kg * 128 + block * 64);
-          mma_e4m3(acc, a.x, 0u, a.y, 0u, b.x, b.y);
-          mma_e4m3(acc, a.z, 0u, a.w, 0u, b.z, b.w);
+          uint4 a = make_uint4(0u, 0u, 0u, 0u), c = a;
+          if (valid0) a = *reinterpret_cast<const uint4*>(a_ptr + kg * 128 + block * 64);
+          if (second && valid1) c = *reinterpret_cast<const uint4*>(a_ptr + 8 * stride + kg * 128 + block * 64);
+          mma_e4m3(acc, a.x, c.x, a.y, c.y, b.x, b.y);
+          mma_e4m3(acc, a.z, c.z, a.w, c.w, b.z, b.w);
         }
-        // the element whose B half matches this lane's A half
-        total = fmaf(my_half ? acc[1] : acc[0], wscale[kg] * my_xscale[kg], total);
+        const float ws = wscale[kg];
+        total0 = fmaf(odd ? acc[1] : acc[0], ws * xscale0[kg], total0);
+        if (second) total1 = fmaf(odd ? acc[3] : acc[2], ws * xscale1[kg], total1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[st]);
     }
-    total += __shfl_xor_sync(0xffffffffu, total, 4);   // the two halves: lanes g and g ^ 1
+    // the pieces of a row: P lanes g, of each of which the one with the matching q counts
+    if (!match) total0 = total1 = 0.0f;
+#pragma unroll
+    for (int o = 1; o < P / 2; o <<= 1) {
+      total0 += __shfl_xor_sync(0xffffffffu, total0, o);
+      if (second) total1 += __shfl_xor_sync(0xffffffffu, total1, o);
+    }
+#pragma unroll
+    for (int o = 4; o < 4 * P; o <<= 1) {
+      total0 += __shfl_xor_sync(0xffffffffu, total0, o);
+      if (second) total1 += __shfl_xor_sync(0xffffffffu, total1, o);
+    }
     // [buffer][group][warp of the group][token][row]
-    float* mine = partial + (((turn & 1) * kGroups + group) * kGroupWarps) * 4 * kRows;
-    if (my_half == 0) mine[(gwarp * 4 + my_token) * kRows + q] = total;
+    float* mine = partial + (((turn & 1) * kGroups + group) * kGroupWarps) * kStreamMmaTokens * kRows;
+    if (my_piece == 0 && q % (P / 2) == 0) {
+      mine[(gwarp * kStreamMmaTokens + token0) * kRows + my_row] = total0;
+      if (second) mine[(gwarp * kStreamMmaTokens + token1) * kRows + my_row] = total1;
+    }
     asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kGroupThreads) : "memory");
     if (*reinterpret_cast<volatile int*>(failed + group)) break;   // same for the whole group
-    if (gthread < 4 * kRows) {
-      const int t = gthread / kRows, r = gthread % kRows;
-      float v = 0.0f;
+    if (gthread < kStreamMmaTokens * kSlabRows) {
+      const int t = gthread / kSlabRows, r = gthread % kSlabRows;
+      if (t < tokens && r < rows_here) {
+        float v = 0.0f;
 #pragma unroll
-      for (int w = 0; w < kGroupWarps; ++w) v += mine[(w * 4 + t) * kRows + r];
-      if (t < tokens && r < rows_here) y[static_cast<size_t>(t) * rows + row0 + r] = __float2bfloat16_rn(v);
+        for (int w = 0; w < kGroupWarps; ++w) v += mine[(w * kStreamMmaTokens + t) * kRows + r];
+        y[static_cast<size_t>(t) * rows + row0 + r] = __float2bfloat16_rn(v);
+      }
     }
   }
 }
 
-// Rows so long that only slabs of fewer than 4 rows fit the ring leave B columns unused and were
-// measured slower than the FMA form ([5120 x 8192]: 19.8 against 18.3 us), so they do not qualify.
-inline bool stream_mma_ok(const void* weights, const void* x, int cols, int rows, int tokens, int sms) {
-  if (tokens > 4 || cols % 256 != 0 || reinterpret_cast<uintptr_t>(weights) % 16 != 0 ||
-      reinterpret_cast<uintptr_t>(x) % 8 != 0 || rows < 2 * kRows * kStreamCtasPerSm * sms)
-    return false;
-  const StreamMmaLayout layout = stream_mma_layout(cols, tokens);
-  return layout.stages > 0 && layout.slab_rows == kRows;
+// Tokens of one pass over the weights, 0 if the shape does not qualify: all of them (of eight) if they
+// fit, else four.  Passes of fewer lose to the forms that take the batch in one (5120 x 10240, 4 tokens:
+// 47.3 us in passes of two against 43.7).
+inline int stream_mma_tokens(const void* weights, const void* x, int cols, int rows, int tokens, int sms) {
+  if (reinterpret_cast<uintptr_t>(weights) % 16 != 0 || reinterpret_cast<uintptr_t>(x) % 8 != 0) return 0;
+  const int all = std::min(tokens, kStreamMmaTokens), ctas = kStreamCtasPerSm * sms;
+  if (stream_mma_layout(cols, rows, all, ctas).stages > 0) return all;
+  return all > 4 && stream_mma_layout(cols, rows, 4, ctas).stages > 0 ? 4 : 0;
 }
 
-inline cudaError_t launch_stream_mma(cudaStream_t stream, const void* weights, const float* scales,
-                                     const void* x, void* y, int cols, int rows, int tokens, int sms) {
-  const StreamMmaLayout layout = stream_mma_layout(cols, tokens);
-  const cudaError_t e = cudaFuncSetAttribute(linear_gemv_stream_e4m3, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <int P, bool second>
+cudaError_t launch_stream_mma(cudaStream_t stream, const void* weights, const float* scales, const void* x, void* y,
+                              int cols, int rows, int tokens, int ctas, const StreamMmaLayout& layout) {
+  const cudaError_t e = cudaFuncSetAttribute(linear_gemv_stream_e4m3<P, second>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(layout.total));
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(kStreamCtasPerSm * sms);
+  config.gridDim = dim3(ctas);
   config.blockDim = dim3(kThreads + 32);
   config.dynamicSmemBytes = layout.total;
   config.stream = stream;
@@ -804,7 +834,7 @@ inline cudaError_t launch_stream_mma(cudaStream_t stream, const void* weights, c
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, linear_gemv_stream_e4m3, static_cast<const uint8_t*>(weights), scales,
+  return cudaLaunchKernelEx(&config, linear_gemv_stream_e4m3<P, second>, static_cast<const uint8_t*>(weights), scales,
                             static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), cols, rows,
                             tokens, layout, kernel_status_word());
 }
@@ -904,11 +934,18 @@ cudaError_t dispatch(cudaStream_t stream, const void* weights, const float* scal
     int sms = 148, device = 0;
     if (cudaGetDevice(&device) == cudaSuccess)
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (STORAGE == 2 && stream_mma_ok(weights, x, cols, rows, std::min(tokens, 4), sms)) {
-      for (int t0 = 0; t0 < tokens; t0 += 4) {
-        const cudaError_t e = launch_stream_mma(stream, weights, scales, xin + static_cast<size_t>(t0) * cols,
-                                                yout + static_cast<size_t>(t0) * rows, cols, rows,
-                                                std::min(4, tokens - t0), sms);
+    const int pass = STORAGE == 2 ? stream_mma_tokens(weights, x, cols, rows, tokens, sms) : 0;
+    if (pass > 0) {
+      const int ctas = kStreamCtasPerSm * sms;
+      for (int t0 = 0; t0 < tokens; t0 += pass) {
+        const int n = std::min(pass, tokens - t0);
+        const StreamMmaLayout layout = stream_mma_layout(cols, rows, n, ctas);   // fewer tokens fit wherever more do
+        const bool second = n * layout.pieces > 8;
+        auto run = layout.pieces == 2   ? (second ? launch_stream_mma<2, true> : launch_stream_mma<2, false>)
+                   : layout.pieces == 4 ? (second ? launch_stream_mma<4, true> : launch_stream_mma<4, false>)
+                                        : (second ? launch_stream_mma<8, true> : launch_stream_mma<8, false>);
+        const cudaError_t e = run(stream, weights, scales, xin + static_cast<size_t>(t0) * cols,
+                                  yout + static_cast<size_t>(t0) * rows, cols, rows, n, ctas, layout);
         if (e != cudaSuccess) return e;
       }
       return cudaSuccess;
