@@ -826,7 +826,7 @@ int check_dense(int rows, int input_dim, int output_dim, int dtype, const void* 
   if (dtype != PLUTO_FP32 && dtype != PLUTO_BF16)
     return fail(PLUTO_E_UNIMPLEMENTED, "dense layers compute in FP16 (fp32 activations) or BF16");
   if (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 != 0 ||
-      workspace_bytes < pluto_dense_workspace_bytes(rows, input_dim, output_dim))
+      workspace_bytes < pluto::dense_least_workspace_bytes(rows, input_dim, output_dim))
     return fail(PLUTO_E_INVALID, "dense layer workspace is missing, misaligned or too small");
   return PLUTO_OK;
 }
@@ -841,7 +841,7 @@ int pluto_dense_fwd(pluto_stream_t stream, const void* input, int dtype, const f
   uint32_t* status = pluto::kernel_status_word();
   if (!status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
   return from_cuda(pluto::dense_fwd(stream, input, dtype == PLUTO_BF16, matrix, bias, output, rows,
-                                    input_dim, output_dim, workspace, status),
+                                    input_dim, output_dim, workspace, workspace_bytes, status),
                    "DenseForwardKernel launch");
 }
 
@@ -856,7 +856,7 @@ int pluto_dense_bwd(pluto_stream_t stream, const void* input, int dtype, const f
   if (!status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
   return from_cuda(pluto::dense_bwd(stream, input, dtype == PLUTO_BF16, matrix, output_gradient,
                                     input_gradient, matrix_gradient, bias_gradient, rows, input_dim,
-                                    output_dim, workspace, status),
+                                    output_dim, workspace, workspace_bytes, status),
                    "dense backward launch");
 }
 
@@ -873,7 +873,7 @@ int check_block_linear(int tokens, int input_dim, int output_dim, const void* wo
       static_cast<long long>(tokens) * output_dim > 0x7fffffffLL)
     return fail(PLUTO_E_INVALID, "invalid block parameter dimensions, storage or executor");
   if (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 != 0 ||
-      workspace_bytes < pluto_block_linear_workspace_bytes(tokens, input_dim, output_dim))
+      workspace_bytes < pluto::block_linear_least_workspace_bytes(tokens, input_dim, output_dim))
     return fail(PLUTO_E_INVALID, "block linear workspace is missing, misaligned or too small");
   return PLUTO_OK;
 }
@@ -888,7 +888,7 @@ int pluto_block_linear_fwd(pluto_stream_t stream, const void* weight, const void
   uint32_t* status = pluto::kernel_status_word();
   if (!status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
   return from_cuda(pluto::block_linear_fwd(stream, weight, input, output, output_dtype == PLUTO_FP32,
-                                           tokens, input_dim, output_dim, workspace, status),
+                                           tokens, input_dim, output_dim, workspace, workspace_bytes, status),
                    "block linear forward");
 }
 
@@ -902,8 +902,7 @@ int pluto_block_linear_bwd(pluto_stream_t stream, const void* weight, const void
   uint32_t* status = pluto::kernel_status_word();
   if (!status) return fail(PLUTO_E_INTERNAL, "kernel status word unavailable");
   return from_cuda(pluto::block_linear_bwd(stream, weight, input, output_gradient, input_gradient,
-                                           weight_gradient, tokens, input_dim, output_dim, workspace,
-                                           status),
+                                           weight_gradient, tokens, input_dim, output_dim, workspace, workspace_bytes, status),
                    "block linear input gradient");
 }
 

@@ -294,22 +294,25 @@ cudaError_t linear_imported(cudaStream_t stream, const void* weights, int storag
                             const void* x, void* y, int tokens, int cols, int rows);
 
 // ---- gemm_sm100.cu: trainable dense projection (tcgen05 GEMMs over 2-byte casts of the operands) --
+// what a call needs at least, and what lets products of few tiles be cut along K
+size_t dense_least_workspace_bytes(int rows, int in, int out);
 size_t dense_workspace_bytes(int rows, int in, int out);
 cudaError_t dense_fwd(cudaStream_t stream, const void* x, bool x_is_bf16, const float* w,
                       const float* bias, void* y, int rows, int in, int out, void* workspace,
-                      uint32_t* status);
+                      size_t workspace_bytes, uint32_t* status);
 cudaError_t dense_bwd(cudaStream_t stream, const void* x, bool x_is_bf16, const float* w,
                       const float* dy, float* dx, float* dw, float* db, int rows, int in, int out,
-                      void* workspace, uint32_t* status);
+                      void* workspace, size_t workspace_bytes, uint32_t* status);
 
 // BlockLinearLayer: resident bf16 weight [out, in], bf16 x [tokens, in]; see gemm_sm100.cu
+size_t block_linear_least_workspace_bytes(int tokens, int in, int out);
 size_t block_linear_workspace_bytes(int tokens, int in, int out);
 cudaError_t block_linear_fwd(cudaStream_t stream, const void* weight, const void* x, void* y,
                              bool y_is_fp32, int tokens, int in, int out, void* workspace,
-                             uint32_t* status);
+                             size_t workspace_bytes, uint32_t* status);
 cudaError_t block_linear_bwd(cudaStream_t stream, const void* weight, const void* x, const float* dy,
                              float* dx, float* d_weight, int tokens, int in, int out, void* workspace,
-                             uint32_t* status);
+                             size_t workspace_bytes, uint32_t* status);
 // storage 1 = fp32, 2 = FP8 E4M3 with block scales -> bf16 [rows, cols]
 cudaError_t dequantize_matrix(cudaStream_t stream, const void* input, int storage, const float* scales,
                               long long rows, int cols, void* output);

@@ -46,6 +46,8 @@ struct GemmParams {
   size_t ldc;
   int c_kind;          // 0 fp32, 1 bf16
   uint32_t* status;
+  int splits = 1;           // the one-SM kernel's parts of K; part s of C goes to c + s * part_stride floats
+  size_t part_stride = 0;
 };
 
 struct GemmBarriers {
@@ -82,9 +84,9 @@ __device__ __forceinline__ void tile_origin(int tile, int m_tiles, int n_tiles, 
 // Ragged or unaligned blocks keep the row-per-thread stores.
 constexpr int kDrainStageBytes = 4 * 32 * 32 * 4;   // four epilogue warps
 __device__ __forceinline__ void drain_accumulator(uint32_t acc_tmem, int m0_warp, int lane, int n0,
-                                                  const GemmParams& p, uint32_t stage) {
-  const bool vec = (p.ldc % 4 == 0) && (reinterpret_cast<uintptr_t>(p.c) % 16 == 0);
-  const bool vec16 = p.ldc % 8 == 0 && reinterpret_cast<uintptr_t>(p.c) % 16 == 0;
+                                                  const GemmParams& p, void* c_out, uint32_t stage) {
+  const bool vec = (p.ldc % 4 == 0) && (reinterpret_cast<uintptr_t>(c_out) % 16 == 0);
+  const bool vec16 = p.ldc % 8 == 0 && reinterpret_cast<uintptr_t>(c_out) % 16 == 0;
   const int m = m0_warp + lane;
 #pragma unroll 2
   for (int c = 0; c < kTileN / 32; ++c) {
@@ -95,13 +97,15 @@ __device__ __forceinline__ void drain_accumulator(uint32_t acc_tmem, int m0_warp
     if (m0_warp >= p.M || n_base >= p.N) continue;   // (uniform over the warp)
     float v[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      v[i] = __uint_as_float(acc[i]);
-      if (p.bias != nullptr && n_base + i < p.N) v[i] += p.bias[n_base + i];
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]);
+    if (p.bias != nullptr) {   // a lane's column of the bias, handed round: one load in place of 32
+      const float own = n_base + lane < p.N ? p.bias[n_base + lane] : 0.0f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] += __shfl_sync(0xffffffffu, own, i);
     }
     const bool full = n_base + 32 <= p.N;
     if (p.c_kind == 0 && vec && full) {
-      float* block = static_cast<float*>(p.c) + static_cast<size_t>(m0_warp) * p.ldc + n_base;
+      float* block = static_cast<float*>(c_out) + static_cast<size_t>(m0_warp) * p.ldc + n_base;
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         sts_b32x4(stage + lane * 128 + ((i ^ (lane & 7)) << 4), __float_as_uint(v[4 * i]),
@@ -124,7 +128,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t acc_tmem, int m0_warp
       }
       __syncwarp();
     } else if (p.c_kind == 1 && vec16 && full) {
-      __nv_bfloat16* block = static_cast<__nv_bfloat16*>(p.c) + static_cast<size_t>(m0_warp) * p.ldc + n_base;
+      __nv_bfloat16* block = static_cast<__nv_bfloat16*>(c_out) + static_cast<size_t>(m0_warp) * p.ldc + n_base;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         sts_b32x4(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4), pack_bf16(v[8 * i], v[8 * i + 1]),
@@ -139,15 +143,18 @@ __device__ __forceinline__ void drain_accumulator(uint32_t acc_tmem, int m0_warp
       }
       __syncwarp();
     } else if (m < p.M) {
+      // (unrolled: a loop of unknown length over v would put it into local memory, on every path)
+      const int valid = p.N - n_base;
       if (p.c_kind == 0) {
-        float* dst = static_cast<float*>(p.c) + static_cast<size_t>(m) * p.ldc + n_base;
-        if (p.c_accumulate) {
-          for (int i = 0; i < 32 && n_base + i < p.N; ++i) v[i] += dst[i];
-        }
-        for (int i = 0; i < 32 && n_base + i < p.N; ++i) dst[i] = v[i];
+        float* dst = static_cast<float*>(c_out) + static_cast<size_t>(m) * p.ldc + n_base;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i < valid) dst[i] = p.c_accumulate ? v[i] + dst[i] : v[i];
       } else {
-        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.c) + static_cast<size_t>(m) * p.ldc + n_base;
-        for (int i = 0; i < 32 && n_base + i < p.N; ++i) dst[i] = __float2bfloat16_rn(v[i]);
+        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(c_out) + static_cast<size_t>(m) * p.ldc + n_base;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i < valid) dst[i] = __float2bfloat16_rn(v[i]);
       }
     }
   }
@@ -166,7 +173,8 @@ gemm_sm100(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   GemmBarriers* bar = reinterpret_cast<GemmBarriers*>(drain_stage + kDrainStageBytes);
   const int warp = uniform_warp_index(), lane = threadIdx.x % 32;
   const int m_tiles = (p.M + kTile - 1) / kTile, n_tiles = (p.N + kTileN - 1) / kTileN;
-  const int tiles = m_tiles * n_tiles;
+  const int tiles = m_tiles * n_tiles, units = tiles * p.splits;   // unit u: part u / tiles of tile u % tiles
+  auto first_step = [&](int part) { return static_cast<int>(static_cast<long long>(p.k_tiles) * part / p.splits); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGemmStages; ++s) {
@@ -198,10 +206,11 @@ gemm_sm100(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       tma_prefetch_desc(&map_b);
       bool ok = true;
       int it = 0;   // k-tile counter over all tiles of this CTA: the ring never restarts
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
         int m0, n0;
-        tile_origin(tile, m_tiles, n_tiles, m0, n0);
-        for (int kt = 0; kt < p.k_tiles && ok; ++kt, ++it) {
+        tile_origin(unit % tiles, m_tiles, n_tiles, m0, n0);
+        const int k_end = first_step(unit / tiles + 1);
+        for (int kt = first_step(unit / tiles); kt < k_end && ok; ++kt, ++it) {
           const int st = it % kGemmStages, use = it / kGemmStages;
           if (use > 0) ok = mbar_wait(&bar->empty[st], (use - 1) & 1, p.status, 70);
           if (!ok) break;
@@ -229,13 +238,14 @@ gemm_sm100(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   } else if (warp == 1) {
     bool ok = true;
     int it = 0, local = 0;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++local) {
+    for (int unit = blockIdx.x; unit < units && ok; unit += gridDim.x, ++local) {
+      const int k_begin = first_step(unit / tiles), k_end = first_step(unit / tiles + 1);
       const int buf = local & 1, use = local >> 1;
       if (use > 0)   // the epilogue has drained this accumulator's previous tile
         ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_empty[buf], (use - 1) & 1, p.status, 74));
       if (!ok) break;
       tc_fence_after();
-      for (int kt = 0; kt < p.k_tiles && ok; ++kt, ++it) {
+      for (int kt = k_begin; kt < k_end && ok; ++kt, ++it) {
         const int st = it % kGemmStages;
         ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[st], (it / kGemmStages) & 1, p.status, 72));
         if (!ok) break;
@@ -253,9 +263,9 @@ gemm_sm100(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll
           for (int ks = 0; ks < kBK / 16; ++ks)
             umma_ss(tmem + buf * kTileN, a_desc + ks * ((A_MN ? 2048 : 32) >> 4),
-                    b_desc + ks * ((B_MN ? 2048 : 32) >> 4), p.idesc, kt > 0 || ks > 0);
+                    b_desc + ks * ((B_MN ? 2048 : 32) >> 4), p.idesc, kt > k_begin || ks > 0);
           tc_commit(&bar->empty[st]);
-          if (kt + 1 == p.k_tiles) tc_commit(&bar->acc_full[buf]);
+          if (kt + 1 == k_end) tc_commit(&bar->acc_full[buf]);
         }
         __syncwarp();
       }
@@ -264,13 +274,14 @@ gemm_sm100(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     const int quarter = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     int local = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++local) {
       const int buf = local & 1;
       int m0, n0;
-      tile_origin(tile, m_tiles, n_tiles, m0, n0);
+      tile_origin(unit % tiles, m_tiles, n_tiles, m0, n0);
+      void* c = p.splits > 1 ? static_cast<float*>(p.c) + (unit / tiles) * p.part_stride : p.c;
       if (!mbar_wait(&bar->acc_full[buf], (local >> 1) & 1, p.status, 73)) break;
       tc_fence_after();
-      drain_accumulator(tmem + lane_base + buf * kTileN, m0 + quarter * 32, lane, n0, p,
+      drain_accumulator(tmem + lane_base + buf * kTileN, m0 + quarter * 32, lane, n0, p, c,
                         smem_u32(drain_stage) + quarter * (kDrainStageBytes / 4));
       // the accumulator has been read into registers by every lane of this warp
       tc_fence_before();
@@ -479,7 +490,7 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       pair_tile_origin(tile, m_tiles, n_tiles, m0, n0);
       if (!mbar_wait(&bar->acc_full[buf], (local >> 1) & 1, p.status, 79)) break;
       tc_fence_after();
-      drain_accumulator(tmem + lane_base + buf * kPairTile, m0 + rank * kTile + quarter * 32, lane, n0, p,
+      drain_accumulator(tmem + lane_base + buf * kPairTile, m0 + rank * kTile + quarter * 32, lane, n0, p, p.c,
                         smem_u32(drain_stage) + quarter * (kDrainStageBytes / 4));
       tc_fence_before();
       __syncwarp();
@@ -537,24 +548,54 @@ cast_pad_kernel(const In* __restrict__ src, uint16_t* __restrict__ dst, int rows
   *reinterpret_cast<uint4*>(dst + static_cast<size_t>(r) * cols_p + c) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Column sums of dy [rows, cols] in two fixed-order levels: CTA (x, y) sums rows y, y + gridDim.y,
-// ... of its 128 columns (a lane owns 4, the 8 warps split the rows and are added in warp order)
-// into partial[y][cols]; the second kernel adds the partial rows in order.
-constexpr int kBiasChunks = 16;
-__global__ void __launch_bounds__(256) bias_partial_kernel(const float* __restrict__ dy, int rows, int cols,
-                                                           float* __restrict__ partial) {
+// The upstream gradient's cast (as cast_pad_kernel, fp32 in) and its column sums from one reading of it:
+// CTA (x, y) takes the rows y * 8 + warp, + 8 gridDim.y, ... of its 128 columns, a lane four of them
+// and four rows at a time (one row in flight per warp and 16 chunks left three quarters of
+// the bandwidth unused; 16.5 us for 8192 x 2304 with the cast); the eight warps are added in order into partial[y][cols], the second kernel adds the
+// partial rows in order.
+constexpr int kBiasChunks = 64, kLeastBiasChunks = 16, kCastRows = 4;
+template <bool kHalf>
+__global__ void __launch_bounds__(256)
+cast_sum_kernel(const float* __restrict__ dy, uint16_t* __restrict__ dst, int rows, int cols, int rows_p, int cols_p,
+                float* __restrict__ partial) {
+  pdl_launch_dependents();   // the product behind this cast may set itself up meanwhile
   __shared__ float part[8][128];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int n = blockIdx.x * 128 + lane * 4;
+  const int n = blockIdx.x * 128 + lane * 4;   // (cols_p is a multiple of 128)
   float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  const bool vec = cols % 4 == 0 && reinterpret_cast<uintptr_t>(dy) % 16 == 0 && n + 4 <= cols;
-  for (int r = blockIdx.y * 8 + warp; r < rows; r += gridDim.y * 8) {
-    const float* p = dy + static_cast<size_t>(r) * cols + n;
-    if (vec) {
-      const float4 v = *reinterpret_cast<const float4*>(p);
-      sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
-    } else {
-      for (int i = 0; i < 4 && n + i < cols; ++i) sum[i] += p[i];
+  const bool vec = cols % 4 == 0 && reinterpret_cast<uintptr_t>(dy) % 16 == 0;
+  const int step = gridDim.y * 8;
+  for (int first = blockIdx.y * 8 + warp; first < rows_p; first += kCastRows * step) {
+    float v[kCastRows][4];
+#pragma unroll
+    for (int u = 0; u < kCastRows; ++u) {
+      const int r = first + u * step;
+      const float* p = dy + static_cast<size_t>(r) * cols + n;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[u][i] = 0.0f;
+      if (r < rows && vec && n < cols) {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        v[u][0] = f.x; v[u][1] = f.y; v[u][2] = f.z; v[u][3] = f.w;
+      } else if (r < rows) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (n + i < cols) v[u][i] = p[i];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kCastRows; ++u) {
+      const int r = first + u * step;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] += v[u][i];
+      if (r >= rows_p) continue;
+      uint2 w;
+      if (kHalf) {
+        const __half2 a = __floats2half2_rn(v[u][0], v[u][1]), b = __floats2half2_rn(v[u][2], v[u][3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      } else {
+        w = make_uint2(pack_bf16(v[u][0], v[u][1]), pack_bf16(v[u][2], v[u][3]));
+      }
+      *reinterpret_cast<uint2*>(dst + static_cast<size_t>(r) * cols_p + n) = w;
     }
   }
 #pragma unroll
@@ -577,14 +618,79 @@ __global__ void bias_final_kernel(const float* __restrict__ partial, int chunks,
 
 int pad128(int v) { return (v + 127) / 128 * 128; }
 
+// c [M][N] (row stride ldc; fp32 or bf16) = or += the sum of the parts [splits][M][N] in order, + bias.
+// One thread per four columns.
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ parts, GemmParams p) {
+  pdl_wait();
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  const int quads = p.N / 4;
+  if (i >= static_cast<long long>(p.M) * quads) return;
+  const int m = static_cast<int>(i / quads), n = static_cast<int>(i % quads) * 4;
+  float4 sum = *reinterpret_cast<const float4*>(parts + i * 4);
+  for (int s = 1; s < p.splits; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(parts + s * p.part_stride + i * 4);
+    sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+  }
+  if (p.bias != nullptr) {
+    sum.x += p.bias[n]; sum.y += p.bias[n + 1]; sum.z += p.bias[n + 2]; sum.w += p.bias[n + 3];
+  }
+  const size_t at = static_cast<size_t>(m) * p.ldc + n;
+  if (p.c_kind == 1) {
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.c) + at) =
+        make_uint2(pack_bf16(sum.x, sum.y), pack_bf16(sum.z, sum.w));
+    return;
+  }
+  float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.c) + at);
+  if (p.c_accumulate) {
+    const float4 old = *dst;
+    sum.x += old.x; sum.y += old.y; sum.z += old.z; sum.w += old.w;
+  }
+  *dst = sum;
+}
+
+// Parts of K for a product of few tiles on `sms` SMs.  In microseconds: a CTA takes 0.4 per K step and
+// about 2 to fill its pipeline and drain its tile; the parts cross L2 twice, at about 8 bytes/ps, and
+// their sum is one more launch.
+constexpr size_t kMaxPartBytes = size_t{96} << 20;
+int gemm_splits(int M, int N, int k_tiles, int sms) {
+  const long long tiles = static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + kTile - 1) / kTile);
+  const size_t part = static_cast<size_t>(M) * N * sizeof(float);
+  int best = 1;
+  double least = 1e30;
+  for (int z = 1; z <= 32 && z * 4 <= std::max(k_tiles, 4); ++z) {
+    if (z > 1 && (N % 4 != 0 || z * part > kMaxPartBytes)) break;
+    const double waves = static_cast<double>((tiles * z + sms - 1) / sms), steps = (k_tiles + z - 1) / z;
+    const double us = waves * (0.4 * steps + 2.0) + (z > 1 ? 3.0 + 2.0 * z * part / 8e6 : 0.0);
+    if (us < 0.95 * least) {
+      least = us;
+      best = z;
+    }
+  }
+  return best;
+}
+int sm_count() {
+  int sms = 148, device = 0;
+  if (cudaGetDevice(&device) == cudaSuccess)
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms;
+}
+// Scratch that launch_gemm can use for a product (0: it is not split).
+size_t gemm_part_bytes(int M, int N, int k_tiles) {
+  const int z = gemm_splits(M, N, k_tiles, sm_count());
+  return z > 1 ? z * static_cast<size_t>(M) * N * sizeof(float) : 0;
+}
+struct Scratch {   // for parts of K: 16-byte aligned, or none
+  void* base = nullptr;
+  size_t bytes = 0;
+};
+
 // b_pair: the B operand's map for the two-SM kernel (K-major B: boxes of 128 rows; MN-major B: the
 // same slab map as `b`), or null to keep the call on the one-SM kernel.
 template <bool A_MN, bool B_MN>
 cudaError_t launch_gemm(cudaStream_t stream, const CUtensorMap& a, const CUtensorMap& b,
-                        const GemmParams& p, const CUtensorMap* b_pair = nullptr) {
-  int sms = 148, device = 0;
-  if (cudaGetDevice(&device) == cudaSuccess)
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+                        const GemmParams& params, const CUtensorMap* b_pair = nullptr, Scratch scratch = {}) {
+  GemmParams p = params;
+  const int sms = sm_count();
   const int pair_tiles = ((p.N + kPairTile - 1) / kPairTile) * ((p.M + kPairTile - 1) / kPairTile);
   if (b_pair != nullptr && pair_tiles >= sms / 2) {   // enough 256 x 256 tiles to occupy every pair of SMs
     const size_t pair_smem =
@@ -611,7 +717,20 @@ cudaError_t launch_gemm(cudaStream_t stream, const CUtensorMap& a, const CUtenso
   cudaError_t e = cudaFuncSetAttribute(gemm_sm100<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  const int tiles = ((p.N + kTileN - 1) / kTileN) * ((p.M + kTile - 1) / kTile);
+  const int splits = gemm_splits(p.M, p.N, p.k_tiles, sms);
+  const size_t part = static_cast<size_t>(p.M) * p.N;
+  // (the sum writes four columns at a time)
+  const bool split = splits > 1 && scratch.bytes >= splits * part * sizeof(float) && p.ldc % 4 == 0 &&
+                     reinterpret_cast<uintptr_t>(p.c) % 16 == 0;
+  if (split) {
+    p.splits = splits;
+    p.part_stride = part;
+    p.c = scratch.base;
+    p.ldc = p.N;
+    p.c_kind = p.c_accumulate = 0;
+    p.bias = nullptr;
+  }
+  const int tiles = ((p.N + kTileN - 1) / kTileN) * ((p.M + kTile - 1) / kTile) * p.splits;
   cudaLaunchAttribute attribute;
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
@@ -622,7 +741,15 @@ cudaError_t launch_gemm(cudaStream_t stream, const CUtensorMap& a, const CUtenso
   config.stream = stream;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, gemm_sm100<A_MN, B_MN>, a, b, p);
+  e = cudaLaunchKernelEx(&config, gemm_sm100<A_MN, B_MN>, a, b, p);
+  if (e != cudaSuccess || !split) return e;
+  GemmParams out = params;
+  out.splits = splits;
+  out.part_stride = part;
+  config.gridDim = dim3(static_cast<unsigned>((part / 4 + 255) / 256));
+  config.blockDim = dim3(256);
+  config.dynamicSmemBytes = 0;
+  return cudaLaunchKernelEx(&config, sum_parts_kernel, static_cast<const float*>(scratch.base), out);
 }
 
 template <typename In>
@@ -655,24 +782,38 @@ cudaError_t activation_operand(cudaStream_t stream, const void* x, bool x_is_bf1
   return x_is_bf16 ? cast_pad<__nv_bfloat16>(stream, x, copy, rows, cols, false)
                    : cast_pad<float>(stream, x, copy, rows, cols, true);
 }
+Scratch rest_of(void* workspace, size_t bytes, size_t used) {   // `used` is a multiple of 16, the workspace aligned
+  if (bytes <= used) return {};
+  return {static_cast<uint8_t*>(workspace) + used, bytes - used};
+}
 bool operand_map(CUtensorMap* map, const Operand& t, int box_rows) {
   return make_token_map(map, t.base, t.cols, t.rows, 1, t.pitch, box_rows);
 }
 
 }  // namespace
 
+// The casts of X, W and dY and the bias partials; beyond that, parts of K for the products that have
+// too few tiles to fill the chip (a caller without that much gets them unsplit).
+size_t dense_least_workspace_bytes(int rows, int in, int out) {
+  const size_t r = pad128(rows), i = pad128(in), o = pad128(out);
+  return 2 * (r * i + i * o + r * o) + sizeof(float) * kLeastBiasChunks * o;
+}
 size_t dense_workspace_bytes(int rows, int in, int out) {
   const size_t r = pad128(rows), i = pad128(in), o = pad128(out);
-  return 2 * (r * i + i * o + r * o) + sizeof(float) * kBiasChunks * o;   // casts of X, W, dY; bias partials
+  const size_t parts = std::max(gemm_part_bytes(rows, out, static_cast<int>(i / kBK)),
+                                std::max(gemm_part_bytes(rows, in, static_cast<int>(o / kBK)),
+                                         gemm_part_bytes(in, out, static_cast<int>(r / kBK))));
+  return 2 * (r * i + i * o + r * o) + sizeof(float) * kBiasChunks * o + parts;
 }
 
 // x: [rows, in] bf16 (x_is_bf16) or fp32; w fp32 [in, out]; bias fp32 [out]; y same dtype as x.
 cudaError_t dense_fwd(cudaStream_t stream, const void* x, bool x_is_bf16, const float* w,
                       const float* bias, void* y, int rows, int in, int out, void* workspace,
-                      uint32_t* status) {
+                      size_t workspace_bytes, uint32_t* status) {
   const int r = pad128(rows), i = pad128(in), o = pad128(out);
   auto* xc = static_cast<uint8_t*>(workspace);
   auto* wc = xc + 2 * static_cast<size_t>(r) * i;
+  const Scratch scratch = rest_of(workspace, workspace_bytes, 2 * (static_cast<size_t>(r) * i + static_cast<size_t>(i) * o));
   const bool half = !x_is_bf16;
   Operand xo;
   cudaError_t e = activation_operand(stream, x, x_is_bf16, rows, in, xc, &xo);
@@ -685,22 +826,29 @@ cudaError_t dense_fwd(cudaStream_t stream, const void* x, bool x_is_bf16, const 
     return cudaErrorInvalidValue;
   GemmParams p{rows, out, i / kBK, i / kBK, i / kBK, 0, gemm_idesc(half ? 0 : 1, false, true), bias, y,
                static_cast<size_t>(out), x_is_bf16 ? 1 : 0, status};
-  return launch_gemm<false, true>(stream, ma, mb, p, &mb);
+  return launch_gemm<false, true>(stream, ma, mb, p, &mb, scratch);
 }
 
 // dy fp32 [rows, out]; dx fp32 [rows, in]; dw fp32 [in, out]; db fp32 [out] (all overwritten)
 cudaError_t dense_bwd(cudaStream_t stream, const void* x, bool x_is_bf16, const float* w,
                       const float* dy, float* dx, float* dw, float* db, int rows, int in, int out,
-                      void* workspace, uint32_t* status) {
+                      void* workspace, size_t workspace_bytes, uint32_t* status) {
   const int r = pad128(rows), i = pad128(in), o = pad128(out);
   auto* xc = static_cast<uint8_t*>(workspace);
   auto* wc = xc + 2 * static_cast<size_t>(r) * i;
   auto* gc = wc + 2 * static_cast<size_t>(i) * o;
+  float* partial = reinterpret_cast<float*>(gc + 2 * static_cast<size_t>(r) * o);
+  const size_t casts = static_cast<size_t>(reinterpret_cast<uint8_t*>(partial) - xc);
+  const int chunks = workspace_bytes >= casts + sizeof(float) * kBiasChunks * o ? kBiasChunks : kLeastBiasChunks;
+  const Scratch scratch = rest_of(workspace, workspace_bytes, casts + sizeof(float) * chunks * o);
   const bool half = !x_is_bf16;
   Operand xo;
   cudaError_t e = activation_operand(stream, x, x_is_bf16, rows, in, xc, &xo);
   if (e == cudaSuccess) e = cast_pad<float>(stream, w, wc, in, out, half);
-  if (e == cudaSuccess) e = cast_pad<float>(stream, dy, gc, rows, out, half);
+  if (e != cudaSuccess) return e;
+  auto cast = half ? cast_sum_kernel<true> : cast_sum_kernel<false>;
+  cast<<<dim3(o / 128, chunks), 256, 0, stream>>>(dy, reinterpret_cast<uint16_t*>(gc), rows, out, r, o, partial);
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int format = half ? 0 : 1;
   CUtensorMap ma, mb;
@@ -711,20 +859,16 @@ cudaError_t dense_bwd(cudaStream_t stream, const void* x, bool x_is_bf16, const 
     return cudaErrorInvalidValue;
   GemmParams pdx{rows, in, o / kBK, o / kBK, o / kBK, 0, gemm_idesc(format, false, false), nullptr, dx,
                  static_cast<size_t>(in), 0, status};
-  e = launch_gemm<false, false>(stream, ma, mb, pdx, &mb_pair);
+  e = launch_gemm<false, false>(stream, ma, mb, pdx, &mb_pair, scratch);
   if (e != cudaSuccess) return e;
   // dW[in, out] = X^T dY: A(m, k) = X[k][m], memory [rows][in] = MN-major; B = dY [rows][out] MN-major
   if (!operand_map(&ma, xo, kBK) || !make_token_map(&mb, gc, o, r, 1, o, kBK))
     return cudaErrorInvalidValue;
   GemmParams pdw{in, out, r / kBK, r / kBK, r / kBK, 0, gemm_idesc(format, true, true), nullptr, dw,
                  static_cast<size_t>(out), 0, status};
-  e = launch_gemm<true, true>(stream, ma, mb, pdw, &mb);
+  e = launch_gemm<true, true>(stream, ma, mb, pdw, &mb, scratch);
   if (e != cudaSuccess) return e;
-  float* partial = reinterpret_cast<float*>(gc + 2 * static_cast<size_t>(r) * o);
-  bias_partial_kernel<<<dim3((out + 127) / 128, kBiasChunks), 256, 0, stream>>>(dy, rows, out, partial);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  bias_final_kernel<<<(out + 255) / 256, 256, 0, stream>>>(partial, kBiasChunks, out, db);
+  bias_final_kernel<<<(out + 255) / 256, 256, 0, stream>>>(partial, chunks, out, db);
   return cudaGetLastError();
 }
 
@@ -802,15 +946,22 @@ cudaError_t bf16_operand(cudaStream_t stream, const void* x, int rows, int cols,
 
 }  // namespace
 
-size_t block_linear_workspace_bytes(int tokens, int in, int out) {
+size_t block_linear_least_workspace_bytes(int tokens, int in, int out) {
   const size_t t = pad128(tokens), i = pad128(in), o = pad128(out);
   return 2 * (t * i + o * i + 2 * t * o);   // copies of X and W (only if unaligned), hi/lo split of dY
+}
+size_t block_linear_workspace_bytes(int tokens, int in, int out) {   // and parts of K, as in dense_workspace_bytes
+  const int t = pad128(tokens), i = pad128(in), o = pad128(out);
+  return block_linear_least_workspace_bytes(tokens, in, out) +
+         std::max(gemm_part_bytes(tokens, out, i / kBK),
+                  std::max(gemm_part_bytes(tokens, in, 2 * (o / kBK)), gemm_part_bytes(out, in, 2 * (t / kBK))));
 }
 
 cudaError_t block_linear_fwd(cudaStream_t stream, const void* weight, const void* x, void* y,
                              bool y_is_fp32, int tokens, int in, int out, void* workspace,
-                             uint32_t* status) {
+                             size_t workspace_bytes, uint32_t* status) {
   const size_t t = pad128(tokens), i = pad128(in), o = pad128(out);
+  const Scratch scratch = rest_of(workspace, workspace_bytes, block_linear_least_workspace_bytes(tokens, in, out));
   auto* xc = static_cast<uint8_t*>(workspace);
   auto* wc = xc + 2 * t * i;
   Operand xo, wo;
@@ -823,13 +974,14 @@ cudaError_t block_linear_fwd(cudaStream_t stream, const void* weight, const void
   const int k_tiles = static_cast<int>(i / kBK);
   GemmParams p{tokens, out, k_tiles, k_tiles, k_tiles, 0, gemm_idesc(1, false, false), nullptr, y,
                static_cast<size_t>(out), y_is_fp32 ? 0 : 1, status};
-  return launch_gemm<false, false>(stream, ma, mb, p, &mb_pair);
+  return launch_gemm<false, false>(stream, ma, mb, p, &mb_pair, scratch);
 }
 
 cudaError_t block_linear_bwd(cudaStream_t stream, const void* weight, const void* x, const float* dy,
                              float* dx, float* d_weight, int tokens, int in, int out, void* workspace,
-                             uint32_t* status) {
+                             size_t workspace_bytes, uint32_t* status) {
   const size_t t = pad128(tokens), i = pad128(in), o = pad128(out);
+  const Scratch scratch = rest_of(workspace, workspace_bytes, block_linear_least_workspace_bytes(tokens, in, out));
   auto* xc = static_cast<uint8_t*>(workspace);
   auto* wc = xc + 2 * t * i;
   auto* gc = wc + 2 * o * i;
@@ -851,7 +1003,7 @@ cudaError_t block_linear_bwd(cudaStream_t stream, const void* weight, const void
   const int ko = static_cast<int>(o / kBK), kt = static_cast<int>(t / kBK);
   GemmParams pdx{tokens, in, 2 * ko, ko, ko, 0, gemm_idesc(1, false, true), nullptr, dx,
                  static_cast<size_t>(in), 0, status};
-  e = launch_gemm<false, true>(stream, ma, mb, pdx, &mb);
+  e = launch_gemm<false, true>(stream, ma, mb, pdx, &mb, scratch);
   if (e != cudaSuccess || d_weight == nullptr) return e;
   // dW[out, in] += dY^T X: A(m = r, k = t) = dY[t][r]: MN-major halves over tokens; B = X MN-major
   if (!make_token_map(&ma, gc, static_cast<int>(o), static_cast<int>(t), 2, o, kBK) ||
@@ -859,7 +1011,7 @@ cudaError_t block_linear_bwd(cudaStream_t stream, const void* weight, const void
     return cudaErrorInvalidValue;
   GemmParams pdw{out, in, 2 * kt, kt, kt, 1, gemm_idesc(1, true, true), nullptr, d_weight,
                  static_cast<size_t>(in), 0, status};
-  return launch_gemm<true, true>(stream, ma, mb, pdw, &mb);
+  return launch_gemm<true, true>(stream, ma, mb, pdw, &mb, scratch);
 }
 
 cudaError_t dequantize_matrix(cudaStream_t stream, const void* input, int storage, const float* scales,
