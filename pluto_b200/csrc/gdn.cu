@@ -226,16 +226,18 @@ __device__ __forceinline__ void store_four(void* p, size_t i, const float (&v)[4
 // with the window in registers.  It is a stream (every input and output element once), so what
 // counts is that there are enough threads to keep HBM busy: one thread per channel walked all
 // tokens of a sequence by itself, 80 CTAs of dependent loads (565 us at 1000 tokens x 10240
-// channels; 30 us in this form).  Segment 0 is the only reader of the state, so it also writes the
+// channels; 17 us in this form).  Segment 0 is the only reader of the state, so it also writes the
 // new one: it never races with a later segment, which takes its history from the input.
 constexpr int kConvSegment = 16;
 template <int W, bool IN_BF16, bool OUT_BF16>
-__global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* __restrict__ input,
+__global__ void __launch_bounds__(128, 8) gdn_conv_segment_kernel(const void* __restrict__ input,
                                                                const float* __restrict__ weight, int tokens,
                                                                int channels, int round, float* state,
                                                                void* __restrict__ output) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= channels) return;
+  // (a bf16 input is rounded already, and a bf16 output is rounded by its store)
+  auto rounded_in = [&](float v) { return IN_BF16 ? v : rnd(v, round); };
   const int b = blockIdx.z, t0 = blockIdx.y * kConvSegment, t1 = min(tokens, t0 + kConvSegment);
   const size_t seq = static_cast<size_t>(b) * tokens * channels + c;
   float* own_state = state + (static_cast<size_t>(b) * channels + c) * W;   // [4][W]
@@ -249,8 +251,8 @@ __global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* _
     const int t = t0 - W + tap;
     if (t >= 0) {
       const float4 v = load_four<IN_BF16>(input, seq + static_cast<size_t>(t) * channels);
-      x[tap][0] = rnd(v.x, round); x[tap][1] = rnd(v.y, round);
-      x[tap][2] = rnd(v.z, round); x[tap][3] = rnd(v.w, round);
+      x[tap][0] = rounded_in(v.x); x[tap][1] = rounded_in(v.y);
+      x[tap][2] = rounded_in(v.z); x[tap][3] = rounded_in(v.w);
     } else {
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[tap][i] = own_state[i * W + W + t];
@@ -264,8 +266,8 @@ __global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* _
     for (int tap = 0; tap + 1 < W; ++tap)
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[tap][i] = x[tap + 1][i];
-    x[W - 1][0] = rnd(v.x, round); x[W - 1][1] = rnd(v.y, round);
-    x[W - 1][2] = rnd(v.z, round); x[W - 1][3] = rnd(v.w, round);
+    x[W - 1][0] = rounded_in(v.x); x[W - 1][1] = rounded_in(v.y);
+    x[W - 1][2] = rounded_in(v.z); x[W - 1][3] = rounded_in(v.w);
     float y[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* _
 #pragma unroll
       for (int tap = 0; tap + 1 < W; ++tap) sum += x[tap][i] * w[i][tap];
       sum = rnd(sum + x[W - 1][i] * w[i][W - 1], round);
-      y[i] = rnd(sum * sigmoid_fast(sum), round);
+      y[i] = OUT_BF16 ? sum * sigmoid_fast(sum) : rnd(sum * sigmoid_fast(sum), round);
     }
     store_four<OUT_BF16>(output, at, y);
   }
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(128, 10) gdn_conv_segment_kernel(const void* _
 #pragma unroll
       for (int tap = 0; tap < W; ++tap) {   // token tokens - W + tap, or an entry of the old window
         const int t = tokens - W + tap;
-        kept[tap] = t >= 0 ? rnd(load_any(input, seq + static_cast<size_t>(t) * channels + i, IN_BF16), round)
+        kept[tap] = t >= 0 ? rounded_in(load_any(input, seq + static_cast<size_t>(t) * channels + i, IN_BF16))
                            : own_state[i * W + W + t];
       }
 #pragma unroll

@@ -475,7 +475,7 @@ __global__ void gdn_conv_weight_bwd_kernel(const void* input, int in_is_bf16, co
 // shared memory.  Every element of x and dpost is read once (plus W - 1 at the seams of the ranges)
 // and dpre is computed once; the two kernels above recompute it for every tap, and the weight one
 // leaves a channel to a single thread for the whole sequence (220 + 938 us at 1000 tokens x 10240
-// channels, 100 MB of traffic; 52 us in this form, where the sigmoid and the rounding of 10 M
+// channels, 100 MB of traffic; 39 us in this form, where the sigmoid and the rounding of 10 M
 // elements keep the issue slots busy).
 constexpr int kConvWarps = 4, kConvCluster = 8;
 template <int P, bool BF16>
@@ -492,11 +492,12 @@ __device__ __forceinline__ void load_channels(const void* p, size_t i, float (&v
 }
 
 template <int W, int P, bool IN_BF16>
-__global__ void __launch_bounds__(kConvWarps * 32, 8) __cluster_dims__(1, kConvCluster, 1)
+__global__ void __launch_bounds__(kConvWarps * 32, 6) __cluster_dims__(1, kConvCluster, 1)
 gdn_conv_bwd_kernel(const void* __restrict__ input, const float* __restrict__ weight,
                     const float* __restrict__ dpost, int batch, int tokens, int channels, int round,
                     float* __restrict__ dx, float* dw) {
-  constexpr int kBatch = 2;   // tokens whose loads are in flight together
+  // tokens whose loads are in flight together; four also make the windows' shifts a matter of register names
+  constexpr int kBatch = 4;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int c = (blockIdx.x * 32 + lane) * P;
   const bool live = c < channels;
@@ -519,7 +520,7 @@ gdn_conv_bwd_kernel(const void* __restrict__ input, const float* __restrict__ we
       const int t = t0 - W + tap;
       load_channels<P, IN_BF16>(input, seq + static_cast<size_t>(max(t, 0)) * channels, x[tap]);
 #pragma unroll
-      for (int i = 0; i < P; ++i) x[tap][i] = t >= 0 ? rnd(x[tap][i], round) : 0.0f;
+      for (int i = 0; i < P; ++i) x[tap][i] = t >= 0 ? (IN_BF16 ? x[tap][i] : rnd(x[tap][i], round)) : 0.0f;
     }
 #pragma unroll
     for (int tap = 0; tap < W; ++tap)
@@ -546,7 +547,7 @@ gdn_conv_bwd_kernel(const void* __restrict__ input, const float* __restrict__ we
             x[tap][i] = x[tap + 1][i];
             dpre[tap][i] = dpre[tap + 1][i];
           }
-          x[W - 1][i] = rnd(in[u][i], round);
+          x[W - 1][i] = IN_BF16 ? in[u][i] : rnd(in[u][i], round);   // (a bf16 input is rounded already)
           float sum = 0.0f;
 #pragma unroll
           for (int tap = 0; tap < W; ++tap) sum += x[tap][i] * w[tap][i];

@@ -215,14 +215,17 @@ __device__ __forceinline__ void load_a_fragment(const float* A, int pa, int m0, 
   split_pair(x2.x, x2.y, hi[2], lo[2]);
   split_pair(x3.x, x3.y, hi[3], lo[3]);
 }
-// out1 = A1 Bg (and out2 = sign2 A2 Bg when kTwo) for a [128 x 128] matrix Bg in global memory, whose
-// rows pass through `ring` ([4 stages][16 rows][132] floats, one 16-byte asynchronous copy per thread
-// and stage, three stages in flight).  Warp w owns the 16 x 32 block (rows 16 (w / 4), columns
-// 32 (w % 4)) of the [64 x 128] results.  out2 may be the matrix A1 lives in: the results are
-// written after the last read of the operands.  All 512 threads call this together; on return the
-// results are visible to every thread and the ring is free.
-template <bool kTwo>
-__device__ __forceinline__ void nn_ring_mma(const float* A1, const float* A2, int pa, const float* __restrict__ Bg,
+// out1 = A1 Bg (and out2 = sign2 A2 Bg when kTwo) for a [128 x 128] matrix Bg in global memory, or, with
+// kTransB, A1 Bg^T.  Bg passes through `ring` (one 16-byte asynchronous copy per thread and stage, three
+// stages in flight): 16 rows of Bg, [16][132] floats, per stage, or 16 columns, [128 rows][16], whose
+// 16-byte chunk c of row r lies at chunk c ^ (r & 2) so that the fragment loads of half a warp (4 rows x 4
+// pairs) cover all banks.  (Reading the state matrices both ways from here saves the 2 x 50 MB, 47 us, that
+// transposed copies of them cost at 1000 tokens of 48 heads.)  Warp w owns the 16 x 32 block (rows
+// 16 (w / 4), columns 32 (w % 4)) of the [64 x 128] results.  out2 may be the matrix A1 lives in: the
+// results are written after the last read of the operands.  All 512 threads call this together; on
+// return the results are visible to every thread and the ring is free.
+template <bool kTransB, bool kTwo>
+__device__ __forceinline__ void ring_mma(const float* A1, const float* A2, int pa, const float* __restrict__ Bg,
                                             float* ring, int tid, float* out1, float* out2, float sign2) {
   const int warp = tid >> 5, lane = tid & 31;
   const int m0 = (warp >> 2) * 16, n0 = (warp & 3) * 32, g = lane >> 2, t = lane & 3;
@@ -231,10 +234,11 @@ __device__ __forceinline__ void nn_ring_mma(const float* A1, const float* A2, in
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) c1[i][j] = c2[i][j] = 0.0f;
-  const int row = tid >> 5, c4 = tid & 31;   // this thread's 16 bytes of a stage
-  auto issue = [&](int s) {
-    cp_async16(ring + (s % 4) * kMmaStageFloats + row * kMmaRingPitch + c4 * 4, Bg + (s * 16 + row) * kLD + c4 * 4);
-  };
+  // this thread's 16 bytes of a stage
+  const int row = kTransB ? tid >> 2 : tid >> 5, c4 = kTransB ? tid & 3 : tid & 31;
+  float* to = ring + (kTransB ? row * 16 + ((c4 ^ (row & 2)) << 2) : row * kMmaRingPitch + c4 * 4);
+  const float* from = Bg + row * kLD + c4 * 4;
+  auto issue = [&](int s) { cp_async16(to + (s % 4) * kMmaStageFloats, from + s * 16 * (kTransB ? 1 : kLD)); };
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
     issue(s);
@@ -252,10 +256,18 @@ __device__ __forceinline__ void nn_ring_mma(const float* A1, const float* A2, in
     if (kTwo) load_a_fragment(A2, pa, m0, s * 16, g, t, a2h, a2l);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      const float* col = Bs + n0 + nt * 8 + g;
       uint32_t bh0, bl0, bh1, bl1;
-      split_pair(col[(2 * t) * kMmaRingPitch], col[(2 * t + 1) * kMmaRingPitch], bh0, bl0);
-      split_pair(col[(2 * t + 8) * kMmaRingPitch], col[(2 * t + 9) * kMmaRingPitch], bh1, bl1);
+      if (kTransB) {
+        const float* own = Bs + (n0 + nt * 8 + g) * 16;
+        const int at = (((t >> 1) ^ (g & 2)) << 2) + 2 * (t & 1);
+        const float2 y0 = *reinterpret_cast<const float2*>(own + at), y1 = *reinterpret_cast<const float2*>(own + (at ^ 8));
+        split_pair(y0.x, y0.y, bh0, bl0);
+        split_pair(y1.x, y1.y, bh1, bl1);
+      } else {
+        const float* col = Bs + n0 + nt * 8 + g;
+        split_pair(col[(2 * t) * kMmaRingPitch], col[(2 * t + 1) * kMmaRingPitch], bh0, bl0);
+        split_pair(col[(2 * t + 8) * kMmaRingPitch], col[(2 * t + 9) * kMmaRingPitch], bh1, bl1);
+      }
       mma16816(c1[nt], a1h, bh0, bh1);
       mma16816(c1[nt], a1h, bl0, bl1);
       mma16816(c1[nt], a1l, bh0, bh1);
@@ -328,7 +340,7 @@ __device__ __forceinline__ void nt_mma(const float* A1, const float* A2, int pa,
 }
 // out1 (+)= op(A) diag(sc1) B1  (and out2 = op(A) diag(sc2) B2 when kTwoB) for A [64 x K] (or, kTransA,
 // stored [K x 64]) and B [K x 128] in shared memory; sc: optional factor per k.  Warp blocks and result
-// matrices as nn_ring_mma; kAccumulate adds to what out1 holds.  No barrier inside.
+// matrices as ring_mma; kAccumulate adds to what out1 holds.  No barrier inside.
 template <int K, bool kTransA, bool kTwoB, bool kAccumulate>
 __device__ __forceinline__ void nn_mma(const float* A, int pa, const float* B1, const float* sc1, const float* B2,
                                        const float* sc2, int pb, int tid, float* out1, float* out2) {
@@ -462,9 +474,7 @@ __device__ __forceinline__ void store_dense(float* dst, const Lane& l, const flo
 struct LocalArgs {
   GdnBwdArgs a;
   const float* states;      // [sequence, head, chunk, key, value column]: state at each chunk's start
-  const float* states_t;    // the same matrices transposed, [.., value column, key]
   const float* dstates;     // [sequence, head, chunk, key, value column]: state gradient at each chunk's end
-  const float* dstates_t;
   int chunks;
   // Where the q / k gradients of a token's head go: rows of 2 x 128 floats (q then k) in the
   // partials when several value heads share a key head (the gather kernel sums them), or the
@@ -492,17 +502,15 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
   const size_t unit = static_cast<size_t>(b) * a.value_heads + h;
   const size_t matrix = (unit * la.chunks + chunk) * kLD * kLD;
   const float* S0 = la.states + matrix;        // [key][value column]
-  const float* S0t = la.states_t + matrix;     // [value column][key]
   const float* dS = la.dstates + matrix;
-  const float* dSt = la.dstates_t + matrix;
   float* Kh = sm.big[0];
   const float q_scale = rsqrtf(static_cast<float>(kLD));
   const size_t token0 = static_cast<size_t>(b) * a.tokens + t0;   // first token of the chunk
 
-  // The four state matrices are first needed tens of microseconds from now and would come from
+  // The state matrices are first needed tens of microseconds from now and would come from
   // DRAM then: ask for them in L2 now.
-  if (tid < 4) {
-    const float* m = tid == 0 ? S0 : (tid == 1 ? dS : (tid == 2 ? S0t : dSt));
+  if (tid < 2) {
+    const float* m = tid == 0 ? S0 : dS;
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(m), "r"(kLD * kLD * 4) : "memory");
   }
   // ---- gates
@@ -534,9 +542,16 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
     *reinterpret_cast<float4*>(sm.big[which] + t * kLP + c4 * 4) = v;
   }
   __syncthreads();
-  if (tid == 0) {
-    float run = 0.0f;
-    for (int t = 0; t < kLC; ++t) { run += sm.b[t]; sm.b[t] = run; }
+  if (warp == 0) {   // running sums: a lane holds two tokens
+    const float2 own = *reinterpret_cast<const float2*>(sm.b + 2 * lane);
+    float run = own.x + own.y;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float below = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += below;
+    }
+    const float before = __shfl_up_sync(0xffffffffu, run, 1);
+    *reinterpret_cast<float2*>(sm.b + 2 * lane) = make_float2((lane > 0 ? before : 0.0f) + own.x, run);
   }
   for (int vec = warp; vec < 2 * kLC; vec += kLThreads / 32) {
     const int which = vec / kLC, t = vec % kLC;
@@ -618,7 +633,7 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
   // ---- U = U' - W S_0 -> big[4]
   {
     float acc[4][4];
-    nn_ring_mma<false>(sm.big[1], nullptr, kLP, S0, sm.big[2], tid, sm.big[4], nullptr, 0.0f);   // (v in big[2] is dead: U' is complete)
+    ring_mma<false, false>(sm.big[1], nullptr, kLP, S0, sm.big[2], tid, sm.big[4], nullptr, 0.0f);   // (v in big[2] is dead: U' is complete)
     load_dense(sm.big[4], l, acc);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -627,7 +642,7 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
           make_float4(up.x - acc[i][0], up.y - acc[i][1], up.z - acc[i][2], up.w - acc[i][3]);
     }
   }
-  // ---- dO -> big[2] (the ring is free: nn_ring ends with a barrier)
+  // ---- dO -> big[2] (the ring is free: ring_mma ends with a barrier)
   for (int idx = tid; idx < kLC * (kLD / 4); idx += kLThreads) {
     const int t = idx / (kLD / 4), c4 = idx % (kLD / 4);
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -687,7 +702,7 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
   // ---- dKt = U dS^T (dense columns = keys)
   {
     float acc[4][4];
-    nn_ring_mma<false>(sm.big[4], nullptr, kLP, dSt, sm.big[3], tid, sm.big[1], nullptr, 0.0f);   // (W and U' are dead from here on: big[1], big[3])
+    ring_mma<true, false>(sm.big[4], nullptr, kLP, dS, sm.big[3], tid, sm.big[1], nullptr, 0.0f);   // (W and U' are dead from here on: big[1], big[3])
     load_dense(sm.big[1], l, acc);
     float rows[4];
 #pragma unroll
@@ -709,11 +724,11 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
     }
     add_rows(sm.db, rows, -1.0f);
   }
-  // ---- dU = M^T dO + Kt dS -> big[4]   (every read of U is done: nn_ring ends with a barrier)
+  // ---- dU = M^T dO + Kt dS -> big[4]   (every read of U is done: ring_mma ends with a barrier)
   {
     float acc[4][4], from_state[4][4];
     nn_mma<kLC, true, false, false>(Mm, kLQ, sm.big[2], nullptr, nullptr, nullptr, kLP, tid, sm.big[4], nullptr);   // M^T dO (U is dead)
-    nn_ring_mma<false>(Kh, nullptr, kLP, dS, sm.big[3], tid, sm.big[1], nullptr, 0.0f);   // (starts with a barrier: the dKt tiles are out of big[1])
+    ring_mma<false, false>(Kh, nullptr, kLP, dS, sm.big[3], tid, sm.big[1], nullptr, 0.0f);   // (starts with a barrier: the dKt tiles are out of big[1])
     load_dense(sm.big[4], l, acc);
     load_dense(sm.big[1], l, from_state);
 #pragma unroll
@@ -734,7 +749,7 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
                                : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float acc[4][4];
     __syncthreads();   // every thread has its tile of the dU product's state term out of big[1]; dU is stored
-    nn_ring_mma<true>(sm.big[2], sm.big[4], kLP, S0t, sm.big[3], tid, sm.big[1], sm.big[2], -1.0f);
+    ring_mma<true, true>(sm.big[2], sm.big[4], kLP, S0, sm.big[3], tid, sm.big[1], sm.big[2], -1.0f);
     load_dense(sm.big[1], l, acc);
     float rows[4];
 #pragma unroll
@@ -919,15 +934,25 @@ __global__ void __launch_bounds__(kLThreads, 1) gdn_bwd_chunk_local(LocalArgs la
                       ikt * (dk_acc[i][2] - kv[i][2] * pk), ikt * (dk_acc[i][3] - kv[i][3] * pk));
     }
   }
-  if (tid == 0) {
-    float total = 0.0f;
-    for (int w = 0; w < kLThreads / 32; ++w) total += sm.red[w];
-    // d log g_s = sum of db_t over t >= s (db: both column halves, minus the column sums of A-bar)
-    float run = 0.0f;
-    for (int t = kLC - 1; t >= 0; --t) {
-      run += sm.db[0][t] + sm.db[1][t] - sm.part[0][t] + (t == kLC - 1 ? total : 0.0f);
-      sm.db[0][t] = run;
+  if (warp == 0) {
+    float total = lane < kLThreads / 32 ? sm.red[lane] : 0.0f;
+#pragma unroll
+    for (int o = kLThreads / 64; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    total = __shfl_sync(0xffffffffu, total, 0);
+    // d log g_s = sum of db_t over t >= s (db: both column halves, minus the column sums of A-bar); a lane
+    // holds two tokens
+    const int t = 2 * lane;
+    const float first = sm.db[0][t] + sm.db[1][t] - sm.part[0][t];
+    const float second = sm.db[0][t + 1] + sm.db[1][t + 1] - sm.part[0][t + 1] + (lane == 31 ? total : 0.0f);
+    float run = first + second;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float above = __shfl_down_sync(0xffffffffu, run, o);
+      if (lane + o < 32) run += above;
     }
+    const float later = __shfl_down_sync(0xffffffffu, run, 1);   // the tokens of the lanes above
+    sm.db[0][t] = run;
+    sm.db[0][t + 1] = second + (lane < 31 ? later : 0.0f);
   }
   __syncthreads();
   if (tid < count) {
@@ -950,27 +975,9 @@ __global__ void cast_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16
   }
 }
 
-// out[m] = in[m]^T for a batch of [128 x 128] fp32 matrices; one CTA of 256 threads per matrix
-__global__ void __launch_bounds__(256) transpose_128_kernel(const float* __restrict__ in, float* __restrict__ out) {
-  __shared__ float tile[32][129];
-  const size_t base = static_cast<size_t>(blockIdx.x) * kLD * kLD;
-  for (int strip = 0; strip < 4; ++strip) {   // rows strip*32 .. +31 of the input
-    for (int e = threadIdx.x; e < 32 * kLD; e += 256) {
-      const int r = e / kLD, c = e % kLD;
-      tile[r][c] = in[base + static_cast<size_t>(strip * 32 + r) * kLD + c];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 32 * kLD; e += 256) {
-      const int c = e / 32, r = e % 32;
-      out[base + static_cast<size_t>(c) * kLD + strip * 32 + r] = tile[r][c];
-    }
-    __syncthreads();
-  }
-}
-
 // A second stream per device: the reverse scan needs the forward's records but not its states, so
 // it runs beside the forward scan (both fill only sequences x heads SMs), with the bf16 copy of the
-// output gradient made there too; the caller's stream joins before the transposes.
+// output gradient made there too; the caller's stream joins before the chunk kernel.
 struct BwdLanes {
   cudaStream_t aux = nullptr;
   cudaEvent_t forked = nullptr, prepared = nullptr, aux_done = nullptr;
@@ -1003,9 +1010,9 @@ bool gdn_bwd_chunked_supported(const GdnBwdArgs& a) {
 }
 
 // Layout of the workspace: records | g, beta | dcore as bf16 | forward output (bf16, unused) |
-// states, their transposes | state gradients, their transposes | q/k partials | scalar partials
+// states | state gradients | the scan's running state | q/k partials | scalar partials
 struct ChunkedBwdLayout {
-  size_t records, gates, dcore16, out16, states, states_t, dstates, dstates_t, qk_partials, scalar_partials, total;
+  size_t records, gates, dcore16, out16, states, dstates, running, qk_partials, scalar_partials, total;
 };
 static ChunkedBwdLayout chunked_bwd_layout(int batch, int tokens, int value_heads) {
   const size_t chunks = (tokens + kLC - 1) / kLC, units = static_cast<size_t>(batch) * value_heads;
@@ -1017,9 +1024,8 @@ static ChunkedBwdLayout chunked_bwd_layout(int batch, int tokens, int value_head
   l.dcore16 = at; at += align_up(rows * kLD * 2);
   l.out16 = at; at += align_up(rows * kLD * 2);
   l.states = at; at += align_up(units * chunks * kLD * kLD * sizeof(float));
-  l.states_t = at; at += align_up(units * chunks * kLD * kLD * sizeof(float));
   l.dstates = at; at += align_up(units * chunks * kLD * kLD * sizeof(float));
-  l.dstates_t = at; at += align_up(units * chunks * kLD * kLD * sizeof(float));
+  l.running = at; at += align_up(units * kLD * kLD * sizeof(float));
   l.qk_partials = at; at += align_up(rows * 2 * kLD * sizeof(float));
   l.scalar_partials = at; at += align_up(rows * 3 * sizeof(float));
   l.total = at + 1024;   // room to align the base
@@ -1043,8 +1049,7 @@ cudaError_t gdn_bwd_chunked(cudaStream_t stream, GdnBwdArgs& a, float* dq_out, f
   __nv_bfloat16* dcore16 = reinterpret_cast<__nv_bfloat16*>(base + l.dcore16);
   float* states = reinterpret_cast<float*>(base + l.states);
   float* dstates = reinterpret_cast<float*>(base + l.dstates);
-  float* states_t = reinterpret_cast<float*>(base + l.states_t);
-  float* dstates_t = reinterpret_cast<float*>(base + l.dstates_t);
+  float* running = reinterpret_cast<float*>(base + l.running);
   a.qk_partials = reinterpret_cast<float*>(base + l.qk_partials);
   a.scalar_partials = reinterpret_cast<float*>(base + l.scalar_partials);
 
@@ -1072,29 +1077,19 @@ cudaError_t gdn_bwd_chunked(cudaStream_t stream, GdnBwdArgs& a, float* dq_out, f
   f.batch = a.batch; f.tokens = a.tokens; f.key_heads = a.key_heads; f.value_heads = a.value_heads;
   f.key_dim = kLD; f.value_dim = kLD;
   f.normalize_qk = 1; f.q_scale = 1.0f; f.round = a.round;
-  // the scan reads its initial state from and leaves its final state in f.state: the transposed
-  // state-gradient area is free until the transposes run
-  f.state = dstates_t;
+  f.state = running;   // the scan reads its initial state from here and leaves its final one
   if (e == cudaSuccess)
-    e = cudaMemsetAsync(dstates_t, 0, static_cast<size_t>(a.batch) * a.value_heads * kLD * kLD * sizeof(float), stream);
+    e = cudaMemsetAsync(running, 0, static_cast<size_t>(a.batch) * a.value_heads * kLD * kLD * sizeof(float), stream);
   if (e == cudaSuccess) e = gdn_chunked_with_states(stream, f, base + l.records, states, status, lanes->prepared);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(lanes->aux, lanes->prepared, 0);
   if (e == cudaSuccess)
     e = gdn_scan_bwd_launch(lanes->aux, dcore16, base + l.records, a.batch, a.tokens, a.value_heads, chunks, dstates, status);
   // (joined even after a failed launch, so that nothing of this call is left running unordered)
   cudaError_t joined = cudaEventRecord(lanes->aux_done, lanes->aux);
-  const unsigned matrices = static_cast<unsigned>(a.batch) * a.value_heads * chunks;
-  if (e == cudaSuccess && joined == cudaSuccess) {
-    transpose_128_kernel<<<matrices, 256, 0, stream>>>(states, states_t);   // (needs the forward only)
-    e = cudaGetLastError();
-  }
   if (joined == cudaSuccess) joined = cudaStreamWaitEvent(stream, lanes->aux_done, 0);
   if (e != cudaSuccess) return e;
   if (joined != cudaSuccess) return joined;
-  transpose_128_kernel<<<matrices, 256, 0, stream>>>(dstates, dstates_t);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  LocalArgs la{a, states, states_t, dstates, dstates_t, chunks, nullptr, nullptr, 0, 0};
+  LocalArgs la{a, states, dstates, chunks, nullptr, nullptr, 0, 0};
   *qk_direct = a.value_heads == a.key_heads && dqk_token % 4 == 0 && (reinterpret_cast<uintptr_t>(dq_out) & 15u) == 0 &&
                (reinterpret_cast<uintptr_t>(dk_out) & 15u) == 0;
   if (*qk_direct) {
