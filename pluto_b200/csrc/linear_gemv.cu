@@ -509,23 +509,32 @@ linear_gemv_mma(const void* __restrict__ weights, const float* __restrict__ scal
     for (int i = threadIdx.x; i < chunks; i += kThreads)
       reinterpret_cast<uint4*>(xs)[i] = reinterpret_cast<const uint4*>(x)[i];
   } else {
-    for (int group = warp; group < tokens * groups; group += kWarps) {
-      const int t = group / groups, g = group % groups;
-      float v[4], maximum = 0.0f;
+    // (every CTA does this for itself: with one group after another in flight it was most of the time of a
+    // call: 5120 x 10240, 8 tokens, 120 us, 81 in batches)
+    constexpr int kBatch = 5;   // groups whose loads and reductions are in flight together
+    const int total = tokens * groups;
+    for (int first = warp; first < total; first += kWarps * kBatch) {
+      uint2 raw[kBatch];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[i] = __bfloat162float(x[static_cast<size_t>(t) * cols + g * 128 + lane * 4 + i]);
-        maximum = fmaxf(maximum, fabsf(v[i]));
+      for (int u = 0; u < kBatch; ++u) {   // past the end: repeats the last group
+        const int group = min(first + u * kWarps, total - 1);
+        raw[u] = *reinterpret_cast<const uint2*>(x + static_cast<size_t>(group) * 128 + lane * 4);   // (x rows are contiguous)
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, o));
-      const float scale = maximum / 448.0f, divisor = fmaxf(scale, 1e-12f);
-      uint32_t word = 0;
+      for (int u = 0; u < kBatch; ++u) {
+        const int group = min(first + u * kWarps, total - 1);
+        const float v[4] = {bf16_lo(raw[u].x), bf16_hi(raw[u].x), bf16_lo(raw[u].y), bf16_hi(raw[u].y)};
+        float maximum = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        word |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(v[i] / divisor, __NV_SATFINITE, __NV_E4M3)) << (8 * i);
-      reinterpret_cast<uint32_t*>(xs + static_cast<size_t>(t) * cols + g * 128)[lane] = word;
-      if (lane == 0) xscale[t * groups + g] = scale;
+        for (int o = 16; o > 0; o >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, o));
+        const float scale = maximum / 448.0f, divisor = fmaxf(scale, 1e-12f);
+        uint32_t word = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          word |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(v[i] / divisor, __NV_SATFINITE, __NV_E4M3)) << (8 * i);
+        reinterpret_cast<uint32_t*>(xs + static_cast<size_t>(group) * 128)[lane] = word;
+        if (lane == 0) xscale[group] = scale;
+      }
     }
   }
   __syncthreads();
@@ -927,10 +936,11 @@ cudaError_t dispatch(cudaStream_t stream, const void* weights, const float* scal
     //   FP8 ring, FMA                  17.2   23.2   38.3   56.1    -
     //   FP8 tensor cores from global   26.9   33.0    -     45.1   69.0
     // (the FMA form without the ring: 25.7 and 23.3 for one token, 80-143 for FP8 batches whose
-    // activation no longer fits its staging buffer).  So FP8 takes the ring with tensor cores in
-    // passes of 4 tokens when the shape qualifies, else the FMA ring for up to three tokens; one
-    // bf16 token takes the FMA ring; everything else that qualifies takes the tensor-core form
-    // that loads from global memory, 8 tokens per pass.
+    // activation no longer fits its staging buffer).  So FP8 takes the ring with tensor cores, all tokens
+    // in one pass or four at a time, when the shape qualifies (long rows: 5120 x 10240 with one token 17.4
+    // against 24.4 on the FMA ring; few rows: 1280 x 5120 5.9 against 14.4 from global memory), else the FMA
+    // ring for up to three tokens; one bf16 token takes the FMA ring; everything else that qualifies takes
+    // the tensor-core form that loads from global memory, 8 tokens per pass.
     int sms = 148, device = 0;
     if (cudaGetDevice(&device) == cudaSuccess)
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
