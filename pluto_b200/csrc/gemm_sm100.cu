@@ -46,7 +46,7 @@ struct GemmParams {
   size_t ldc;
   int c_kind;          // 0 fp32, 1 bf16
   uint32_t* status;
-  int splits = 1;           // the one-SM kernel's parts of K; part s of C goes to c + s * part_stride floats
+  int splits = 1;           // parts of K; part s of C goes to c + s * part_stride floats
   size_t part_stride = 0;
 };
 
@@ -387,7 +387,8 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int rank = static_cast<int>(cluster_cta_rank());   // 0 issues the MMAs
   const int cluster = blockIdx.x / 2, clusters = gridDim.x / 2;
   const int m_tiles = (p.M + kPairTile - 1) / kPairTile, n_tiles = (p.N + kPairTile - 1) / kPairTile;
-  const int tiles = m_tiles * n_tiles;
+  const int tiles = m_tiles * n_tiles, units = tiles * p.splits;   // as in gemm_sm100
+  auto first_step = [&](int part) { return static_cast<int>(static_cast<long long>(p.k_tiles) * part / p.splits); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -419,12 +420,13 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       tma_prefetch_desc(&map_b);
       bool ok = true;
       int it = 0;
-      for (int tile = cluster; tile < tiles && ok; tile += clusters) {
+      for (int unit = cluster; unit < units && ok; unit += clusters) {
         int m0, n0;
-        pair_tile_origin(tile, m_tiles, n_tiles, m0, n0);
+        pair_tile_origin(unit % tiles, m_tiles, n_tiles, m0, n0);
+        const int k_end = first_step(unit / tiles + 1);
         m0 += rank * kTile;   // this CTA's rows of A
         n0 += rank * kTile;   // this CTA's columns of B
-        for (int kt = 0; kt < p.k_tiles && ok; ++kt, ++it) {
+        for (int kt = first_step(unit / tiles); kt < k_end && ok; ++kt, ++it) {
           const int st = it % kPairStages, use = it / kPairStages;
           if (use > 0) ok = mbar_wait(&bar->empty[st], (use - 1) & 1, p.status, 75);
           if (!ok) break;
@@ -454,13 +456,14 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   } else if (warp == 1 && rank == 0) {
     bool ok = true;
     int it = 0, local = 0;
-    for (int tile = cluster; tile < tiles && ok; tile += clusters, ++local) {
+    for (int unit = cluster; unit < units && ok; unit += clusters, ++local) {
+      const int k_begin = first_step(unit / tiles), k_end = first_step(unit / tiles + 1);
       const int buf = local & 1, use = local >> 1;
       if (use > 0)   // both CTAs' epilogues have drained this accumulator's previous tile
         ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_empty[buf], (use - 1) & 1, p.status, 77));
       if (!ok) break;
       tc_fence_after();
-      for (int kt = 0; kt < p.k_tiles && ok; ++kt, ++it) {
+      for (int kt = k_begin; kt < k_end && ok; ++kt, ++it) {
         const int st = it % kPairStages;
         ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[st], (it / kPairStages) & 1, p.status, 78));
         if (!ok) break;
@@ -473,9 +476,9 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
           for (int ks = 0; ks < kBK / 16; ++ks)
             umma_ss_pair(tmem + buf * kPairTile, a_desc + ks * ((A_MN ? 2048 : 32) >> 4),
-                         b_desc + ks * ((B_MN ? 2048 : 32) >> 4), pair_idesc, kt > 0 || ks > 0);
+                         b_desc + ks * ((B_MN ? 2048 : 32) >> 4), pair_idesc, kt > k_begin || ks > 0);
           tc_commit_pair(&bar->empty[st]);
-          if (kt + 1 == p.k_tiles) tc_commit_pair(&bar->acc_full[buf]);
+          if (kt + 1 == k_end) tc_commit_pair(&bar->acc_full[buf]);
         }
         __syncwarp();
       }
@@ -484,13 +487,14 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int quarter = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     int local = 0;
-    for (int tile = cluster; tile < tiles; tile += clusters, ++local) {
+    for (int unit = cluster; unit < units; unit += clusters, ++local) {
       const int buf = local & 1;
       int m0, n0;
-      pair_tile_origin(tile, m_tiles, n_tiles, m0, n0);
+      pair_tile_origin(unit % tiles, m_tiles, n_tiles, m0, n0);
+      void* c = p.splits > 1 ? static_cast<float*>(p.c) + (unit / tiles) * p.part_stride : p.c;
       if (!mbar_wait(&bar->acc_full[buf], (local >> 1) & 1, p.status, 79)) break;
       tc_fence_after();
-      drain_accumulator(tmem + lane_base + buf * kPairTile, m0 + rank * kTile + quarter * 32, lane, n0, p, p.c,
+      drain_accumulator(tmem + lane_base + buf * kPairTile, m0 + rank * kTile + quarter * 32, lane, n0, p, c,
                         smem_u32(drain_stage) + quarter * (kDrainStageBytes / 4));
       tc_fence_before();
       __syncwarp();
@@ -612,6 +616,7 @@ __global__ void bias_final_kernel(const float* __restrict__ partial, int chunks,
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= cols) return;
   float total = 0.0f;
+#pragma unroll 16
   for (int c = 0; c < chunks; ++c) total += partial[static_cast<size_t>(c) * cols + n];
   db[n] = total;
 }
@@ -648,22 +653,34 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
   *dst = sum;
 }
 
-// Parts of K for a product of few tiles on `sms` SMs.  In microseconds: a CTA takes 0.4 per K step and
-// about 2 to fill its pipeline and drain its tile; the parts cross L2 twice, at about 8 bytes/ps, and
-// their sum is one more launch.
+// Which kernel a product takes and in how many parts of K.  In microseconds: an SM takes 0.4 per K step
+// of 128 x 256 alone and 0.6 when all SMs pull their operands through L2, a pair of SMs 0.45 per step of
+// 256 x 256; 2 to fill the pipeline and drain a tile; the parts' sum is one more launch that reads them at
+// about 6.5 bytes/ps.  (8192 x 768 -> 2304: forward 30 for 35 measured, dX 36 for 36, dW in five parts
+// on single SMs 45 for 45.)
 constexpr size_t kMaxPartBytes = size_t{96} << 20;
-int gemm_splits(int M, int N, int k_tiles, int sms) {
-  const long long tiles = static_cast<long long>((N + kTileN - 1) / kTileN) * ((M + kTile - 1) / kTile);
+struct GemmPlan {
+  bool pair;
+  int splits;
+};
+GemmPlan gemm_plan(int M, int N, int k_tiles, int sms, bool pair_allowed) {
   const size_t part = static_cast<size_t>(M) * N * sizeof(float);
-  int best = 1;
+  GemmPlan best = {false, 1};
   double least = 1e30;
-  for (int z = 1; z <= 32 && z * 4 <= std::max(k_tiles, 4); ++z) {
-    if (z > 1 && (N % 4 != 0 || z * part > kMaxPartBytes)) break;
-    const double waves = static_cast<double>((tiles * z + sms - 1) / sms), steps = (k_tiles + z - 1) / z;
-    const double us = waves * (0.4 * steps + 2.0) + (z > 1 ? 3.0 + 2.0 * z * part / 8e6 : 0.0);
-    if (us < 0.95 * least) {
-      least = us;
-      best = z;
+  for (int kind = 0; kind < 2; ++kind) {
+    const bool pair = kind == 1;
+    if (pair && !pair_allowed) continue;
+    const int tile_m = pair ? 256 : kTile, workers = pair ? sms / 2 : sms;
+    const long long tiles = static_cast<long long>((N + 255) / 256) * ((M + tile_m - 1) / tile_m);
+    for (int z = 1; z <= 32 && z * 4 <= std::max(k_tiles, 4); ++z) {
+      if (z > 1 && (N % 4 != 0 || z * part > kMaxPartBytes)) break;
+      const double waves = static_cast<double>((tiles * z + workers - 1) / workers), steps = (k_tiles + z - 1) / z;
+      const double busy = std::min(1.0, static_cast<double>(tiles * z) / workers);
+      const double us = waves * ((pair ? 0.45 : 0.4 + 0.2 * busy) * steps + 2.0) + (z > 1 ? 2.0 + z * part / 6.5e6 : 0.0);
+      if (us < 0.95 * least) {
+        least = us;
+        best = {pair, z};
+      }
     }
   }
   return best;
@@ -676,7 +693,7 @@ int sm_count() {
 }
 // Scratch that launch_gemm can use for a product (0: it is not split).
 size_t gemm_part_bytes(int M, int N, int k_tiles) {
-  const int z = gemm_splits(M, N, k_tiles, sm_count());
+  const int z = gemm_plan(M, N, k_tiles, sm_count(), true).splits;
   return z > 1 ? z * static_cast<size_t>(M) * N * sizeof(float) : 0;
 }
 struct Scratch {   // for parts of K: 16-byte aligned, or none
@@ -685,66 +702,60 @@ struct Scratch {   // for parts of K: 16-byte aligned, or none
 };
 
 // b_pair: the B operand's map for the two-SM kernel (K-major B: boxes of 128 rows; MN-major B: the
-// same slab map as `b`), or null to keep the call on the one-SM kernel.
+// same slab map as `b`), or null to keep the call on the one-SM kernel.  scratch: room for parts of K.
 template <bool A_MN, bool B_MN>
 cudaError_t launch_gemm(cudaStream_t stream, const CUtensorMap& a, const CUtensorMap& b,
                         const GemmParams& params, const CUtensorMap* b_pair = nullptr, Scratch scratch = {}) {
   GemmParams p = params;
   const int sms = sm_count();
-  const int pair_tiles = ((p.N + kPairTile - 1) / kPairTile) * ((p.M + kPairTile - 1) / kPairTile);
-  if (b_pair != nullptr && pair_tiles >= sms / 2) {   // enough 256 x 256 tiles to occupy every pair of SMs
-    const size_t pair_smem =
-        1024 + kPairStages * (kPairABytes + kPairBBytes) + kDrainStageBytes + sizeof(PairGemmBarriers);
-    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_pair<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(pair_smem));
-    if (e != cudaSuccess) return e;
-    const uint32_t format = (p.idesc >> 7) & 7u;
-    const int clusters = std::min(pair_tiles, sms / 2);
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(2 * clusters);
-    config.blockDim = dim3(kGemmThreads);
-    config.dynamicSmemBytes = pair_smem;
-    config.stream = stream;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, gemm_sm100_pair<A_MN, B_MN>, a, *b_pair, p,
-                              gemm_idesc_pair(static_cast<int>(format), A_MN, B_MN));
-  }
-  const size_t smem = 1024 + kGemmStages * (kABytes + kBBytes) + kDrainStageBytes + sizeof(GemmBarriers);
-  cudaError_t e = cudaFuncSetAttribute(gemm_sm100<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
-  const int splits = gemm_splits(p.M, p.N, p.k_tiles, sms);
+  GemmPlan plan = gemm_plan(p.M, p.N, p.k_tiles, sms, b_pair != nullptr);
   const size_t part = static_cast<size_t>(p.M) * p.N;
   // (the sum writes four columns at a time)
-  const bool split = splits > 1 && scratch.bytes >= splits * part * sizeof(float) && p.ldc % 4 == 0 &&
-                     reinterpret_cast<uintptr_t>(p.c) % 16 == 0;
-  if (split) {
-    p.splits = splits;
+  if (plan.splits > 1 && (scratch.bytes < plan.splits * part * sizeof(float) || p.ldc % 4 != 0 ||
+                          reinterpret_cast<uintptr_t>(p.c) % 16 != 0)) {
+    plan.splits = 1;   // the kernel with enough tiles to occupy the chip, as without parts
+    plan.pair = b_pair != nullptr && ((p.N + kPairTile - 1) / kPairTile) * ((p.M + kPairTile - 1) / kPairTile) >= sms / 2;
+  }
+  if (plan.splits > 1) {
+    p.splits = plan.splits;
     p.part_stride = part;
     p.c = scratch.base;
     p.ldc = p.N;
     p.c_kind = p.c_accumulate = 0;
     p.bias = nullptr;
   }
-  const int tiles = ((p.N + kTileN - 1) / kTileN) * ((p.M + kTile - 1) / kTile) * p.splits;
   cudaLaunchAttribute attribute;
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(std::min(tiles, sms));
   config.blockDim = dim3(kGemmThreads);
-  config.dynamicSmemBytes = smem;
   config.stream = stream;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  e = cudaLaunchKernelEx(&config, gemm_sm100<A_MN, B_MN>, a, b, p);
-  if (e != cudaSuccess || !split) return e;
+  cudaError_t e;
+  if (plan.pair) {
+    const int units = ((p.N + kPairTile - 1) / kPairTile) * ((p.M + kPairTile - 1) / kPairTile) * p.splits;
+    config.dynamicSmemBytes =
+        1024 + kPairStages * (kPairABytes + kPairBBytes) + kDrainStageBytes + sizeof(PairGemmBarriers);
+    e = cudaFuncSetAttribute(gemm_sm100_pair<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(config.dynamicSmemBytes));
+    if (e != cudaSuccess) return e;
+    const uint32_t format = (p.idesc >> 7) & 7u;
+    config.gridDim = dim3(2 * std::min(units, sms / 2));
+    e = cudaLaunchKernelEx(&config, gemm_sm100_pair<A_MN, B_MN>, a, *b_pair, p,
+                           gemm_idesc_pair(static_cast<int>(format), A_MN, B_MN));
+  } else {
+    const int units = ((p.N + kTileN - 1) / kTileN) * ((p.M + kTile - 1) / kTile) * p.splits;
+    config.dynamicSmemBytes = 1024 + kGemmStages * (kABytes + kBBytes) + kDrainStageBytes + sizeof(GemmBarriers);
+    e = cudaFuncSetAttribute(gemm_sm100<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(config.dynamicSmemBytes));
+    if (e != cudaSuccess) return e;
+    config.gridDim = dim3(std::min(units, sms));
+    e = cudaLaunchKernelEx(&config, gemm_sm100<A_MN, B_MN>, a, b, p);
+  }
+  if (e != cudaSuccess || plan.splits == 1) return e;
   GemmParams out = params;
-  out.splits = splits;
+  out.splits = plan.splits;
   out.part_stride = part;
   config.gridDim = dim3(static_cast<unsigned>((part / 4 + 255) / 256));
   config.blockDim = dim3(256);
