@@ -2,9 +2,11 @@
 // decoder's default width: 24 query heads over 4 key/value heads).  bf16 tensors, fp32
 // accumulation; every fp32 quantity that becomes an operand of a second product (the
 // probabilities P, the score gradient dS, the upstream gradient dO) enters it as a bf16 high part
-// plus a bf16 remainder, 2^-17 relative, so that the results stay at the level of the fp32 kernels
-// in attn_generic.cu that this width ran on before (forward 1078 us, dQ 2258 us, dK/dV 3798 us at
-// 1000 tokens, against 31, 37 and 82 us here).
+// plus a bf16 remainder, 2^-17 relative, far below the layer's own bf16 rounding points: at 64 to 2048
+// tokens its output and gradients differ from float64 by 2.5e-3 to 4.1e-3, to three digits what they
+// differ by with the fp32 kernels in attn_generic.cu that this width ran on before (the unrounded core by
+// 2e-6, there 3e-7).  At 1000 tokens those took 1078 us forward, 2258 dQ and 3798 dK/dV, these 44, 53
+// and 99 + 11.
 // Reference: src/llm/layers/qwen_attention.cc:68-119 (forward), :140-190 (backward).
 //
 // The width decides the layout.  An fp32 accumulator tile of 128 rows x 256 channels takes half of

@@ -74,10 +74,10 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwdArgs a, long long 
 // A CTA walks blocks of `per_block` tokens: their cos / sin tables go to shared memory, then every
 // warp takes (token, head) rows, a lane owning kPer channels of every 32 * kPer.  HBM bound; the
 // earlier form (a CTA per row with its own sines, the per-row parts written out and reduced from
-// memory by 24 CTAs) took 64 + 71 us at 1000 tokens of 24 and 4 heads of 256, this 29 + 8.
+// memory by 24 CTAs) took 64 + 71 us at 1000 tokens of 24 and 4 heads of 256, this 24 + 10.
 constexpr int kBlockTokens = 8;   // tokens of one block when a token has a single head
 template <int kPer>
-__global__ void __launch_bounds__(256) norm_bwd_kernel(NormBwdArgs a, int per_block) {
+__global__ void __launch_bounds__(256, 4) norm_bwd_kernel(NormBwdArgs a, int per_block) {
   constexpr int kOwn = 8;   // channels a lane owns at width 256
   __shared__ float cosine[kBlockTokens][128], sine[kBlockTokens][128];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
