@@ -80,13 +80,14 @@ int pluto_selftest_bounded_wait(pluto_stream_t stream, unsigned long long limit_
  *   maxima, normalizers   fp32 [batch*heads*seq] at (b*heads+h)*seq + s: the row maximum of the
  *                scaled scores and sum exp(score - max), the state backward reuses.
  * Attention restarts at every multiple of seq (the layer's context_length); scale = 1/sqrt(head_dim).
- * head_dim <= 256.  bf16 with head_dim 64 or 128 runs on the tcgen05 tensor-core kernel, every
+ * head_dim <= 256.  bf16 with head_dim 64, 128 or 256 runs on the tcgen05 tensor-core kernel, every
  * other shape on the exact fp32 kernel. */
 int pluto_attn_fwd(pluto_stream_t stream, const void* qkv, void* out, float* maxima,
                    float* normalizers, int batch, int seq, int heads, int head_dim, int dtype);
 
 /* Bytes of scratch the tensor-core backward needs (host-only query; 0 when the shape has no
- * tensor-core path: it needs bf16 activations and head_dim 64 or 128). */
+ * tensor-core path: it needs bf16 activations and head_dim 64, 128 or 256; width 256 runs on the exact
+ * kernels when the workspace is too small or a tensor is not 16-byte aligned). */
 size_t pluto_attn_bwd_workspace_bytes(int batch, int seq, int heads, int head_dim, int dtype);
 
 /* Stands in for AttentionLayer::bwd_impl + FlashAttentionQueryBackwardKernel +
@@ -133,7 +134,7 @@ int pluto_attn_probs(pluto_stream_t stream, const void* qkv, const float* maxima
  *                (a few heads of a long causal prompt, e.g. one GPU's share of a head-sharded
  *                layer) have their longest query-tile pairs cut along the keys into 2 to 4 CTAs,
  *                combined by a second kernel; the query returns 0 for shapes that are not cut
- * q_heads % kv_heads == 0, head_dim <= 256; head_dim 64/128 runs on tcgen05. */
+ * q_heads % kv_heads == 0, head_dim <= 256; head_dim 64/128/256 runs on tcgen05. */
 int pluto_gqa_prefill_fwd(pluto_stream_t stream, const void* q, const void* gate, const void* k,
                           const void* v, void* out, float* core, float* maxima,
                           float* normalizers, int batch, int seq, int q_heads, int kv_heads,
@@ -185,7 +186,7 @@ int pluto_gqa_prefill_fwd_host(pluto_stream_t stream, const void* q_host, const 
  *    k, v are the prepared tensors of the forward, bf16 or fp32 (dtype); dq fp32
  *    [batch, seq, q_heads, head_dim], dk / dv fp32 [batch, seq, kv_heads, head_dim]: gradients
  *    of the normalised, rotated vectors.  With a workspace of
- *    pluto_gqa_prefill_bwd_workspace_bytes (non-zero for bf16 tensors of head width 64/128) and
+ *    pluto_gqa_prefill_bwd_workspace_bytes (non-zero for bf16 tensors of head width 64/128/256) and
  *    a dense query (q_head_stride == head_dim) the two passes run on tcgen05 with bf16 operands;
  *    with workspace null, or for any other shape, in exact fp32 arithmetic.
  * 3. pluto_qk_prepare_bwd: NormBackwardKernel + ReduceNormKernel (:192-239): inverse partial
@@ -283,7 +284,7 @@ size_t pluto_gqa_decode_workspace_bytes(int batch, int q_heads, int kv_heads, in
  *   max_seq_len  host upper bound of seq_lens (sizes the grid; no device read-back)
  *   out          [batch, Hq, D] (out_dtype);  lse optional fp32 [batch, Hq]
  *   workspace    >= pluto_gqa_decode_workspace_bytes(...) bytes, 16-byte aligned
- * bf16 cache with head_dim 64/128 takes the bandwidth-bound path (bulk copies + mma); anything
+ * bf16 cache with head_dim 64/128/256 takes the bandwidth-bound path (bulk copies + mma); anything
  * else the exact fp32 path.  The result does not depend on which SM ran which chunk. */
 int pluto_gqa_decode(pluto_stream_t stream, const void* q, int q_dtype, const void* gate,
                      int gate_dtype, size_t gate_token_stride, size_t gate_head_stride,
@@ -499,7 +500,8 @@ int pluto_linear_imported_fwd(pluto_stream_t stream, const void* weights, int st
  * (dtype PLUTO_BF16) or fp32 (PLUTO_FP32: the reference's FP16 compute policy); cast = bf16 or
  * fp16 respectively, accumulation fp32, as in the reference's tile MMAs.  The gradients are
  * overwritten, not accumulated, like the reference's.  workspace: device memory of
- * pluto_dense_workspace_bytes (the 2-byte operand copies), 256-byte aligned.  Any positive
+ * pluto_dense_workspace_bytes (the 2-byte operand copies, and parts of products with few tiles;
+ * 2 (r i + i o + r o) + 64 o bytes, extents rounded up to 128, are enough without those), 256-byte aligned.  Any positive
  * extents (tiles are padded inside the workspace). */
 size_t pluto_dense_workspace_bytes(int rows, int input_dim, int output_dim);
 int pluto_dense_fwd(pluto_stream_t stream, const void* input, int dtype, const float* matrix,
