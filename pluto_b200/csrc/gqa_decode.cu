@@ -743,7 +743,7 @@ cudaError_t launch_tc(cudaStream_t stream, const CUtensorMap& map_k, const CUten
 // the grid near the 296 CTAs that are resident at once (up to 400: the ragged lengths leave gaps) and
 // a part above 32 tokens; 16 parts are beyond the portable cluster size and opted into.  Measured, best
 // one-launch form against chunks + merge: 8 units (sequence x KV head) of up to 30000 tokens 33 against
-// 44 us, 16 of 3000 (width 256) 18 / 20, 128 of 2000 22 / 27, 480 of 500 27 / 34.  Above, the merge is a
+// 44 us, 16 of 3000 (width 256, P in two parts; 22 with three) 18 / 20, 128 of 2000 22 / 27, 480 of 500 27 / 34.  Above, the merge is a
 // few per cent and whole-chip balance counts: 240 units of 4000 tokens (width 256) 143 against 113 us,
 // 64 of 20000 171 / 144, 720 of 8000 (width 64) 175 / 138.
 int cluster_parts(const DecodeArgs& a) {
