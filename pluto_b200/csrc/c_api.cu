@@ -519,7 +519,7 @@ int pluto_cached_attention_step(pluto_stream_t stream, const void* q_gate, const
   s.k_cache = cache->k_base; s.v_cache = cache->v_base; s.kv_is_bf16 = cache->dtype == PLUTO_BF16;
   s.token_stride = cache->token_stride;
   s.out = out; s.out_is_bf16 = out_dtype == PLUTO_BF16;
-  s.position = position; s.q_heads = q_heads; s.kv_heads = kv_heads; s.head_dim = head_dim; s.rotary = rotary_dim;
+  s.position = position; s.capacity = cache->page_size; s.q_heads = q_heads; s.kv_heads = kv_heads; s.head_dim = head_dim; s.rotary = rotary_dim;
   s.epsilon = rms_norm_epsilon; s.log_theta = logf(rope_theta);
   s.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
   s.round = round_to_bf16;

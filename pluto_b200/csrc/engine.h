@@ -242,7 +242,7 @@ struct CachedStepArgs {
   size_t token_stride;
   void* out;                    // [q_heads, D]
   int out_is_bf16;
-  int position, q_heads, kv_heads, head_dim, rotary;
+  int position, capacity, q_heads, kv_heads, head_dim, rotary;
   float epsilon, log_theta, scale;
   int round;
 };

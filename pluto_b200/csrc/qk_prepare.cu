@@ -12,6 +12,7 @@
 // tokens of 24 + 4 heads of 256, this 20.  Token (b, t) has RoPE position positions[b] + t.
 #include "common.cuh"
 #include "engine.h"
+#include "qk_rows.cuh"
 
 namespace pluto {
 namespace {
@@ -50,19 +51,14 @@ __device__ __forceinline__ void store_out_vec(void* p, size_t i, int is_bf16, co
 
 template <int kPer>
 __global__ void __launch_bounds__(256) qk_prepare_kernel(PrepareArgs a) {
-  constexpr int kOwn = 8;   // channels a lane owns at width 256
   __shared__ float cosine[128], sine[128];
   const int heads = a.q_heads + a.kv_heads;
   const int token = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int b = token / a.tokens, t = token % a.tokens;
   const int D = a.head_dim, half = a.rotary / 2;
   const int position = (a.positions ? a.positions[b] : a.first_position) + t;
-  if (static_cast<int>(threadIdx.x) < half) {
-    const float angle = static_cast<float>(position) *
-                        expf(static_cast<float>(threadIdx.x) * (-2.0f * a.log_theta / static_cast<float>(a.rotary)));
-    cosine[threadIdx.x] = rnd(cosf(angle), a.round);
-    sine[threadIdx.x] = rnd(sinf(angle), a.round);
-  }
+  if (static_cast<int>(threadIdx.x) < half)
+    rotary_angle(position, threadIdx.x, a.log_theta, a.rotary, a.round, cosine[threadIdx.x], sine[threadIdx.x]);
   __syncthreads();
   // where the token's key/value rows go
   size_t kv_row = 0;
@@ -76,7 +72,6 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(PrepareArgs a) {
     const int page = a.block_table ? a.block_table[static_cast<size_t>(b) * a.max_blocks + position / a.page_size] : b;
     kv_row = static_cast<size_t>(page) * a.page_stride + static_cast<size_t>(position % a.page_size) * a.token_stride;
   }
-  auto channel = [&](int i) { return (i / kPer) * 32 * kPer + lane * kPer; };   // first of the kPer at i
   const int stride = 8 * gridDim.y;
   for (int head = blockIdx.y * 8 + warp; head < heads; head += stride) {
     const bool is_query = head < a.q_heads;
@@ -85,23 +80,21 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(PrepareArgs a) {
     const size_t in0 = is_query ? static_cast<size_t>(token) * a.q_token + static_cast<size_t>(h) * a.q_head : dense;
     const void* in = is_query ? a.q_in : a.k_in;
     const float* norm = is_query ? a.q_norm : a.k_norm;
-    float x[kOwn], value[kOwn];
-    float sq = 0.0f;
+    float x[kRowOwn], value[kRowOwn];
 #pragma unroll
-    for (int i = 0; i < kOwn; i += kPer) {
-      if (channel(i) < D) {
-        load_in_vec<kPer>(in, in0 + channel(i), a.in_is_bf16, x + i);
-        if (!is_query) load_in_vec<kPer>(a.v_in, dense + channel(i), a.in_is_bf16, value + i);
+    for (int i = 0; i < kRowOwn; i += kPer) {
+      const int c = row_channel<kPer>(i, lane);
 #pragma unroll
-        for (int u = 0; u < kPer; ++u) sq += x[i + u] * x[i + u];
+      for (int u = 0; u < kPer; ++u) x[i + u] = 0.0f;
+      if (c < D) {
+        load_in_vec<kPer>(in, in0 + c, a.in_is_bf16, x + i);
+        if (!is_query) load_in_vec<kPer>(a.v_in, dense + c, a.in_is_bf16, value + i);
       }
     }
+    const float inverse = rsqrtf(row_square_sum<kPer>(x, lane) / static_cast<float>(D) + a.epsilon);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    const float inverse = rsqrtf(sq / static_cast<float>(D) + a.epsilon);
-#pragma unroll
-    for (int i = 0; i < kOwn; i += kPer) {
-      const int c = channel(i);
+    for (int i = 0; i < kRowOwn; i += kPer) {
+      const int c = row_channel<kPer>(i, lane);
       if (c >= D) continue;
       float result[kPer];
 #pragma unroll
@@ -115,7 +108,7 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(PrepareArgs a) {
           float rotated = rnd(p[u] * inverse * (1.0f + norm[partner + u]), a.round);
           if (c < half) rotated = -rotated;
           const int f = (c < half ? c : c - half) + u;
-          result[u] = rnd(rnd(result[u] * cosine[f], a.round) + rnd(rotated * sine[f], a.round), a.round);
+          result[u] = rotate(result[u], rotated, cosine[f], sine[f], a.round);
         }
       }
       if (is_query) {

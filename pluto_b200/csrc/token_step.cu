@@ -8,6 +8,7 @@
 //                        gates, recurrence, output norm and gate.
 #include "common.cuh"
 #include "engine.h"
+#include "qk_rows.cuh"
 
 namespace pluto {
 namespace {
@@ -29,216 +30,499 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ------------------------------------------------------------------------------------------------
 // attention
 // ------------------------------------------------------------------------------------------------
-constexpr int kStepWarps = 16;
+// The arithmetic is that of prepare + split decode + merge, in their order, so that a result does not
+// depend on the number of launches: the context is cut into decode_chunk_*'s chunks, a chunk into four
+// token groups with an online softmax each, the groups meet in a chunk and the chunks in the row.  What
+// the one launch saves is the launches and the round trips between them.
+constexpr int kStepMaxChunks = 7;     // chunks of kCachedStepTokens tokens cut as one sequence is
+constexpr int kStepSplit = 256;       // decode_chunk_*'s split_tokens for one sequence of this length
+constexpr float kLog2e = 1.4426950408889634f;
 
-// kPer consecutive cache elements of a row.
-template <int kPer, bool KV_BF16>
-__device__ __forceinline__ void load_row(const void* base, size_t at, float (&v)[kPer]) {
+// Four consecutive channels of a row of the call's input.
+__device__ __forceinline__ void load_input(const void* p, size_t i, int is_bf16, float* v) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = load_any(p, i + u, is_bf16);
+}
+
+// n = R(x * inv * (1 + w)) of one row of width D into `row` (shared memory), by one warp.
+template <int D>
+__device__ __forceinline__ void normalise_row(const void* in, size_t at, int is_bf16, const float* norm, float epsilon,
+                                              int round, int lane, float* row) {
+  float x[kRowOwn];
+#pragma unroll
+  for (int i = 0; i < kRowOwn; i += 4) {
+    const int c = row_channel<4>(i, lane);
+    if (c < D) load_input(in, at + c, is_bf16, x + i);
+    else x[i] = x[i + 1] = x[i + 2] = x[i + 3] = 0.0f;
+  }
+  const float inverse = rsqrtf(row_square_sum<4>(x, lane) / static_cast<float>(D) + epsilon);
+#pragma unroll
+  for (int i = 0; i < kRowOwn; ++i) {
+    const int c = row_channel<4>(i, lane);
+    if (c < D) row[c] = rnd(x[i] * inverse * (1.0f + norm[c]), round);
+  }
+}
+// Rotates that row in place, by the same warp.
+template <int D>
+__device__ __forceinline__ void rotate_row(float* row, const float* cosine, const float* sine, int rotary, int round,
+                                           int lane) {
+  const int half = rotary / 2;
+  float result[D / 32];
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i) {
+    const int c = i * 32 + lane, f = c < half ? c : c - half;
+    result[i] = row[c];
+    if (c < rotary) result[i] = rotate(result[i], c < half ? -row[c + half] : row[c - half], cosine[f], sine[f], round);
+  }
+  __syncwarp();   // every partner has been read
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i) row[i * 32 + lane] = result[i];
+}
+template <int D>
+__device__ __forceinline__ void value_row(const void* in, size_t at, int is_bf16, int round, int lane, float* row) {
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i) row[i * 32 + lane] = rnd(load_any(in, at + i * 32 + lane, is_bf16), round);
+}
+
+// The chunks' (maximum in log2 units, sum) in shared memory -> every chunk's weight; returns the row's sum.
+__device__ __forceinline__ float chunk_weights(const float2* ml, int chunks, float (&weight)[kStepMaxChunks]) {
+  float top = -INFINITY, total = 0.0f;
+#pragma unroll
+  for (int s = 0; s < kStepMaxChunks; ++s)
+    if (s < chunks) top = fmaxf(top, ml[s].x);
+#pragma unroll
+  for (int s = 0; s < kStepMaxChunks; ++s) {
+    weight[s] = s < chunks ? exp2f(ml[s].x - top) : 0.0f;
+    if (s < chunks) total = __fadd_rn(total, __fmul_rn(ml[s].y, weight[s]));
+  }
+  return total;
+}
+// The reference's output stage (cached_attention_ops.cc:120-125): R(R(acc / l) * R(sigmoid(gate))).
+__device__ __forceinline__ void store_gated(const CachedStepArgs& a, int head, int d, float value) {
+  value = rnd(value, a.round);
+  const float gate = load_any(a.q_gate, (static_cast<size_t>(head) * 2 + 1) * a.head_dim + d, a.in_is_bf16);
+  const float sigmoid = rnd(1.0f / (1.0f + expf(-gate)), a.round);
+  store_any(a.out, static_cast<size_t>(head) * a.head_dim + d, a.out_is_bf16, rnd(value * sigmoid, a.round));
+}
+
+// kCount (2, 4 or 8) consecutive cache elements of a row.
+template <int kCount, bool KV_BF16>
+__device__ __forceinline__ void load_cache(const void* base, size_t at, float (&v)[kCount]) {
   if (!KV_BF16) {
     const float* p = static_cast<const float*>(base) + at;
 #pragma unroll
-    for (int i = 0; i < kPer; i += 2) {
+    for (int i = 0; i < kCount; i += 2) {
       const float2 f = *reinterpret_cast<const float2*>(p + i);
       v[i] = f.x; v[i + 1] = f.y;
     }
     return;
   }
   const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(base) + at;
-  uint32_t w[kPer / 2];
-  if (kPer == 8) {
+  uint32_t w[kCount / 2];
+  if (kCount == 8) {
     const uint4 raw = *reinterpret_cast<const uint4*>(p);
-    w[0] = raw.x; w[1 % (kPer / 2)] = raw.y; w[2 % (kPer / 2)] = raw.z; w[3 % (kPer / 2)] = raw.w;
-  } else if (kPer == 4) {
+    w[0] = raw.x; w[1 % (kCount / 2)] = raw.y; w[2 % (kCount / 2)] = raw.z; w[3 % (kCount / 2)] = raw.w;
+  } else if (kCount == 4) {
     const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    w[0] = raw.x; w[1 % (kPer / 2)] = raw.y;
+    w[0] = raw.x; w[1 % (kCount / 2)] = raw.y;
   } else {
     w[0] = *reinterpret_cast<const uint32_t*>(p);
   }
 #pragma unroll
-  for (int i = 0; i < kPer; i += 2) { v[i] = bf16_lo(w[i / 2]); v[i + 1] = bf16_hi(w[i / 2]); }
+  for (int i = 0; i < kCount; i += 2) { v[i] = bf16_lo(w[i / 2]); v[i + 1] = bf16_hi(w[i / 2]); }
 }
 
-// One CTA per query head, head width 32 * kPer, a lane owning kPer consecutive channels of a row.
-// Every CTA prepares its query and its group's new key and value itself (the first head of a group
-// writes the two into the cache); the scores of all tokens go to shared memory, so the softmax is
-// two-pass fp32 as in the reference.  K and V are read once per query head: with at most
-// kCachedStepTokens rows they come from L2.
-template <int kPer, bool KV_BF16>
+// fp32 products, one CTA per query head: every CTA prepares its query and its group's new key and value
+// itself (the first head of a group writes the two into the cache).  K is read by eight tokens per warp,
+// four lanes each: a lane sums the channels 8 j .. 8 j + 7 of every 32, which are the chains that the
+// decode kernel's lanes form, and the butterfly over a token's chains runs half in shuffles and half in
+// the lane.  With at most kCachedStepTokens rows, K and V come from L2 for the heads of a group.
+constexpr int kStepWarps = 16;
+template <int D, bool KV_BF16>
 __global__ void __launch_bounds__(kStepWarps * 32) cached_step_kernel(CachedStepArgs a) {
-  constexpr int D = 32 * kPer;
-  __shared__ float cosine[128], sine[128], vec[3][D];   // query, new key, new value
+  constexpr int kPer = D / 32, kUnits = 4 * kStepMaxChunks;
+  __shared__ float cosine[128], sine[128];
+  __shared__ __align__(16) float query[D], new_key[D], new_value[D];
   __shared__ float score[kCachedStepTokens];
-  __shared__ float acc_s[kStepWarps][D];
-  __shared__ float red[2][kStepWarps];
+  __shared__ float2 weigh[kCachedStepTokens];        // (p, correction of what came before)
+  __shared__ float unit_acc[kUnits][D];              // unit: a token group of a chunk
+  __shared__ float2 unit_ml[kUnits], chunk_ml[kStepMaxChunks];
   const int head = blockIdx.x, group = a.q_heads / a.kv_heads, kv_head = head / group;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, c0 = lane * kPer;
-  const int length = a.position + 1, half = a.rotary / 2;
-  const size_t row0 = static_cast<size_t>(kv_head) * D + c0;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int length = a.position + 1, chunks = decode_chunk_count(length, kStepSplit);
+  const size_t head_row = static_cast<size_t>(kv_head) * D;
+  const int last_row = max(a.position - 1, 0);
 
   pdl_wait();   // every input, the weights too: the kernel before this one may have written them
   pdl_launch_dependents();   // the next launch sets itself up meanwhile and waits for this grid in turn
-  float w_norm[kPer];
-  if (warp < 2) {
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) w_norm[i] = 1.0f + (warp == 0 ? a.q_norm : a.k_norm)[c0 + i];
-  }
-  // The first rows of the cache and the gate of this thread's output channel are requested before
-  // anything waits: at short contexts the kernel is a chain of memory round trips.
-  constexpr int kAhead = 2;
-  float k_ahead[kAhead][kPer], v_ahead[kAhead][kPer];
-#pragma unroll
-  for (int u = 0; u < kAhead; ++u) {
-    const int t = warp + u * kStepWarps;
-    if (t < a.position) {
-      load_row<kPer, KV_BF16>(a.k_cache, static_cast<size_t>(t) * a.token_stride + row0, k_ahead[u]);
-      load_row<kPer, KV_BF16>(a.v_cache, static_cast<size_t>(t) * a.token_stride + row0, v_ahead[u]);
-    }
-  }
-  float gate = 0.0f;
-  if (threadIdx.x < D) gate = load_any(a.q_gate, static_cast<size_t>(head) * 2 * D + D + threadIdx.x, a.in_is_bf16);
-  if (static_cast<int>(threadIdx.x) < half) {
-    const float angle = static_cast<float>(a.position) *
-                        expf(static_cast<float>(threadIdx.x) * (-2.0f * a.log_theta / static_cast<float>(a.rotary)));
-    cosine[threadIdx.x] = rnd(cosf(angle), a.round);
-    sine[threadIdx.x] = rnd(sinf(angle), a.round);
-  }
-  // warp 0: query, warp 1: new key; R(x * inv * (1 + w)), then the rotation in qk_prepare.cu's steps
-  float n[kPer];
-  if (warp < 2) {
-    const void* in = warp == 0 ? a.q_gate : a.k;
-    const size_t in0 = warp == 0 ? static_cast<size_t>(head) * 2 * D : static_cast<size_t>(kv_head) * D;
-    float sq = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) n[i] = load_any(in, in0 + c0 + i, a.in_is_bf16);
-    // the sum of squares in qk_prepare.cu's order (four channels of every 128 per lane): the prepared
-    // vectors of the two kernels are equal bit for bit
-#pragma unroll
-    for (int c = lane * 4; c < D; c += 128)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float x = load_any(in, in0 + c + u, a.in_is_bf16);
-        sq += x * x;
-      }
-    const float inverse = rsqrtf(warp_sum(sq) / static_cast<float>(D) + a.epsilon);
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      n[i] = rnd(n[i] * inverse * w_norm[i], a.round);
-      vec[warp][c0 + i] = n[i];
-    }
-  } else if (warp == 2) {
+  // K of this lane's first token is requested before anything waits: at short contexts the kernel is a
+  // chain of memory round trips
+  const int own = warp * 8 + lane / 4, part = lane % 4 * 8;
+  constexpr int kRaw = KV_BF16 ? 1 : 2;   // 16-byte pieces of eight elements
+  auto load_key = [&](int t, uint4 (&raw)[kPer][kRaw]) {
+    const size_t at = static_cast<size_t>(min(t, last_row)) * a.token_stride + head_row + part;
 #pragma unroll
     for (int i = 0; i < kPer; ++i)
-      vec[2][c0 + i] = rnd(load_any(a.v, static_cast<size_t>(kv_head) * D + c0 + i, a.in_is_bf16), a.round);
-  }
-  __syncthreads();
-  if (warp < 2) {
-    float result[kPer];
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int c = c0 + i;
-      result[i] = n[i];
-      if (c < a.rotary) {
-        const int f = c < half ? c : c - half;
-        const float partner = c < half ? -vec[warp][c + half] : vec[warp][c - half];
-        result[i] = rnd(rnd(n[i] * cosine[f], a.round) + rnd(partner * sine[f], a.round), a.round);
-      }
-    }
-    __syncwarp();   // every partner has been read
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) vec[warp][c0 + i] = result[i];
-    if (warp == 1 && head % group == 0) {
-#pragma unroll
-      for (int i = 0; i < kPer; ++i)
-        store_any(a.k_cache, static_cast<size_t>(a.position) * a.token_stride + row0 + i, KV_BF16, result[i]);
-    }
-  } else if (warp == 2 && head % group == 0) {
-#pragma unroll
-    for (int i = 0; i < kPer; ++i)
-      store_any(a.v_cache, static_cast<size_t>(a.position) * a.token_stride + row0 + i, KV_BF16, vec[2][c0 + i]);
-  }
-  __syncthreads();
-
-  float q[kPer];
-#pragma unroll
-  for (int i = 0; i < kPer; ++i) q[i] = vec[0][c0 + i];
-  float top = -INFINITY;
-  auto attend = [&](int t, const float (&k)[kPer]) {
-    float dot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) dot = fmaf(k[i], q[i], dot);
-    dot = warp_sum(dot) * a.scale;
-    if (lane == 0) score[t] = dot;
-    top = fmaxf(top, dot);
+      for (int u = 0; u < kRaw; ++u)
+        raw[i][u] = KV_BF16 ? *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.k_cache) + at + i * 32)
+                            : *reinterpret_cast<const uint4*>(static_cast<const float*>(a.k_cache) + at + i * 32 + u * 4);
   };
+  uint4 keys[kPer][kRaw];
+  load_key(own, keys);
+  if (static_cast<int>(threadIdx.x) < a.rotary / 2)
+    rotary_angle(a.position, threadIdx.x, a.log_theta, a.rotary, a.round, cosine[threadIdx.x], sine[threadIdx.x]);
+  if (warp == 0)
+    normalise_row<D>(a.q_gate, static_cast<size_t>(head) * 2 * D, a.in_is_bf16, a.q_norm, a.epsilon, a.round, lane, query);
+  else if (warp == 1)
+    normalise_row<D>(a.k, head_row, a.in_is_bf16, a.k_norm, a.epsilon, a.round, lane, new_key);
+  else if (warp == 2)
+    value_row<D>(a.v, head_row, a.in_is_bf16, a.round, lane, new_value);
+  __syncthreads();   // (the rotary tables)
+  if (warp < 2) rotate_row<D>(warp == 0 ? query : new_key, cosine, sine, a.rotary, a.round, lane);
+  if (warp == 1 || warp == 2) {   // attended to as the cache holds them
+    float* row = warp == 1 ? new_key : new_value;
+    void* cache = warp == 1 ? a.k_cache : a.v_cache;
 #pragma unroll
-  for (int u = 0; u < kAhead; ++u)
-    if (warp + u * kStepWarps < a.position) attend(warp + u * kStepWarps, k_ahead[u]);
-#pragma unroll 8
-  for (int t = warp + kAhead * kStepWarps; t < a.position; t += kStepWarps) {
-    float k[kPer];
-    load_row<kPer, KV_BF16>(a.k_cache, static_cast<size_t>(t) * a.token_stride + row0, k);
-    attend(t, k);
+    for (int i = 0; i < kPer; ++i) {
+      const int c = i * 32 + lane;
+      row[c] = rnd(row[c], KV_BF16);
+      if (head % group == 0) store_any(cache, static_cast<size_t>(a.position) * a.token_stride + head_row + c, KV_BF16, row[c]);
+    }
   }
-  if (warp == a.position % kStepWarps) {   // the new token, as the cache holds it
-    float dot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) dot = fmaf(rnd(vec[1][c0 + i], KV_BF16), q[i], dot);
-    dot = warp_sum(dot) * a.scale;
-    if (lane == 0) score[a.position] = dot;
-    top = fmaxf(top, dot);
-  }
-  if (lane == 0) red[0][warp] = top;
-  __syncthreads();
-  top = red[0][0];
-#pragma unroll
-  for (int w = 1; w < kStepWarps; ++w) top = fmaxf(top, red[0][w]);
-  float sum = 0.0f;
-  for (int t = threadIdx.x; t < length; t += kStepWarps * 32) {
-    const float p = expf(score[t] - top);
-    score[t] = p;
-    sum += p;
-  }
-  sum = warp_sum(sum);
-  if (lane == 0) red[1][warp] = sum;
   __syncthreads();
 
-  float acc[kPer];
+  for (int t0 = 0; t0 < length; t0 += 8 * kStepWarps) {   // (uniform: the shuffles want whole warps)
+    const int t = t0 + own;
+    if (t0 > 0) load_key(t, keys);
+    float dot[8];
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) acc[i] = 0.0f;
+    for (int r = 0; r < 8; ++r) dot[r] = 0.0f;
 #pragma unroll
-  for (int u = 0; u < kAhead; ++u)
-    if (warp + u * kStepWarps < a.position) {
-      const float p = score[warp + u * kStepWarps];
+    for (int i = 0; i < kPer; ++i) {
+      float q[8], k[8];
+      *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(query + i * 32 + part);
+      *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(query + i * 32 + part + 4);
+      const uint32_t* raw = reinterpret_cast<const uint32_t*>(keys[i]);
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) acc[i] = fmaf(p, v_ahead[u][i], acc[i]);
+      for (int r = 0; r < 8; ++r)
+        k[r] = !KV_BF16 ? __uint_as_float(raw[r % (4 * kRaw)]) : r % 2 ? bf16_hi(raw[r / 2]) : bf16_lo(raw[r / 2]);
+      if (t >= a.position) {   // the new token (and whatever past the end: not stored)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) k[r] = new_key[i * 32 + part + r];
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) dot[r] = fmaf(k[r], q[r], dot[r]);
     }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 2);
+      dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 1);
+    }
+    const float sum = ((dot[0] + dot[4]) + (dot[2] + dot[6])) + ((dot[1] + dot[5]) + (dot[3] + dot[7]));
+    if (t < length && lane % 4 == 0) score[t] = __fmul_rn(sum, a.scale);
+  }
+  __syncthreads();
+
+  for (int unit = warp; unit < 4 * chunks; unit += kStepWarps) {
+    const int chunk = unit / 4, begin = decode_chunk_begin(chunk, kStepSplit) + unit % 4;
+    const int end = min(length, decode_chunk_begin(chunk, kStepSplit) + decode_chunk_tokens(chunk, kStepSplit));
+    const int count = begin < end ? (end - begin + 3) / 4 : 0;   // tokens begin, begin + 4, ... (64 at most)
+    // the running maxima of the online softmax, all at once
+    float top = -INFINITY;
+#pragma unroll
+    for (int k0 = 0; k0 < 64; k0 += 32) {
+      const int t = begin + (k0 + lane) * 4;
+      const float s = k0 + lane < count ? score[t] : -INFINITY;
+      float m = s;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float below = __shfl_up_sync(0xffffffffu, m, o);
+        if (lane >= o) m = fmaxf(m, below);
+      }
+      m = fmaxf(m, top);
+      float before = __shfl_up_sync(0xffffffffu, m, 1);
+      if (lane == 0) before = top;
+      if (k0 + lane < count) weigh[t] = make_float2(expf(s - m), expf(before - m));
+      top = __shfl_sync(0xffffffffu, m, 31);
+    }
+    __syncwarp();
+    float acc[kPer], l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) acc[i] = 0.0f;
 #pragma unroll 8
-  for (int t = warp + kAhead * kStepWarps; t < a.position; t += kStepWarps) {
-    float v[kPer];
-    load_row<kPer, KV_BF16>(a.v_cache, static_cast<size_t>(t) * a.token_stride + row0, v);
-    const float p = score[t];
+    for (int k = 0; k < count; ++k) {
+      const int t = begin + 4 * k;
+      float v[kPer];
+      // (the new token is the last one; its row of the cache may be another CTA's to write at this moment)
+      load_cache<kPer, KV_BF16>(a.v_cache, static_cast<size_t>(min(t, last_row)) * a.token_stride + head_row + lane * kPer, v);
+      if (t >= a.position) {
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) acc[i] = fmaf(p, v[i], acc[i]);
+        for (int i = 0; i < kPer; ++i) v[i] = new_value[lane * kPer + i];
+      }
+      const float2 w = weigh[t];
+      l = fmaf(l, w.y, w.x);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) acc[i] = fmaf(w.x, v[i], __fmul_rn(acc[i], w.y));
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) unit_acc[unit][lane * kPer + i] = acc[i];
+    if (lane == 0) unit_ml[unit] = make_float2(top, l);
   }
-  if (warp == a.position % kStepWarps) {
+  __syncthreads();
+  auto chunk_top = [&](int s) {
+    return fmaxf(fmaxf(unit_ml[4 * s].x, unit_ml[4 * s + 1].x), fmaxf(unit_ml[4 * s + 2].x, unit_ml[4 * s + 3].x));
+  };
+  if (static_cast<int>(threadIdx.x) < chunks) {
+    const int s = threadIdx.x;
+    const float top = chunk_top(s);
+    float l = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) acc[i] = fmaf(score[a.position], rnd(vec[2][c0 + i], KV_BF16), acc[i]);
+    for (int w = 0; w < 4; ++w) l = fmaf(unit_ml[4 * s + w].y, expf(unit_ml[4 * s + w].x - top), l);
+    chunk_ml[s] = make_float2(__fmul_rn(top, kLog2e), l);
   }
-#pragma unroll
-  for (int i = 0; i < kPer; ++i) acc_s[warp][c0 + i] = acc[i];
   __syncthreads();
   if (threadIdx.x >= D) return;
-  // the warps' parts in double (a warp holds few terms at these lengths): the quotient is then good to
-  // the last bit, and its rounding to bf16 falls where the exact result's would
-  double parts = 0.0, total = 0.0;
+  float weight[kStepMaxChunks];
+  const float total = chunk_weights(chunk_ml, chunks, weight);
+  float acc = 0.0f;
 #pragma unroll
-  for (int w = 0; w < kStepWarps; ++w) {
-    parts += static_cast<double>(acc_s[w][threadIdx.x]);
-    total += static_cast<double>(red[1][w]);
+  for (int s = 0; s < kStepMaxChunks; ++s) {
+    if (s >= chunks) break;
+    const float top = chunk_top(s);
+    float sum = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) sum = fmaf(unit_acc[4 * s + w][threadIdx.x], expf(unit_ml[4 * s + w].x - top), sum);
+    acc = fmaf(sum, weight[s], acc);
   }
-  float value = rnd(static_cast<float>(parts / total), a.round);
-  value = rnd(value * rnd(1.0f / (1.0f + expf(-gate)), a.round), a.round);
-  store_any(a.out, static_cast<size_t>(head) * D + threadIdx.x, a.out_is_bf16, value);
+  store_gated(a, head, threadIdx.x, acc / total);
+}
+
+// Products on the tensor cores (mma.sync), where the decode kernel takes them: bf16 cache and rounded
+// queries of width 64 or 128.  One CTA of eight warps per key/value head, whose query heads are the rows
+// of the tile; a warp owns 16 tokens of every 64, so four warps make a chunk and the CTA walks two at a
+// time.  P enters P V as a bf16 high part and a remainder.  A warp's K and V rows come by asynchronous
+// copies into shared memory of its own; the first are requested before anything waits.
+constexpr int kTcStepWarps = 8;
+template <int D>
+struct TcStepLayout {
+  static constexpr int kPitch = D + 8;                              // bf16 elements: rows 16 bytes further round the banks
+  static constexpr int kTileBytes = 16 * kPitch * 2;                // K or V of a warp
+  static constexpr int kOwnBytes = 2 * kTileBytes;                  // both; later fp32 [16][D]
+  static constexpr int kVectors = kTcStepWarps * kOwnBytes;         // fp32 [18][D]: queries, new key, new value
+  static constexpr int kChunkAcc = kVectors + 18 * D * 4;           // fp32 [chunk][16][D]
+  static constexpr int kMl = kChunkAcc + kStepMaxChunks * 16 * D * 4;   // float2 [16][chunks], then [warp][16]
+  static constexpr int kTotal = kMl + (kStepMaxChunks + kTcStepWarps) * 16 * 8;
+  static_assert(16 * D * 4 <= kOwnBytes, "a warp's accumulators fit its tiles");
+};
+
+__device__ __forceinline__ void step_ldmatrix(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void step_ldmatrix_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void step_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int D>
+__global__ void __launch_bounds__(kTcStepWarps * 32) cached_step_tc_kernel(CachedStepArgs a) {
+  using Layout = TcStepLayout<D>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ float cosine[64], sine[64];
+  float* vectors = reinterpret_cast<float*>(smem + Layout::kVectors);
+  float* chunk_acc = reinterpret_cast<float*>(smem + Layout::kChunkAcc);
+  float2* chunk_ml = reinterpret_cast<float2*>(smem + Layout::kMl);
+  float2* warp_ml = chunk_ml + kStepMaxChunks * 16;
+  const int kv_head = blockIdx.x, group = a.q_heads / a.kv_heads;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, quarter = warp % 4;
+  const int length = a.position + 1, chunks = decode_chunk_count(length, kStepSplit);
+  const size_t head_row = static_cast<size_t>(kv_head) * D;
+  uint8_t* own = smem + warp * Layout::kOwnBytes;
+  float* own_acc = reinterpret_cast<float*>(own);
+  const uint32_t k_tile = smem_u32(own), v_tile = k_tile + Layout::kTileBytes;
+
+  pdl_wait();
+  pdl_launch_dependents();
+  // The cached rows of the 16 tokens from t0 on, the new token's and zeros past the end.
+  auto request = [&](int t0) {
+    constexpr int kPieces = D / 8;   // 16-byte pieces of a row
+    for (int e = lane; e < 2 * 16 * kPieces; e += 32) {
+      const int value = e / (16 * kPieces), r = e / kPieces % 16, c = e % kPieces * 8, t = t0 + r;
+      const uint32_t to = (value ? v_tile : k_tile) + (r * Layout::kPitch + c) * 2;
+      if (t < a.position) {
+        const __nv_bfloat16* from = static_cast<const __nv_bfloat16*>(value ? a.v_cache : a.k_cache) +
+                                    static_cast<size_t>(t) * a.token_stride + head_row + c;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+      } else if (t > a.position) {
+        sts_b32x4(to, 0u, 0u, 0u, 0u);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int first = decode_chunk_begin(warp / 4, kStepSplit) + quarter * 16;
+  if (first < length) request(first);
+  if (static_cast<int>(threadIdx.x) < a.rotary / 2)
+    rotary_angle(a.position, threadIdx.x, a.log_theta, a.rotary, a.round, cosine[threadIdx.x], sine[threadIdx.x]);
+  for (int r = warp; r < group + 2; r += kTcStepWarps) {
+    float* row = vectors + r * D;
+    if (r < group)
+      normalise_row<D>(a.q_gate, (static_cast<size_t>(kv_head) * group + r) * 2 * D, a.in_is_bf16, a.q_norm, a.epsilon,
+                       a.round, lane, row);
+    else if (r == group)
+      normalise_row<D>(a.k, head_row, a.in_is_bf16, a.k_norm, a.epsilon, a.round, lane, row);
+    else
+      value_row<D>(a.v, head_row, a.in_is_bf16, a.round, lane, row);
+  }
+  __syncthreads();   // (the rotary tables)
+  for (int r = warp; r < group + 2; r += kTcStepWarps) {
+    float* row = vectors + r * D;
+    if (r <= group) rotate_row<D>(row, cosine, sine, a.rotary, a.round, lane);
+    if (r >= group) {
+      void* cache = r == group ? a.k_cache : a.v_cache;
+#pragma unroll
+      for (int i = 0; i < D / 32; ++i)
+        store_any(cache, static_cast<size_t>(a.position) * a.token_stride + head_row + i * 32 + lane, 1, row[i * 32 + lane]);
+    }
+  }
+  __syncthreads();
+  // A fragments of Q: rows = query heads of this KV head (rows >= group are zero).
+  uint32_t qf[D / 16][4];
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // rows lane / 4, + 8; columns 0-7, 8-15 of the step
+      const int r = lane / 4 + (i & 1) * 8, c = ks * 16 + (i >> 1) * 8 + (lane % 4) * 2;
+      qf[ks][i] = r < group ? pack_bf16(vectors[r * D + c], vectors[r * D + c + 1]) : 0u;
+    }
+  const float scale_log2 = a.scale * kLog2e;
+  for (int chunk0 = 0; chunk0 < chunks; chunk0 += kTcStepWarps / 4) {
+    const int chunk = chunk0 + warp / 4, begin = decode_chunk_begin(chunk, kStepSplit);
+    const int end = min(length, begin + decode_chunk_tokens(chunk, kStepSplit));
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, o[D / 8][4];
+#pragma unroll
+    for (int nb = 0; nb < D / 8; ++nb)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[nb][i] = 0.0f;
+    if (chunk0 > 0) __syncthreads();   // the chunks before have been read
+    for (int t0 = begin + quarter * 16; t0 < end; t0 += 64) {
+      if (t0 != first) request(t0);
+      const int fresh = a.position - t0;   // the new token's row of the tile, where it has one
+      if (fresh >= 0 && fresh < 16 && lane < D / 8) {
+#pragma unroll
+        for (int value = 0; value < 2; ++value) {
+          const float* row = vectors + (group + value) * D + lane * 8;
+          sts_b32x4((value ? v_tile : k_tile) + (fresh * Layout::kPitch + lane * 8) * 2, pack_bf16(row[0], row[1]),
+                    pack_bf16(row[2], row[3]), pack_bf16(row[4], row[5]), pack_bf16(row[6], row[7]));
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      float s[2][4] = {};
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int kp = 0; kp < D / 32; ++kp) {
+          uint32_t kf[4];
+          step_ldmatrix(kf, k_tile + ((nb * 8 + lane % 8) * Layout::kPitch + kp * 32 + lane / 8 * 8) * 2);
+          step_mma(s[nb], qf[2 * kp], kf[0], kf[1]);
+          step_mma(s[nb], qf[2 * kp + 1], kf[2], kf[3]);
+        }
+      const int token0 = t0 + (lane % 4) * 2;
+      float tile_max[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s[nb][i] = token0 + nb * 8 + (i & 1) < end ? __fmul_rn(s[nb][i], scale_log2) : -INFINITY;
+          tile_max[i >> 1] = fmaxf(tile_max[i >> 1], s[nb][i]);
+        }
+      uint32_t pf[4], pl[4];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 1));
+        tile_max[r] = fmaxf(tile_max[r], __shfl_xor_sync(0xffffffffu, tile_max[r], 2));
+        const float m_new = fmaxf(m_run[r], tile_max[r]);
+        const float m_safe = m_new == -INFINITY ? 0.0f : m_new;
+        const float correction = fast_exp2(m_run[r] - m_safe);
+        const float p00 = fast_exp2(s[0][2 * r] - m_safe), p01 = fast_exp2(s[0][2 * r + 1] - m_safe);
+        const float p10 = fast_exp2(s[1][2 * r] - m_safe), p11 = fast_exp2(s[1][2 * r + 1] - m_safe);
+        float sum = p00 + p01 + p10 + p11;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        l_run[r] = fmaf(l_run[r], correction, sum);
+        m_run[r] = m_new;
+        pf[r] = pack_bf16(p00, p01);      // tokens 0-7
+        pf[2 + r] = pack_bf16(p10, p11);  // tokens 8-15
+        pl[r] = pack_bf16(p00 - bf16_lo(pf[r]), p01 - bf16_hi(pf[r]));
+        pl[2 + r] = pack_bf16(p10 - bf16_lo(pf[2 + r]), p11 - bf16_hi(pf[2 + r]));
+#pragma unroll
+        for (int nb = 0; nb < D / 8; ++nb) {
+          o[nb][2 * r] *= correction;
+          o[nb][2 * r + 1] *= correction;
+        }
+      }
+#pragma unroll
+      for (int np = 0; np < D / 16; ++np) {
+        uint32_t vf[4];
+        step_ldmatrix_trans(vf, v_tile + ((lane / 8 % 2 * 8 + lane % 8) * Layout::kPitch + np * 16 + lane / 16 * 8) * 2);
+        step_mma(o[2 * np], pf, vf[0], vf[1]);
+        step_mma(o[2 * np], pl, vf[0], vf[1]);
+        step_mma(o[2 * np + 1], pf, vf[2], vf[3]);
+        step_mma(o[2 * np + 1], pl, vf[2], vf[3]);
+      }
+      __syncwarp();   // the tiles have been read
+    }
+    if (chunk < chunks) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = lane / 4 + i * 8;
+#pragma unroll
+        for (int nb = 0; nb < D / 8; ++nb)
+          *reinterpret_cast<float2*>(own_acc + r * D + nb * 8 + (lane % 4) * 2) = make_float2(o[nb][2 * i], o[nb][2 * i + 1]);
+        if (lane % 4 == 0) warp_ml[warp * 16 + r] = make_float2(m_run[i], l_run[i]);
+      }
+    }
+    __syncthreads();
+    // the four token groups of a chunk, in order
+    for (int e = threadIdx.x; e < kTcStepWarps / 4 * group * D; e += kTcStepWarps * 32) {
+      const int which = e / (group * D), r = e / D % group, d = e % D, s = chunk0 + which;
+      if (s >= chunks) break;
+      const float2* ml = warp_ml + which * 64 + r;
+      const float top = fmaxf(fmaxf(ml[0].x, ml[16].x), fmaxf(ml[32].x, ml[48].x));
+      float acc = 0.0f, l = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float f = fast_exp2(ml[16 * w].x - top);
+        const float* from = reinterpret_cast<const float*>(smem + (which * 4 + w) * Layout::kOwnBytes);
+        acc = fmaf(from[r * D + d], f, acc);
+        l = fmaf(ml[16 * w].y, f, l);
+      }
+      chunk_acc[(s * 16 + r) * D + d] = acc;
+      if (d == 0) chunk_ml[r * kStepMaxChunks + s] = make_float2(top, l);
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < group * D; e += kTcStepWarps * 32) {
+    const int r = e / D, d = e % D;
+    float weight[kStepMaxChunks], acc = 0.0f;
+    const float total = chunk_weights(chunk_ml + r * kStepMaxChunks, chunks, weight);
+#pragma unroll
+    for (int s = 0; s < kStepMaxChunks; ++s)
+      if (s < chunks) acc = fmaf(chunk_acc[(s * 16 + r) * D + d], weight[s], acc);
+    store_gated(a, kv_head * group + r, d, acc / total);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -376,21 +660,38 @@ bool cached_step_supported(const CachedStepArgs& a) {
          (reinterpret_cast<uintptr_t>(a.v_cache) & 15u) == 0;
 }
 
-cudaError_t cached_step(cudaStream_t stream, const CachedStepArgs& a) {
-  using Kernel = void (*)(CachedStepArgs);
-  static const Kernel kernels[3][2] = {{cached_step_kernel<2, false>, cached_step_kernel<2, true>},
-                                       {cached_step_kernel<4, false>, cached_step_kernel<4, true>},
-                                       {cached_step_kernel<8, false>, cached_step_kernel<8, true>}};
+namespace {
+template <typename Kernel>
+cudaError_t launch_step(Kernel kernel, int ctas, int threads, size_t smem, cudaStream_t stream, const CachedStepArgs& a) {
+  if (smem > 0) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
   cudaLaunchAttribute attribute;
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(a.q_heads);
-  config.blockDim = dim3(kStepWarps * 32);
+  config.gridDim = dim3(ctas);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
   config.stream = stream;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernels[a.head_dim / 128][a.kv_is_bf16 ? 1 : 0], a);
+  return cudaLaunchKernelEx(&config, kernel, a);
+}
+}  // namespace
+
+cudaError_t cached_step(cudaStream_t stream, const CachedStepArgs& a) {
+  // the decode kernel's rule for its tensor-core form, less width 256
+  const bool tc = a.kv_is_bf16 && a.round && a.head_dim <= 128 && a.q_heads / a.kv_heads <= 16 && a.capacity % 16 == 0;
+  if (tc && a.head_dim == 128)
+    return launch_step(cached_step_tc_kernel<128>, a.kv_heads, kTcStepWarps * 32, TcStepLayout<128>::kTotal, stream, a);
+  if (tc) return launch_step(cached_step_tc_kernel<64>, a.kv_heads, kTcStepWarps * 32, TcStepLayout<64>::kTotal, stream, a);
+  using Kernel = void (*)(CachedStepArgs);
+  static const Kernel kernels[3][2] = {{cached_step_kernel<64, false>, cached_step_kernel<64, true>},
+                                       {cached_step_kernel<128, false>, cached_step_kernel<128, true>},
+                                       {cached_step_kernel<256, false>, cached_step_kernel<256, true>}};
+  return launch_step(kernels[a.head_dim / 128][a.kv_is_bf16 ? 1 : 0], a.q_heads, kStepWarps * 32, 0, stream, a);
 }
 
 bool gdn_token_supported(int key_heads, int value_heads, int key_dim, int value_dim, int width) {

@@ -103,3 +103,38 @@ def test_delta_step_matches_its_four_launches(key_heads, value_heads, dk, dv, ta
         bound = (2 ** -6 if rounded or code else 2e-5) * want.float().abs() + 2e-5 * want.float().abs().max()
         assert ((out.float() - want.float()).abs() <= bound).all()
     assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("heads,dim,rotary,cache_dtype,rounded", [
+    (*shape, torch.float32, rounded) for shape in (((24, 4), 256, 64), ((5, 1), 128, 128), ((3, 3), 64, 12))
+    for rounded in (True, False)] + [((24, 4), 256, 64, torch.bfloat16, False)])
+def test_cached_step_is_the_separate_launches_bit_for_bit(heads, dim, rotary, cache_dtype, rounded):
+    """The step forms every sum in the order of prepare + decode + merge, so the number of launches does
+    not show in the result: keys, values and output, one row to the longest context, at the edges of the
+    64-token chunks.  (fp32 output of calls that the decode entry point gives to its plain kernel.)"""
+    hq, hkv = heads
+    p = FullAttentionParameters(query_heads=hq, key_value_heads=hkv, head_dim=dim, rotary_dim=rotary, capacity=1024,
+                                round_to_bfloat16=rounded)
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    keys, values, wq, wk = rnd(1024, hkv, dim).bfloat16(), rnd(1024, hkv, dim).bfloat16(), rnd(dim) * 0.1, rnd(dim) * 0.1
+    for position in (0, 1, 3, 4, 31, 63, 64, 65, 127, 128, 255, 256, 300, 511, 512, 1023):
+        qg, k, v = rnd(hq, 2, dim), rnd(hkv, dim), rnd(hkv, dim)
+        caches = [KeyValueCache.Create(1024, hkv, dim, cache_dtype) for _ in range(2)]
+        for cache in caches:
+            cache.keys().copy_(keys)
+            cache.values().copy_(values)
+            cache.position_ = position
+        out = torch.empty(hq, dim, device="cuda")
+        CachedAttentionStep(p, caches[0], qg, k, v, wq, wk, out)
+        queries = torch.empty(1, hq, dim, device="cuda", dtype=torch.bfloat16 if rounded else torch.float32)
+        at = torch.tensor([position], dtype=torch.int32, device="cuda")
+        _capi.check(_capi.fast().pluto_qk_prepare(
+            stream(), qg.data_ptr(), k.data_ptr(), v.data_ptr(), 0, 2 * hq * dim, 2 * dim, wq.data_ptr(), wk.data_ptr(),
+            at.data_ptr(), queries.data_ptr(), int(rounded), caches[1].packed_layout(), 1, 1, hq, hkv, dim, rotary,
+            p.rms_norm_epsilon, p.rope_theta, int(rounded)))
+        want = gqa_decode(queries, caches[1].keys()[None], caches[1].values()[None], at + 1, position + 1,
+                          gate=qg[None, :, 1], round_to_bfloat16=rounded, out=torch.empty(1, hq, dim, device="cuda"))[0]
+        assert torch.equal(caches[0].keys(), caches[1].keys()) and torch.equal(caches[0].values(), caches[1].values())
+        assert torch.equal(out, want), position
+    assert _capi.kernel_status() == 0
