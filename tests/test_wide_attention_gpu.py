@@ -41,8 +41,8 @@ def test_forward(shape):
     q, k, v, _ = make(shape)
     want, m, l = reference(q, k, v)
     got = gqa_prefill(q, k, v, want_core=True, want_stats=True)
-    # P enters P V as two bf16 parts (2^-17 relative) and ex2.approx is good to 2^-22; values are sums
-    # of |p| <= 1 weighted N(0, 1) entries, so 2^-15 absolute leaves room for the fp32 accumulation
+    # P enters P V with 24 bits and ex2.approx is good to 2^-22; values are sums of |p| <= 1 weighted
+    # N(0, 1) entries: 2^-15 absolute is far above that (test_error_is_that_of_fp32_products is the tight one)
     assert (got["core"].double() - want).abs().max().item() < 3.1e-5
     assert torch.equal(got["out"], got["core"].bfloat16())
     assert (got["maxima"].view_as(m).double() - m).abs().max().item() < 1e-5
@@ -88,10 +88,30 @@ def test_backward_matches_exact_kernels_and_repeats(shape):
     again = backward(q, k, v, d_out, stats, True)
     for name, x, y, z in zip(("dq", "dk", "dv"), got, exact, again):
         assert torch.equal(x, z), name
-        # Every operand carries 16 bits (2^-17 relative, random signs), products accumulate in fp32: 3e-5
-        # of the largest gradient.  Where dP - delta cancels (a single visible key: dS is exactly 0), what is
-        # left is the rounding of dP's own terms: 256 products of N(0, 1) entries, 2^-17 * 16 = 1.2e-4,
-        # weighted by P (sums to 1), by |K|, |Q| <= 5 and by the scale 1/16: 4e-5.
+        # Every operand carries 24 bits, products accumulate in fp32.  3e-5 of the largest gradient, and where
+        # dP - delta cancels (a single visible key: dS is exactly 0) 4e-5, would do for operands of 16 bits
+        # (test_error_is_that_of_fp32_products is the tight one).
         scale = y.abs().max().item()
         assert (x - y).abs().max().item() <= 3e-5 * scale + 4e-5, (name, (x - y).abs().max().item(), scale)
+    assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [64, 200, 1000])
+@pytest.mark.parametrize("std", [0.5, 1.0])
+def test_error_is_that_of_fp32_products(tokens, std):
+    """Unrounded core and gradients against float64, 2-norm.  The bounds are what fp32 leaves: a score is 256
+    products, rounded to some 2^-23 of |s| <= 5, which is the relative error of its probability; the sums
+    behind it add a few 2^-24 apiece.  10 * 2^-24 for the core, 14 for the gradients, which go through two
+    more products; operands of 16 bits leave 1.5e-6 and 4e-6."""
+    q, k, v, d_out = make((1, tokens, 24, 4), 11)
+    q, k, v = ((x.float() * std).bfloat16() for x in (q, k, v))
+    relative = lambda x, y: ((x.double() - y).norm() / y.norm()).item()
+    qd, kd, vd = (x.double().requires_grad_() for x in (q, k, v))
+    core = reference(qd, kd, vd)[0]
+    core.backward(d_out.double())
+    got = gqa_prefill(q, k, v, round_to_bfloat16=False, want_core=True, want_stats=True)
+    assert relative(got["core"], core.detach()) < 10 * 2 ** -24
+    stats = dict(got, core=core.detach().float())   # deltas as the caller would have them without an error
+    for name, x, y in zip(("dq", "dk", "dv"), backward(q, k, v, d_out, stats, True), (qd.grad, kd.grad, vd.grad)):
+        assert relative(x, y) < 14 * 2 ** -24, name
     assert _capi.kernel_status() == 0
