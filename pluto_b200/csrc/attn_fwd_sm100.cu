@@ -308,7 +308,7 @@ attn_fwd_sm100(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (gate) {
               const float g0 = __bfloat162float(gate[c * 32 + i]);
               const float g1 = __bfloat162float(gate[c * 32 + i + 1]);
-              float s0 = sigmoid_fast(g0), s1 = sigmoid_fast(g1);
+              float s0 = sigmoid(g0), s1 = sigmoid(g1);
               if (p.round_gate) {
                 s0 = bf16_round(s0);
                 s1 = bf16_round(s1);
@@ -749,7 +749,7 @@ attn_fwd_sm100_pair(const __grid_constant__ CUtensorMap map_q,
             if (gate && live) {
               const float g0 = __bfloat162float(gate[c * 32 + i]);
               const float g1 = __bfloat162float(gate[c * 32 + i + 1]);
-              float s0 = sigmoid_fast(g0), s1 = sigmoid_fast(g1);
+              float s0 = sigmoid(g0), s1 = sigmoid(g1);
               if (p.round_gate) {
                 s0 = bf16_round(s0);
                 s1 = bf16_round(s1);
@@ -871,7 +871,7 @@ __global__ void __launch_bounds__(256) attn_fwd_merge(FwdParams p, int batch, in
     float a = acc[i] * inv;
     if (core) core[i] = a;
     if (gate) {
-      float g = sigmoid_fast(__bfloat162float(gate[i]));
+      float g = sigmoid(__bfloat162float(gate[i]));
       if (p.round_gate) {
         g = bf16_round(g);
         a = bf16_round(a);

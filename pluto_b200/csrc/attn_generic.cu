@@ -321,12 +321,12 @@ attn_fwd_generic(const T* __restrict__ q, const T* __restrict__ k, const T* __re
         for (int u = 0; u < 4; ++u) {
           if (d + u >= D) continue;
           // R(R(core) * R(sigmoid(gate))), qwen_attention.cc:103-108
-          float sigmoid = 1.0f / (1.0f + expf(-load_as_float(g + d + u)));
+          float factor = sigmoid(load_as_float(g + d + u));
           if (round_gate) {
-            sigmoid = bf16_round(sigmoid);
+            factor = bf16_round(factor);
             value[u] = bf16_round(value[u]);
           }
-          value[u] *= sigmoid;
+          value[u] *= factor;
         }
       }
       store_columns(out + o_off, d, D, out_fours, value);

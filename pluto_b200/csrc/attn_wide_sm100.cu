@@ -407,12 +407,12 @@ attn_fwd_wide(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const float x = (i & 1) ? bf16_hi(w[i / 2]) : bf16_lo(w[i / 2]);
-            float sigmoid = sigmoid_fast(x);
+            float factor = sigmoid(x);
             if (p.round_gate) {
-              sigmoid = bf16_round(sigmoid);
+              factor = bf16_round(factor);
               v[i] = bf16_round(v[i]);
             }
-            v[i] *= sigmoid;
+            v[i] *= factor;
           }
         }
         *reinterpret_cast<uint4*>(p.out + at) =

@@ -411,14 +411,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// 1 / (1 + e^-x) with the reciprocal unit (rcp.approx, within one ulp of the quotient).  The IEEE
-// division costs about ten instructions, which set the pace of the kernels that apply a gate or a
-// SiLU to every element of a stream.
-__device__ __forceinline__ float sigmoid_fast(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-x)));
-  return r;
-}
+// Gates and SiLUs, the same two functions in the sequence kernels and the single-token ones, so that a
+// token gets the same bits from both.  One IEEE division each: the reciprocal unit would be 10 to 15 % of
+// the streaming kernels' time cheaper, but is an ulp off, rounds x * sigmoid(x) twice and flushes the tail
+// below -87 to zero.
+__device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 // Two-lane fp32 arithmetic (one instruction per pair of values).
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
   uint64_t r;

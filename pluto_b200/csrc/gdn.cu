@@ -168,7 +168,7 @@ __global__ void gdn_gates_kernel(const void* a_in, const void* b_in, const float
   const float alpha = load_any(a_in, i, in_is_bf16) + dt_bias[h];
   const float softplus = fmaxf(alpha, 0.0f) + logf(1.0f + expf(-fabsf(alpha)));
   g[i] = expf(-expf(a_log[h]) * softplus);
-  beta[i] = rnd(1.0f / (1.0f + expf(-load_any(b_in, i, in_is_bf16))), round);
+  beta[i] = rnd(sigmoid(load_any(b_in, i, in_is_bf16)), round);
 }
 
 // Causal depthwise convolution + SiLU over a sequence with an explicit history:
@@ -198,7 +198,7 @@ __global__ void gdn_conv_kernel(const void* input, const float* weight, int in_i
     const float current = rnd(load_any(input, idx, in_is_bf16), round);
     window[width - 1] = current;
     sum = rnd(sum + current * w[width - 1], round);
-    store_any(output, idx, out_is_bf16, rnd(sum * sigmoid_fast(sum), round));
+    store_any(output, idx, out_is_bf16, rnd(silu(sum), round));
   }
   for (int tap = 0; tap < width; ++tap)
     state[(static_cast<size_t>(b) * channels + c) * width + tap] = window[tap];
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(128, 8) gdn_conv_segment_kernel(const void* __
 #pragma unroll
       for (int tap = 0; tap + 1 < W; ++tap) sum += x[tap][i] * w[i][tap];
       sum = rnd(sum + x[W - 1][i] * w[i][W - 1], round);
-      y[i] = OUT_BF16 ? sum * sigmoid_fast(sum) : rnd(sum * sigmoid_fast(sum), round);
+      y[i] = OUT_BF16 ? silu(sum) : rnd(silu(sum), round);
     }
     store_four<OUT_BF16>(output, at, y);
   }
@@ -301,7 +301,7 @@ __device__ __forceinline__ float norm_gate(float x, float inverse, float weight,
                                            int final_round) {
   const float normalized = rnd(x * inverse, round);
   const float affine = rnd(normalized * weight, round);
-  return rnd(affine * (gate * sigmoid_fast(gate)), round && final_round);
+  return rnd(affine * silu(gate), round && final_round);
 }
 
 // One warp per row, eight rows per CTA, a lane owning four consecutive channels of every 128.  HBM

@@ -95,12 +95,12 @@ __global__ void __launch_bounds__(256) gdn_out_bwd_kernel(const void* __restrict
     for (int i = 0; i < kOutChannels; ++i) {
       const float normalized = rnd(x[i] * inverse, round);
       const float affine = rnd(normalized * w[i], round);
-      const float sigmoid = sigmoid_fast(gate[i]);
-      const float dnorm = g[i] * gate[i] * sigmoid;
+      const float s = sigmoid(gate[i]);
+      const float dnorm = g[i] * gate[i] * s;
       dn[i] = dnorm * w[i];
       dot += dn[i] * x[i];
       sum[i] = fmaf(dnorm, normalized, sum[i]);
-      gate[i] = g[i] * affine * sigmoid * (1.0f + gate[i] * (1.0f - sigmoid));   // dz
+      gate[i] = g[i] * affine * s * (1.0f + gate[i] * (1.0f - s));   // dz
     }
     const float scale = inverse * inverse * inverse / static_cast<float>(dim) * warp_sum(dot);
 #pragma unroll
@@ -427,8 +427,8 @@ __device__ __forceinline__ float conv_dpre(const void* input, int in_is_bf16, co
              weight[static_cast<size_t>(c) * width + tap];
   }
   sum = rnd(sum, round);
-  const float sigmoid = sigmoid_fast(sum);
-  return dpost[(seq_base + t) * channels + c] * sigmoid * (1.0f + sum * (1.0f - sigmoid));
+  const float s = sigmoid(sum);
+  return dpost[(seq_base + t) * channels + c] * s * (1.0f + sum * (1.0f - s));
 }
 
 // Windows wider than four taps.
@@ -552,8 +552,8 @@ gdn_conv_bwd_kernel(const void* __restrict__ input, const float* __restrict__ we
 #pragma unroll
           for (int tap = 0; tap < W; ++tap) sum += x[tap][i] * w[tap][i];
           sum = rnd(sum, round);
-          const float sigmoid = sigmoid_fast(sum);
-          const float d = (s < tokens ? up[u][i] : 0.0f) * sigmoid * (1.0f + sum * (1.0f - sigmoid));
+          const float gate = sigmoid(sum);
+          const float d = (s < tokens ? up[u][i] : 0.0f) * gate * (1.0f + sum * (1.0f - gate));
           dpre[W - 1][i] = d;
           const float own = s < t1 ? d : 0.0f;
           out[i] = 0.0f;

@@ -111,9 +111,9 @@ __device__ __forceinline__ void store_output(const DecodeArgs& a, int b, int hea
     const size_t g = static_cast<size_t>(b) * a.gate_token + static_cast<size_t>(head) * a.gate_head + d;
     const float x = a.gate_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[g])
                                    : static_cast<const float*>(a.gate)[g];
-    float sigmoid = 1.0f / (1.0f + expf(-x));
-    if (a.round) sigmoid = bf16_round(sigmoid);
-    value *= sigmoid;
+    float factor = sigmoid(x);
+    if (a.round) factor = bf16_round(factor);
+    value *= factor;
     if (a.round) value = bf16_round(value);
   }
   const size_t idx = (static_cast<size_t>(b) * a.q_heads + head) * a.head_dim + d;

@@ -50,9 +50,9 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwdArgs a, long long 
     }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const float sigmoid = sigmoid_fast(g[i]);
-      dc[i] = grad[i] * rnd(sigmoid, a.round);
-      dg[i] = grad[i] * rnd(core[i], a.round) * sigmoid * (1.0f - sigmoid);
+      const float s = sigmoid(g[i]);
+      dc[i] = grad[i] * rnd(s, a.round);
+      dg[i] = grad[i] * rnd(core[i], a.round) * s * (1.0f - s);
       part = fmaf(dc[i], core[i], part);
     }
     if (kPer == 4) {

@@ -102,8 +102,8 @@ __device__ __forceinline__ float chunk_weights(const float2* ml, int chunks, flo
 __device__ __forceinline__ void store_gated(const CachedStepArgs& a, int head, int d, float value) {
   value = rnd(value, a.round);
   const float gate = load_any(a.q_gate, (static_cast<size_t>(head) * 2 + 1) * a.head_dim + d, a.in_is_bf16);
-  const float sigmoid = rnd(1.0f / (1.0f + expf(-gate)), a.round);
-  store_any(a.out, static_cast<size_t>(head) * a.head_dim + d, a.out_is_bf16, rnd(value * sigmoid, a.round));
+  store_any(a.out, static_cast<size_t>(head) * a.head_dim + d, a.out_is_bf16,
+            rnd(value * rnd(sigmoid(gate), a.round), a.round));
 }
 
 // kCount (2, 4 or 8) consecutive cache elements of a row.
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
         sum = rnd(sum + window[tap] * w[tap], a.round);
       }
     }
-    qkv[part][i] = rnd(sum / (1.0f + expf(-sum)), a.round);
+    qkv[part][i] = rnd(silu(sum), a.round);
     if (part == 0) {   // the threads that finish the row
       z = load_any(a.z, static_cast<size_t>(h) * kDim + i, a.z_is_bf16);
     }
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
     const float alpha = load_any(a.a_in, h, a.ab_is_bf16) + a.dt_bias[h];
     const float softplus = fmaxf(alpha, 0.0f) + logf(1.0f + expf(-fabsf(alpha)));
     gates[0] = expf(-expf(a.a_log[h]) * softplus);
-    gates[1] = rnd(1.0f / (1.0f + expf(-load_any(a.b_in, h, a.ab_is_bf16))), a.round);
+    gates[1] = rnd(sigmoid(load_any(a.b_in, h, a.ab_is_bf16)), a.round);
   }
   if (group > 1) cluster_arrive();   // this CTA has read the shared windows
   __syncthreads();
@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kTokenThreads) gdn_token_kernel(GdnTokenArgs a
   if (tid < kDim) {
     const float inverse = rsqrtf((red[0] + red[1] + red[2] + red[3]) / static_cast<float>(kDim) + a.epsilon);
     const float affine = rnd(rnd(core * inverse, a.round) * norm, a.round);
-    store_any(a.out, static_cast<size_t>(h) * kDim + i, a.out_is_bf16, rnd(affine * (z / (1.0f + expf(-z))), a.round));
+    store_any(a.out, static_cast<size_t>(h) * kDim + i, a.out_is_bf16, rnd(affine * silu(z), a.round));
   }
   if (group > 1) cluster_wait();     // everyone has read the shared windows
   if (tid < 3 * kDim && (part == 2 || h % group == 0)) {

@@ -138,3 +138,58 @@ def test_cached_step_is_the_separate_launches_bit_for_bit(heads, dim, rotary, ca
         assert torch.equal(caches[0].keys(), caches[1].keys()) and torch.equal(caches[0].values(), caches[1].values())
         assert torch.equal(out, want), position
     assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("rounded", [True, False])
+def test_delta_step_gates_as_the_sequence_kernels_do(rounded):
+    """Convolution SiLU and output gate of the one launch and of the four, bit for bit.  One live channel in q
+    and in k leaves every sum behind them a single term, so no order of summation can hide a difference."""
+    key_heads, value_heads, taps = 2, 6, 4
+    p = DeltaNetParameters(key_heads=key_heads, value_heads=value_heads, conv_kernel_dim=taps, round_to_bfloat16=rounded)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    kq, width = key_heads * 128, value_heads * 128
+    channels = 2 * kq + width
+    conv, a_log, dt_bias, norm = rnd(channels, taps), rnd(value_heads), rnd(value_heads), rnd(128)
+    conv[:2 * kq].view(2 * key_heads, 128, taps)[:, 1:] = 0
+    state = DeltaNetState.Create(p)
+    window, S = torch.zeros(channels, taps, device="cuda"), torch.zeros(1, value_heads, 128, 128, device="cuda")
+    L, f32 = _capi.fast(), dict(device="cuda", dtype=torch.float32)
+    for _ in range(4):
+        qkv, z, a, b = rnd(channels) * 3, rnd(value_heads, 128) * 4, rnd(value_heads), rnd(value_heads)
+        out, want = torch.empty(value_heads, 128, **f32), torch.empty(value_heads, 128, **f32)
+        state.Step(qkv, z, a, b, conv, a_log, dt_bias, norm, out)
+        post, g, beta, core = (torch.empty(n, **f32) for n in (channels, value_heads, value_heads, width))
+        flag = int(rounded)
+        _capi.check(L.pluto_gdn_conv_silu(stream(), qkv.data_ptr(), conv.data_ptr(), 0, 1, 1, channels, taps, flag,
+                                          window.data_ptr(), post.data_ptr(), 0))
+        _capi.check(L.pluto_gdn_gates(stream(), a.data_ptr(), b.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), 0, 1,
+                                      value_heads, flag, g.data_ptr(), beta.data_ptr()))
+        _capi.check(L.pluto_gdn_step(stream(), post.data_ptr(), post[kq:].data_ptr(), post[2 * kq:].data_ptr(), 0,
+                                     g.data_ptr(), beta.data_ptr(), S.data_ptr(), core.data_ptr(), 0, 1, key_heads,
+                                     value_heads, 128, 128, 1, 1.0, flag))
+        _capi.check(L.pluto_gdn_out_norm_gate(stream(), core.data_ptr(), 0, z.data_ptr(), 0, norm.data_ptr(), value_heads,
+                                              128, p.rms_norm_epsilon, flag, 1, want.data_ptr(), 0))
+        assert torch.equal(state.recurrent_state_, S)
+        if rounded:
+            assert torch.equal(out, want)
+        else:   # the mean square of 128 terms, summed in another order: 2^-23 of its root, and three roundings
+            assert ((out - want).abs() <= 2 ** -21 * want.abs()).all()
+
+
+def test_silu_is_one_quotient_over_its_whole_range():
+    """x / (1 + e^-x) with an identity convolution, several tokens and one.  expf is good to 2 ulp, the sum and
+    the quotient round once each: 3.5 * 2^-23.  The tail below -87 counts (1 + e^-x is finite down to -88.7)."""
+    x = torch.cat([torch.linspace(-88.5, 20, 4096), torch.linspace(-3, 3, 4096)]).cuda()
+    channels, tokens = 4, 2048
+    weight = torch.zeros(channels, 2, device="cuda")
+    weight[:, 1] = 1
+    for t in (tokens, 1):
+        y = torch.empty(x.numel(), device="cuda")
+        c = x.numel() // t
+        window = torch.zeros(1, c, 2, device="cuda")
+        w = weight[:1].expand(c, 2).contiguous()
+        _capi.check(_capi.fast().pluto_gdn_conv_silu(stream(), x.data_ptr(), w.data_ptr(), 0, 1, t, c, 2, 0,
+                                                     window.data_ptr(), y.data_ptr(), 0))
+        want = x.double() / (1 + torch.exp(-x.double()))
+        assert ((y.double() - want).abs() <= 3.5 * 2 ** -23 * want.abs()).all()
