@@ -57,3 +57,19 @@ def test_decode_matches_float64(batch, hq, hkv, dim, longest, page):
     assert ((gated.double() - expected).abs() <= 2 ** -6 * expected.abs() + 4e-5).all()
     assert torch.equal(gated, gqa_decode(q, pool_k, pool_v, lens, longest, block_table=table, gate=gate))
     assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("rounded", [True, False])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_width_256_keeps_fp32_queries(rounded, out_dtype):
+    """fp32 queries that bf16 cannot hold are attended with as given: the log of the softmax sum is an fp32
+    result of the scores, and a query rounded to bf16 moves it by 1e-3 and more."""
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    k, v, q = rnd(2, 200, 2, 256).bfloat16(), rnd(2, 200, 2, 256).bfloat16(), rnd(2, 6, 256)
+    lens = torch.tensor([200, 77], dtype=torch.int32, device="cuda")
+    _, lse = gqa_decode(q, k, v, lens, 200, round_to_bfloat16=rounded, out=torch.empty(2, 6, 256, device="cuda", dtype=out_dtype),
+                        want_lse=True)
+    for b, n in enumerate(lens.tolist()):
+        s = torch.einsum("hd,thd->ht", q[b].double(), k[b, :n].double().repeat_interleave(3, 1)) / 16
+        assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() < 5e-6   # fp32 sums of 256 products
