@@ -740,20 +740,35 @@ cudaError_t launch_tc(cudaStream_t stream, const CUtensorMap& map_k, const CUten
                        decode_smem<D>(), stream, parts, map_k, map_v, a);
 }
 
-// Parts per (sequence, KV head) of the one-launch form, 0 for chunks + merge kernel.
-// One launch while the caches it may read hold at most 256 MB (about 40 us of HBM): as many parts as keep
-// the grid near the 296 CTAs that are resident at once (up to 400: the ragged lengths leave gaps) and
-// a part above 32 tokens; 16 parts are beyond the portable cluster size and opted into.  Measured, best
-// one-launch form against chunks + merge: 8 units (sequence x KV head) of up to 30000 tokens 33 against
-// 44 us, 16 of 3000 (width 256, P in two parts; 22 with three) 18 / 20, 128 of 2000 22 / 27, 480 of 500 27 / 34.  Above, the merge is a
-// few per cent and whole-chip balance counts: 240 units of 4000 tokens (width 256) 143 against 113 us,
-// 64 of 20000 171 / 144, 720 of 8000 (width 64) 175 / 138.
+// Parts per (sequence, KV head) of the one-launch form, 0 for chunks + merge kernel.  A cluster lives in one
+// GPC, so only so many are resident at once, two CTAs per SM: 14 of 16 parts, 20 of 12, 33 of 8, 66 of 4, 148
+// of 2; one more doubles the time (600 tokens, width 128, us: 14 units in 16 parts 6.3, 15 11.1 in 16 and 6.1
+// in 12; 20 in 12 6.3, 22 10.5 in 12 and 6.7 in 8; 33 in 8 7.6, 34 11.7 in 8 and 7.1 in 4; 66 in 4 8.9, 72 14.0
+// in 4 and 9.7 in 2; 148 in 2 13.2, 160 21.0 in 2 and 16.6 in 1).  A part keeps at least 32 tokens.  More than 8
+// parts are beyond the portable cluster size and opted into.
+// Chunks and their merge take over
+// - above 256 MB of cache (about 40 us of HBM), where the merge is a few per cent and whole-chip balance
+//   counts: 240 units of 4000 tokens (width 256) 143 against 113 us, 64 of 20000 171 / 144, 720 of 8000
+//   (width 64) 175 / 138;
+// - where the parts are few and long, so that a few CTAs stream what the chip could.  One launch against
+//   chunks + merge, us:
+//     units       width 64            width 128                    width 256
+//       1    16384 10.9 / 10.8   8192  9.3 / 10.4           4000 14.4 / 18.3, 8192 23.1 / 21.4
+//            32768 19.2 / 15.6  32768 24.8 / 19.3          32768 75.4 / 38.4
+//       2    32768 19.5 / 18.2  16384 15.0 / 14.4, 32768 25.2 / 22.6  8192 23.1 / 20.4, 32768 75.9 / 39.3
+//       4    32768 20.0 / 22.1  32768 26.0 / 29.7           4000 14.7 / 18.6, 16384 41.2 / 30.6
+//       8    32768 23.1 / 32.0  32768 31.9 / 46.0           4000 17.5 / 20.9, 16384 49.7 / 48.2, 32768 92.9 / 95.1
+//      16    32768 41.2 / 50.0  16384 31.4 / 40.4           3000 17.8 / 22.7
+//      32    32768 44.8 / 63.2  16384 43.0 / 68.0           8192 52.0 / 75.5
+//   A CTA of width 256 (32-token tiles, P in three parts) streams 29 GB/s, the others 45 to 50, so there
+//   the line lies at 64 CTAs and 400 tokens a part, else at 32 CTAs and 900 tokens.
 int cluster_parts(const DecodeArgs& a) {
   const long long units = static_cast<long long>(a.batch) * a.kv_heads;
   if (units * a.max_length * a.head_dim * 4 > 256LL << 20) return 0;
-  int z = 1;
-  while (z < kMaxClusterParts && units * z * 2 <= 400 && a.max_length >= z * 2 * 32) z *= 2;
-  return z;
+  int z = units <= 12 ? 16 : units <= 20 ? 12 : units <= 32 ? 8 : units <= 64 ? 4 : units <= 148 ? 2 : 1;
+  while (z > 1 && a.max_length < z * 32) z = z == 12 ? 8 : z / 2;
+  const bool wide = a.head_dim == 256;
+  return units * z <= (wide ? 64 : 32) && a.max_length > z * (wide ? 400 : 900) ? 0 : z;
 }
 
 }  // namespace

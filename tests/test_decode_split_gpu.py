@@ -73,3 +73,13 @@ def test_width_256_keeps_fp32_queries(rounded, out_dtype):
     for b, n in enumerate(lens.tolist()):
         s = torch.einsum("hd,thd->ht", q[b].double(), k[b, :n].double().repeat_interleave(3, 1)) / 16
         assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() < 5e-6   # fp32 sums of 256 products
+
+
+# One, two and a dozen units (sequence x KV head), either side of the lines between the two forms: long
+# parts go to chunks, and 12, 20, 32, 64 and 148 units are the most that are cut into 16, 12, 8, 4 and 2 parts.
+@pytest.mark.parametrize("batch,hq,hkv,dim,longest", [
+    (1, 5, 1, 128, 14400), (1, 5, 1, 128, 14500), (2, 1, 1, 64, 33000), (1, 6, 1, 256, 6400), (1, 6, 1, 256, 6401),
+    (2, 6, 1, 256, 20000), (12, 1, 1, 64, 700), (13, 1, 1, 64, 380), (20, 2, 1, 128, 500), (21, 2, 1, 128, 500), (32, 2, 1, 128, 300), (33, 2, 1, 128, 300),
+    (64, 1, 1, 64, 200), (65, 1, 1, 64, 200), (149, 1, 1, 64, 100)])
+def test_few_units_and_the_lines_between_the_forms(batch, hq, hkv, dim, longest):
+    test_decode_matches_float64(batch, hq, hkv, dim, longest, 0)
