@@ -487,8 +487,14 @@ def ValidateCachedAttention(p: FullAttentionParameters, cache: KeyValueCache) ->
             or p.query_heads > imax // (2 * p.head_dim)
             or p.query_heads > imax - p.key_value_heads):
         raise _invalid("invalid full-attention dimensions or parameters")
-    if (cache.capacity() != p.capacity or cache.key_value_heads() != p.key_value_heads
-            or cache.head_dim() != p.head_dim):
+    _check_cache_shape(p, cache)
+
+
+def _check_cache_shape(p: FullAttentionParameters, cache: KeyValueCache) -> None:
+    """The part of the validation that the C ABI cannot repeat: it sees a row stride and a capacity, not
+    the cache's heads.  A layer's cache or parameters may be replaced, so every token asks."""
+    if (cache.capacity_ != p.capacity or cache.key_value_heads_ != p.key_value_heads
+            or cache.head_dim_ != p.head_dim):
         raise _invalid("attention cache shape or capacity does not match parameters")
 
 
@@ -832,6 +838,7 @@ class QwenAttentionLayer(Layer):
         width = p.query_heads * p.head_dim
         kv = p.key_value_heads * p.head_dim
         _validate_bf16_inputs(inputs, (2 * width, kv, kv), "QwenAttentionLayer")
+        _check_cache_shape(p, cache)
         if cache.position_ >= cache.capacity_:
             raise _resource_exhausted("full-attention cache capacity reached")
         inputs = [x if x.is_contiguous() else x.contiguous() for x in inputs]

@@ -5,7 +5,8 @@ import pytest
 import torch
 
 from pluto_b200 import _capi
-from pluto_b200.layers import CachedAttentionStep, FullAttentionParameters, KeyValueCache, gqa_decode, gqa_prefill
+from pluto_b200.layers import (CachedAttentionStep, FullAttentionParameters, KeyValueCache, QwenAttentionLayer, gqa_decode,
+                               gqa_prefill)
 
 pytestmark = pytest.mark.gpu
 D = 256
@@ -77,3 +78,20 @@ def test_cache_buffers_may_be_replaced():
     cache.keys_, cache.values_ = old.clone(), cache.values_.clone()
     step(2)
     assert old[1].abs().sum().item() == 0 and cache.keys_[1].abs().sum().item() > 0
+
+
+@pytest.mark.parametrize("change", ["cache heads", "cache capacity", "parameters"])
+def test_a_layer_whose_cache_no_longer_fits_is_refused(change):
+    make = lambda **k: FullAttentionParameters(**{**dict(query_heads=2, key_value_heads=1, head_dim=64, rotary_dim=32, capacity=8), **k})
+    norm = torch.zeros(64, device="cuda")
+    layer = QwenAttentionLayer.Create(make(), norm, norm, 1, KeyValueCache.Create(8, 1, 64))
+    token = [rand(1, 1, 256).bfloat16(), rand(2, 1, 64).bfloat16(), rand(3, 1, 64).bfloat16()]
+    layer.fwd(token)
+    if change == "cache heads":
+        layer.cache_ = KeyValueCache.Create(8, 2, 64)
+    elif change == "cache capacity":
+        layer.cache_ = KeyValueCache.Create(16, 1, 64)
+    else:
+        layer.parameters_ = make(capacity=4)
+    with pytest.raises(_capi.PlutoStatusError, match="does not match parameters"):
+        layer.fwd(token)
