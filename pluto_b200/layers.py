@@ -498,16 +498,20 @@ def _check_cache_shape(p: FullAttentionParameters, cache: KeyValueCache) -> None
         raise _invalid("attention cache shape or capacity does not match parameters")
 
 
-_decode_workspaces = {}
+_decode_workspaces = {}   # (device index, stream) -> (tensor, its address, its bytes)
+
+
+def _scratch(index: int, stream: int, nbytes: int):
+    """(tensor, address, bytes) of the stream's scratch, at least nbytes; grown when a call needs more."""
+    entry = _decode_workspaces.get((index, stream))
+    if entry is None or entry[2] < nbytes:
+        ws = torch.empty((max(nbytes, 1 << 20),), dtype=torch.uint8, device=torch.device("cuda", index))
+        entry = _decode_workspaces[(index, stream)] = ws, ws.data_ptr(), ws.numel()
+    return entry
 
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
-    key = (device.index, _stream())
-    ws = _decode_workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty((max(nbytes, 1 << 20),), dtype=torch.uint8, device=device)
-        _decode_workspaces[key] = ws
-    return ws
+    return _scratch(device.index, _stream(), nbytes)[0]
 
 
 def CachedAttentionStep(p: FullAttentionParameters, cache: KeyValueCache, q_gate: torch.Tensor,
@@ -531,21 +535,17 @@ def CachedAttentionStep(p: FullAttentionParameters, cache: KeyValueCache, q_gate
     cache.Advance()
 
 
-_ONE_LAUNCH_TOKENS = 1024   # contexts that pluto_cached_attention_step attends to without scratch
-
-
 def _cached_step(p, cache, q_gate, k, v, q_norm, k_norm, output) -> None:
-    """The launches of CachedAttentionStep at the cache's position, which stays where it is."""
+    """The launches of CachedAttentionStep at the cache's position, which stays where it is.  Which form a
+    step takes is the library's to decide, so it always gets the scratch that the longer one needs."""
     L = _capi.fast()
-    position, ws, ws_bytes = cache.position_, None, 0
-    if position >= _ONE_LAUNCH_TOKENS or p.head_dim not in (64, 128, 256):
-        ws = _workspace(output.device, L.pluto_cached_attention_step_workspace_bytes(
-            p.query_heads, p.key_value_heads, p.head_dim, position + 1))
-        ws, ws_bytes = ws.data_ptr(), ws.numel()
+    heads, kv_heads, width, position, stream = p.query_heads, p.key_value_heads, p.head_dim, cache.position_, _stream()
+    _, scratch, scratch_bytes = _scratch(output.get_device(), stream, L.pluto_cached_attention_step_workspace_bytes(
+        heads, kv_heads, width, position + 1))
     check(L.pluto_cached_attention_step(
-        _stream(), q_gate.data_ptr(), k.data_ptr(), v.data_ptr(), _dt(q_gate), q_norm.data_ptr(), k_norm.data_ptr(),
-        cache.packed_layout(), position, output.data_ptr(), _dt(output), ws, ws_bytes, p.query_heads,
-        p.key_value_heads, p.head_dim, p.rotary_dim, p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16)))
+        stream, q_gate.data_ptr(), k.data_ptr(), v.data_ptr(), _dt(q_gate), q_norm.data_ptr(), k_norm.data_ptr(),
+        cache.packed_layout(), position, output.data_ptr(), _dt(output), scratch, scratch_bytes, heads,
+        kv_heads, width, p.rotary_dim, p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16)))
 
 
 def _cached_probabilities(p, cache, q_gate, k, v, q_norm, k_norm, probabilities) -> None:

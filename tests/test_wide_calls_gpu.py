@@ -95,3 +95,22 @@ def test_a_layer_whose_cache_no_longer_fits_is_refused(change):
         layer.parameters_ = make(capacity=4)
     with pytest.raises(_capi.PlutoStatusError, match="does not match parameters"):
         layer.fwd(token)
+
+
+@pytest.mark.parametrize("dim", [64, 128, 256])
+def test_cache_buffers_off_the_16_byte_boundary(dim):
+    """One element further on, the one-launch step does not apply, and the same call takes the separate launches."""
+    p = FullAttentionParameters(query_heads=4, key_value_heads=2, head_dim=dim, rotary_dim=32, capacity=8)
+    norm, outs = torch.zeros(dim, device="cuda"), []
+    for shift in (0, 1):
+        cache = KeyValueCache.Create(8, 2, dim)
+        cache.keys_, cache.values_ = (torch.zeros(x.numel() + 8, device="cuda", dtype=x.dtype)[shift:shift + x.numel()].view_as(x)
+                                      for x in (cache.keys_, cache.values_))
+        out = torch.empty(4, dim, device="cuda", dtype=torch.bfloat16)
+        for i in range(3):
+            CachedAttentionStep(p, cache, rand(i, 4, 2, dim).bfloat16(), rand(i + 9, 2, dim).bfloat16(),
+                                rand(i + 99, 2, dim).bfloat16(), norm, norm, out)
+        outs.append((out.float(), cache.keys_.clone()))
+    assert torch.equal(outs[0][1], outs[1][1])
+    # the core and its product with the gate can each fall on either side of a tie: one bf16 ulp apiece
+    assert ((outs[0][0] - outs[1][0]).abs() <= 2 ** -6 * outs[1][0].abs() + 1e-6).all()
