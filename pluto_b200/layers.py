@@ -74,12 +74,15 @@ def _invalid(message: str) -> PlutoStatusError:
 
 
 # The current stream of the current device as a raw handle: 0.1 us, where building the Stream object
-# that torch.cuda.current_stream() returns takes 3.
+# that torch.cuda.current_stream() returns takes 3.  (Private functions: a torch without them takes the
+# public way.)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _current_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_current_device())
 
 

@@ -74,3 +74,11 @@ def test_delta_net_create_validation(engine):
                    dict(value_head_dim=257), dict(conv_kernel_dim=33), dict(rms_norm_epsilon=-1.0)):
         bad = DeltaNetParameters(**{**DeltaNetParameters().__dict__, **change})
         assert code_of(DeltaNetState.Create, bad, "cpu")[0] == "InvalidArgument"
+
+
+@pytest.mark.parametrize("missing", ["_raw_stream", "_current_device"])
+def test_stream_handle_without_the_private_functions(engine, monkeypatch, missing):
+    from pluto_b200 import layers
+    monkeypatch.setattr(layers, missing, None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 77})())
+    assert layers._stream() == 77
