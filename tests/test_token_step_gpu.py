@@ -193,3 +193,29 @@ def test_silu_is_one_quotient_over_its_whole_range():
                                                      window.data_ptr(), y.data_ptr(), 0))
         want = x.double() / (1 + torch.exp(-x.double()))
         assert ((y.double() - want).abs() <= 3.5 * 2 ** -23 * want.abs()).all()
+
+
+@pytest.mark.parametrize("dim,rotary", [(256, 64), (64, 4), (64, 12), (128, 20)])
+@pytest.mark.parametrize("rounded", [True, False])
+def test_an_inspection_hook_leaves_the_cache_as_it_is(dim, rotary, rounded):
+    """The probabilities' query is prepared once more, which rewrites the token's cache row: with the same
+    bits, whatever rotary width the prepare kernel's accesses fit, and so the outputs behind it stay too."""
+    hq, hkv = 4, 2
+    p = FullAttentionParameters(query_heads=hq, key_value_heads=hkv, head_dim=dim, rotary_dim=rotary, capacity=16,
+                                round_to_bfloat16=rounded)
+    results = []
+    for hook in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(dim + rotary)
+        rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+        cache, wq, wk = KeyValueCache.Create(16, hkv, dim, torch.float32), rnd(dim) * 0.1, rnd(dim) * 0.1
+        outs = []
+        for t in range(12):
+            out, probabilities = torch.empty(hq, dim, device="cuda"), torch.empty(hq, t + 1, device="cuda")
+            CachedAttentionStep(p, cache, rnd(hq, 2, dim), rnd(hkv, dim), rnd(hkv, dim), wq, wk, out,
+                                probabilities if hook else None)
+            outs.append(out)
+            if hook:   # fp32 sums of at most 12 terms
+                assert (probabilities.sum(1) - 1).abs().max().item() < 12 * 2 ** -23
+        results.append((cache.keys().clone(), cache.values().clone(), torch.stack(outs)))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
