@@ -25,6 +25,10 @@ int from_cuda(cudaError_t e, const char* what) {
   return static_cast<int>(e);
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + b_bytes && y < x + a_bytes;
+}
 }  // namespace
 
 // the same two helpers for entry points defined in other files
@@ -523,9 +527,12 @@ int pluto_cached_attention_step(pluto_stream_t stream, const void* q_gate, const
   s.epsilon = rms_norm_epsilon; s.log_theta = logf(rope_theta);
   s.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
   s.round = round_to_bf16;
-  if (pluto::cached_step_supported(s))
+  // (an output over k or v would be written while another head's CTA still reads them)
+  const size_t in_bytes = s.in_is_bf16 ? 2 : 4, out_size = static_cast<size_t>(q_heads) * head_dim * (s.out_is_bf16 ? 2 : 4);
+  const size_t kv_size = static_cast<size_t>(kv_heads) * head_dim * in_bytes;
+  if (pluto::cached_step_supported(s) && !overlap(out, out_size, k, kv_size) && !overlap(out, out_size, v, kv_size))
     return from_cuda(pluto::cached_step(stream, s), "Qwen cached attention step");
-  // longer contexts and other widths: prepare, split decode, merge
+  // longer contexts, other widths and such outputs: prepare, split decode, merge
   const size_t need = pluto_cached_attention_step_workspace_bytes(q_heads, kv_heads, head_dim, position + 1);
   if (!workspace || workspace_bytes < need || !aligned16(workspace))
     return fail(PLUTO_E_INVALID, "attention decode workspace is too small or misaligned");
@@ -668,7 +675,15 @@ int pluto_gdn_token_step(pluto_stream_t stream, const void* qkv, int qkv_dtype, 
     return fail(PLUTO_E_INVALID, "invalid DeltaNet dimensions or parameters");
   if (!qkv || !z || !a || !b || !conv_weight || !a_log || !dt_bias || !norm_weight || !conv_state || !state || !out)
     return fail(PLUTO_E_INVALID, "DeltaNet requires non-null device pointers");
-  if (pluto::gdn_token_supported(key_heads, value_heads, key_dim, value_dim, conv_width) && aligned16(state)) {
+  // one launch, unless the output would be written over inputs that other heads' CTAs still read (over z,
+  // element on element, it is its own reader)
+  const auto bytes = [](int dtype) { return static_cast<size_t>(dtype == PLUTO_BF16 ? 2 : 4); };
+  const size_t width = static_cast<size_t>(value_heads) * value_dim, out_size = width * bytes(out_dtype);
+  const size_t qkv_size = (2 * static_cast<size_t>(key_heads) * key_dim + width) * bytes(qkv_dtype);
+  const bool apart = !overlap(out, out_size, qkv, qkv_size) && !overlap(out, out_size, a, value_heads * bytes(ab_dtype)) &&
+                     !overlap(out, out_size, b, value_heads * bytes(ab_dtype)) &&
+                     ((out == z && out_dtype == z_dtype) || !overlap(out, out_size, z, width * bytes(z_dtype)));
+  if (pluto::gdn_token_supported(key_heads, value_heads, key_dim, value_dim, conv_width) && aligned16(state) && apart) {
     pluto::GdnTokenArgs t{};
     t.qkv = qkv; t.z = z; t.a_in = a; t.b_in = b;
     t.qkv_is_bf16 = qkv_dtype == PLUTO_BF16; t.z_is_bf16 = z_dtype == PLUTO_BF16; t.ab_is_bf16 = ab_dtype == PLUTO_BF16;

@@ -219,3 +219,42 @@ def test_an_inspection_hook_leaves_the_cache_as_it_is(dim, rotary, rounded):
         results.append((cache.keys().clone(), cache.values().clone(), torch.stack(outs)))
     for x, y in zip(*results):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("over", ["k", "v"])
+def test_attention_output_over_an_input(over):
+    """An output that shares memory with k or v: every head still attends with what the caller passed."""
+    hq, hkv, dim = 4, 4, 128
+    p = FullAttentionParameters(query_heads=hq, key_value_heads=hkv, head_dim=dim, rotary_dim=dim, capacity=8)
+    results = []
+    for shared in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(3)
+        rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+        cache, norm = KeyValueCache.Create(8, hkv, dim, torch.float32), torch.zeros(dim, device="cuda")
+        qg, k, v = rnd(hq, 2, dim), rnd(hkv, dim), rnd(hkv, dim)
+        out = {"k": k, "v": v}[over] if shared else torch.empty(hq, dim, device="cuda")
+        CachedAttentionStep(p, cache, qg, k, v, norm, norm, out)
+        results.append((out, cache.keys(), cache.values()))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("over", ["qkv", "z"])
+def test_delta_output_over_an_input(over):
+    p = DeltaNetParameters(key_heads=2, value_heads=6)
+    results = []
+    for shared in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(3)
+        rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+        channels = 4 * 128 + 6 * 128
+        conv, a_log, dt_bias, norm = rnd(channels, 4), rnd(6), rnd(6), rnd(128)
+        state, qkv, z, a, b = DeltaNetState.Create(p), rnd(channels), rnd(6, 128), rnd(6), rnd(6)
+        out = torch.empty(6, 128, device="cuda")
+        if shared:
+            out = qkv[:6 * 128].view(6, 128) if over == "qkv" else z
+        state.Step(qkv, z, a, b, conv, a_log, dt_bias, norm, out)
+        results.append((out, state.recurrent_state_))
+    (x, s), (y, t) = results
+    # one launch against four: fp32 sums of 128 terms in another order, then bf16 roundings of the output
+    assert (s - t).abs().max() <= 1e-5 * s.abs().max()
+    assert ((x - y).abs() <= 2 ** -6 * x.abs() + 2e-5 * x.abs().max()).all()
