@@ -1,6 +1,7 @@
-"""Tensor-core decode in its two forms (parts of a cluster; chunks + merge kernel) and at all three
-head widths against float64, with lengths at the edges of the 64-token tiles and of the parts: one
-token, fewer tokens than parts, and part boundaries."""
+"""Decode in its two forms (parts of a cluster; chunks + merge kernel) and at all three head widths
+against float64, with lengths at the edges of the tiles (64 tokens, at width 256 32) and of the parts: one
+token, fewer tokens than parts, and part boundaries.  Unrounded fp32 results run on the tensor cores at
+widths 64 and 128 and on the plain kernel at 256, whose tensor-core form has a test of its own."""
 import math
 
 import pytest
@@ -83,3 +84,39 @@ def test_width_256_keeps_fp32_queries(rounded, out_dtype):
     (64, 1, 1, 64, 200), (65, 1, 1, 64, 200), (149, 1, 1, 64, 100)])
 def test_few_units_and_the_lines_between_the_forms(batch, hq, hkv, dim, longest):
     test_decode_matches_float64(batch, hq, hkv, dim, longest, 0)
+
+
+@pytest.mark.parametrize("batch,hq,hkv,longest", [
+    (1, 6, 1, 1), (1, 24, 4, 33), (5, 24, 4, 130), (2, 24, 4, 3000), (40, 8, 4, 300),        # one launch
+    (1, 6, 1, 9000), (3, 24, 4, 6500), (17, 24, 4, 4000)])                                   # chunks and the merge
+@pytest.mark.parametrize("page", [0, 16, 64])
+def test_width_256_on_the_tensor_cores(batch, hq, hkv, longest, page):
+    """bf16 queries, rounded result in fp32: the log of the softmax sum and the ungated output.  The core is
+    good to a few 2^-24 of values of order one, so its rounding to bf16 is the nearest value or, within 2e-6
+    of a tie, the other neighbour; P in two parts instead of three would leave 1e-5."""
+    gen = torch.Generator(device="cuda").manual_seed(longest)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    capacity = (longest + 63) // 64 * 64
+    k, v, q = rnd(batch, capacity, hkv, 256).bfloat16(), rnd(batch, capacity, hkv, 256).bfloat16(), rnd(batch, hq, 256).bfloat16()
+    lens = torch.randint(1, longest + 1, (batch,), device="cuda", generator=gen, dtype=torch.int32)
+    lens[0] = longest
+    for i, x in enumerate([x for x in (31, 32, 33, longest - 1) if 1 <= x <= longest][:batch - 1]):
+        lens[1 + i] = x
+    table, pool_k, pool_v = None, k, v
+    if page:
+        blocks = capacity // page
+        table = torch.randperm(batch * blocks, device="cuda", generator=gen).to(torch.int32).view(batch, blocks)
+        pool_k, pool_v = (torch.empty(batch * blocks, page, hkv, 256, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        pool_k[table.reshape(-1).long()] = k.view(-1, page, hkv, 256)
+        pool_v[table.reshape(-1).long()] = v.view(-1, page, hkv, 256)
+    got, lse = gqa_decode(q, pool_k, pool_v, lens, longest, block_table=table, out=torch.empty(batch, hq, 256, device="cuda"),
+                          want_lse=True)
+    for b, n in enumerate(lens.tolist()):
+        kk, vv = (x[b, :n].double().repeat_interleave(hq // hkv, 1) for x in (k, v))
+        s = torch.einsum("hd,thd->ht", q[b].double(), kk) / 16
+        want = torch.einsum("ht,thd->hd", torch.softmax(s, -1), vv)
+        assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() < 5e-6
+        half_ulp = 2.0 ** (torch.floor(torch.log2(want.abs().clamp(min=1e-30))) - 8)
+        assert ((got[b].double() - want).abs() <= half_ulp + 2e-6).all()
+        assert torch.equal(got[b], got[b].bfloat16().float())
+    assert _capi.kernel_status() == 0

@@ -97,3 +97,55 @@ def test_output_norm_and_its_backward(dim, rows, dtype):
     assert (dz.double() - grads[1]).abs().max().item() < 5e-5
     # up to 5000 products of order one summed in fp32, in runs of at most a few dozen
     assert (dnorm.double() - 1 - grads[2]).abs().max().item() < 1e-5 * rows ** 0.5 + 1e-5
+
+
+@pytest.mark.parametrize("dim", [128, 256, 66])
+@pytest.mark.parametrize("over", ["core", "z"])
+def test_output_norm_in_place(dim, over):
+    rows = 77
+    core, z, weight = rand(1, rows, dim), rand(2, rows, dim), rand(3, dim)
+    run = lambda c, g, out: _capi.check(_capi.fast().pluto_gdn_out_norm_gate(
+        stream(), c.data_ptr(), F32, g.data_ptr(), F32, weight.data_ptr(), rows, dim, 1e-6, 1, 0, out.data_ptr(), F32))
+    want = torch.empty_like(core)
+    run(core, z, want)
+    got = (core if over == "core" else z).clone()
+    run(got if over == "core" else core, got if over == "z" else z, got)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dim", [128, 256, 66])
+@pytest.mark.parametrize("which", ["dcore", "dz"])
+def test_output_norm_backward_over_its_upstream(dim, which):
+    rows = 1203
+    core, z, weight, dy = rand(1, rows, dim), rand(2, rows, dim), rand(3, dim), rand(4, rows, dim)
+    size = _capi.fast().pluto_gdn_out_norm_gate_bwd_workspace_bytes(rows, dim)
+    results = []
+    for shared in (False, True):
+        upstream, dw = dy.clone(), torch.zeros(dim, device="cuda")
+        grads = {name: torch.empty_like(dy) for name in ("dcore", "dz")}
+        if shared:
+            grads[which] = upstream
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        _capi.check(_capi.fast().pluto_gdn_out_norm_gate_bwd(
+            stream(), core.data_ptr(), F32, z.data_ptr(), F32, weight.data_ptr(), upstream.data_ptr(), grads["dcore"].data_ptr(),
+            grads["dz"].data_ptr(), dw.data_ptr(), ws.data_ptr(), size, rows, dim, 1e-6, 1))
+        results.append((grads["dcore"], grads["dz"], dw))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("heads,dim,rotary", [(24, 256, 64), (3, 128, 128), (1, 66, 12)])
+def test_norm_backward_over_its_upstream(heads, dim, rotary):
+    tokens = 45
+    x, weight, grad = rand(1, tokens, heads, dim).bfloat16(), rand(2, dim) * 0.1, rand(3, tokens, heads, dim)
+    size = _capi.fast().pluto_qk_prepare_bwd_workspace_bytes(1, tokens, heads, dim)
+    results = []
+    for shared in (False, True):
+        upstream, dw = grad.clone(), torch.zeros(dim, device="cuda")
+        dx, ws = upstream if shared else torch.empty_like(grad), torch.empty(size, dtype=torch.uint8, device="cuda")
+        _capi.check(_capi.fast().pluto_qk_prepare_bwd(
+            stream(), x.data_ptr(), heads * dim, dim, weight.data_ptr(), upstream.data_ptr(), None, dx.data_ptr(), heads * dim,
+            dim, dw.data_ptr(), ws.data_ptr(), size, 1, tokens, heads, dim, rotary, 1e-6, 1e7, 1))
+        results.append((dx, dw))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from pluto_b200 import _capi
-from pluto_b200.layers import gqa_prefill
+from pluto_b200.layers import AttentionLayer, DataType, gqa_prefill
 
 pytestmark = pytest.mark.gpu
 D = 256
@@ -114,4 +114,35 @@ def test_error_is_that_of_fp32_products(tokens, std):
     stats = dict(got, core=core.detach().float())   # deltas as the caller would have them without an error
     for name, x, y in zip(("dq", "dk", "dv"), backward(q, k, v, d_out, stats, True), (qd.grad, kd.grad, vd.grad)):
         assert relative(x, y) < 14 * 2 ** -24, name
+    assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("batch,tokens,heads", [(1, 1, 1), (2, 63, 3), (1, 129, 2), (3, 200, 5), (1, 640, 6)])
+def test_packed_layer(batch, tokens, heads):
+    """AttentionLayer of width 256 with the scratch it asks for: packed rows of 3 E, gradients of the same
+    layout, row terms from its own bf16 output.  Against float64 with that output, bounds as above, and the
+    exact kernels; single rows of a sequence have no gradient through the scores."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(batch * tokens, 3 * heads * D, device="cuda", generator=gen).bfloat16()
+    d_out = torch.randn(batch * tokens, heads * D, device="cuda", generator=gen)
+    layer = AttentionLayer.Create(tokens, heads, heads * D, DataType.BF16)
+    result = layer.fwd([x])
+    got = layer.bwd([d_out], result.state)[0]
+    layer.tensor_core_backward = False
+    exact = layer.bwd([d_out], result.state)[0]
+    q, k, v = (x.view(batch, tokens, 3, heads, D)[:, :, i].double() for i in range(3))
+    out, g = result.outputs[0].view(batch, tokens, heads, D), d_out.view(batch, tokens, heads, D).double()
+    want, _, _ = reference(q, k, v)
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()   # half a bf16 ulp of the core
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k) / math.sqrt(D)
+    p = torch.softmax(s.masked_fill(torch.triu(torch.ones(tokens, tokens, dtype=torch.bool, device="cuda"), 1), -math.inf), -1)
+    delta = (g * out.double()).sum(-1).permute(0, 2, 1)[..., None]
+    ds = p * (torch.einsum("bqhd,bkhd->bhqk", g, v) - delta) / math.sqrt(D)
+    grads = (torch.einsum("bhqk,bkhd->bqhd", ds, k), torch.einsum("bhqk,bqhd->bkhd", ds, q), torch.einsum("bhqk,bqhd->bkhd", p, g))
+    scale = max(y.norm().item() for y in grads)
+    for i, y in enumerate(grads):
+        for gradient in (got, exact):
+            z = gradient.view(batch, tokens, 3, heads, D)[:, :, i].double()
+            # (dP and delta of one row nearly cancel: what their 256 products leave counts against the largest gradient)
+            assert (z - y).norm().item() <= 14 * 2 ** -24 * max(y.norm().item(), scale if i < 2 else 0), i
     assert _capi.kernel_status() == 0
