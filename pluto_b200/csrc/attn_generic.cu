@@ -9,6 +9,8 @@
 //
 // Like the reference the backward is two single-writer passes with fixed-order reductions and no
 // floating-point atomics, so repeated runs are bitwise identical.
+#include <algorithm>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -206,7 +208,8 @@ __device__ __forceinline__ float group16_sum(float v) {
 }
 
 struct Dims {
-  int seq, heads, head_dim, tile0;   // tile0: first tile of this launch
+  int seq, heads, head_dim;
+  int batch, batch0;   // sequences of this launch, and the first of them
   float scale;
 };
 
@@ -214,8 +217,10 @@ struct Dims {
 // of tiles (with the tile fastest, 148 SMs and 4 tiles put the longest ones together).  The kernels
 // number the tiles so that the longest come first.
 struct Unit { int tile, head, batch; };
-__device__ __forceinline__ Unit block_unit(const Dims& dims) {
-  return {static_cast<int>(blockIdx.z) + dims.tile0, static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.y)};
+__device__ __forceinline__ Unit block_unit(int heads, const Dims& dims) {
+  const unsigned per_tile = static_cast<unsigned>(heads) * dims.batch, rest = blockIdx.x % per_tile;
+  return {static_cast<int>(blockIdx.x / per_tile), static_cast<int>(rest % heads),
+          static_cast<int>(rest / heads) + dims.batch0};
 }
 
 // Addressing of separate Q/K/V tensors for the forward kernel: element strides between tokens
@@ -242,7 +247,7 @@ attn_fwd_generic(const T* __restrict__ q, const T* __restrict__ k, const T* __re
   float(*Ps)[kPitch<BN>] = reinterpret_cast<float(*)[kPitch<BN>]>(Vs + BN);
 
   const int S = dims.seq, H = dims.heads, D = dims.head_dim;
-  const Unit unit = block_unit(dims);
+  const Unit unit = block_unit(H, dims);
   const int qt = (S + BM - 1) / BM - 1 - unit.tile, h = unit.head, b = unit.batch;
   const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
   const T* q_base = q + static_cast<size_t>(b) * S * views.q_token + h * views.q_head;
@@ -416,7 +421,7 @@ attn_bwd_dq_generic(const T* __restrict__ q, const T* __restrict__ k, const T* _
   float(*Ps)[kPitch<BN>] = reinterpret_cast<float(*)[kPitch<BN>]>(Vs + BN);
 
   const int S = dims.seq, H = dims.heads, D = dims.head_dim;
-  const Unit unit = block_unit(dims);
+  const Unit unit = block_unit(H, dims);
   const int qt = (S + BM - 1) / BM - 1 - unit.tile, h = unit.head, b = unit.batch;
   const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
   const T* q_base = q + static_cast<size_t>(b) * S * views.q_token + h * views.q_head;
@@ -509,7 +514,7 @@ attn_bwd_dkv_generic(const T* __restrict__ q, const T* __restrict__ k, const T* 
   float(*Ss)[kPitch<BN>] = Ps + BM;  // dS
 
   const int S = dims.seq, H = dims.heads, D = dims.head_dim;
-  const Unit unit = block_unit(dims);
+  const Unit unit = block_unit(H / views.group, dims);
   const int kt = unit.tile, kvh = unit.head, b = unit.batch;   // the first key tile sees the most queries
   const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
   const T* k_base = k + static_cast<size_t>(b) * S * views.kv_token + kvh * views.kv_head;
@@ -590,11 +595,14 @@ cudaError_t opt_in(K kernel, size_t bytes) {
                               static_cast<int>(bytes));
 }
 
-// One CTA per (tile, head, sequence), at most 65535 tiles a launch.
+// One CTA per (tile, head, sequence), as many sequences a launch as keep the block count in range.
 template <typename Launch>
 cudaError_t launch_units(int tiles, int heads, int batch, Dims dims, Launch launch) {
-  for (dims.tile0 = 0; dims.tile0 < tiles; dims.tile0 += 65535) {
-    launch(dim3(heads, batch, tiles - dims.tile0 < 65535 ? tiles - dims.tile0 : 65535), dims);
+  const long long per_sequence = static_cast<long long>(tiles) * heads;
+  const int step = static_cast<int>(std::max(1LL, std::min<long long>(batch, 0x7fffffffLL / per_sequence)));
+  for (dims.batch0 = 0; dims.batch0 < batch; dims.batch0 += step) {
+    dims.batch = std::min(step, batch - dims.batch0);
+    launch(static_cast<unsigned>(per_sequence * dims.batch), dims);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -608,7 +616,7 @@ cudaError_t launch_fwd(cudaStream_t stream, const void* q, const void* k, const 
   auto kernel = attn_fwd_generic<T, DP, BM>;
   cudaError_t e = opt_in(kernel, fwd_smem<DP, BM>());
   if (e != cudaSuccess) return e;
-  return launch_units((dims.seq + BM - 1) / BM, dims.heads, batch, dims, [&](dim3 grid, const Dims& d) {
+  return launch_units((dims.seq + BM - 1) / BM, dims.heads, batch, dims, [&](unsigned grid, const Dims& d) {
     kernel<<<grid, kThreads, fwd_smem<DP, BM>(), stream>>>(
         static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v),
         static_cast<T*>(out), maxima, normalizers, static_cast<const T*>(gate), core, round_gate, d, views);
@@ -637,14 +645,14 @@ cudaError_t launch_bwd(cudaStream_t stream, const void* q, const void* k, const 
   e = opt_in(dkv, dkv_smem<DP, BM>());
   if (e != cudaSuccess) return e;
   const int tiles = (dims.seq + BM - 1) / BM;
-  e = launch_units(tiles, dims.heads, batch, dims, [&](dim3 grid, const Dims& d) {
+  e = launch_units(tiles, dims.heads, batch, dims, [&](unsigned grid, const Dims& d) {
     dq<<<grid, kThreads, dq_smem<DP, BM>(), stream>>>(
         static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v),
         static_cast<const T*>(out), d_out, maxima, normalizers, dq_out, deltas, d, views);
   });
   if (e != cudaSuccess) return e;
   // Same-stream ordering makes every delta visible to the key/value-owned pass.
-  return launch_units(tiles, dims.heads / views.group, batch, dims, [&](dim3 grid, const Dims& d) {
+  return launch_units(tiles, dims.heads / views.group, batch, dims, [&](unsigned grid, const Dims& d) {
     dkv<<<grid, kThreads, dkv_smem<DP, BM>(), stream>>>(
         static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), d_out, maxima,
         normalizers, deltas, dk_out, dv_out, d, views);
@@ -662,7 +670,7 @@ cudaError_t attn_generic_fwd(cudaStream_t stream, const void* q, const void* k, 
                              size_t kv_token, size_t kv_head, size_t out_token, size_t out_head,
                              int group, const void* gate, size_t gate_token, size_t gate_head,
                              float* core, int round_gate, bool bf16) {
-  Dims dims{seq, heads, head_dim, 0, 1.0f / sqrtf(static_cast<float>(head_dim))};
+  Dims dims{seq, heads, head_dim, batch, 0, 1.0f / sqrtf(static_cast<float>(head_dim))};
   Views views{q_token, q_head, kv_token, kv_head, out_token, out_head, gate_token, gate_head, group};
 #define CALL_FWD(T, DP, BM) \
   launch_fwd<T, DP, BM>(stream, q, k, v, out, maxima, normalizers, gate, core, round_gate, \
@@ -681,7 +689,7 @@ cudaError_t attn_generic_fwd(cudaStream_t stream, const void* q, const void* k, 
 cudaError_t attn_generic_probs(cudaStream_t stream, const void* qkv, const float* maxima,
                                const float* normalizers, float* probs, int batch, int seq,
                                int heads, int head_dim, bool bf16) {
-  Dims dims{seq, heads, head_dim, 0, 1.0f / sqrtf(static_cast<float>(head_dim))};
+  Dims dims{seq, heads, head_dim, batch, 0, 1.0f / sqrtf(static_cast<float>(head_dim))};
 #define CALL_P(T, DP, BM) launch_probs<T, DP, BM>(stream, qkv, maxima, normalizers, probs, batch, dims)
   if (bf16) {
     if (head_dim <= 64) return CALL_P(__nv_bfloat16, 64, 64);
@@ -724,7 +732,7 @@ cudaError_t attn_generic_bwd(cudaStream_t stream, const void* qkv, const void* o
 // Backward of the attention core over separate tensors with grouped query heads (the Qwen
 // sequence layer): see GqaBwdArgs in engine.h.
 cudaError_t gqa_generic_bwd(cudaStream_t stream, const GqaBwdArgs& a) {
-  Dims dims{a.seq, a.q_heads, a.head_dim, 0, 1.0f / sqrtf(static_cast<float>(a.head_dim))};
+  Dims dims{a.seq, a.q_heads, a.head_dim, a.batch, 0, 1.0f / sqrtf(static_cast<float>(a.head_dim))};
   BwdViews views{a.q_token, a.q_head, a.kv_token, a.kv_head, a.o_token, a.o_head, a.g_token,
                  a.g_head, a.dq_token, a.dq_head, a.dkv_token, a.dkv_head, a.q_heads / a.kv_heads};
 #define CALL_B(T, DP, BM)                                                                        \
