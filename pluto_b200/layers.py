@@ -174,8 +174,8 @@ class AttentionLayer(Layer):
         self.num_heads_ = num_heads
         self.embedding_dim_ = embedding_dim
         self.output_type_ = data_type
-        # bf16 layers with head width 64/128 run backward on the tensor cores; set False to force
-        # the exact fp32 kernels (every shape has them)
+        # bf16 layers with head width 64/128 (bf16 operands) or 256 (fp32 operands in three bf16 parts) run
+        # backward on the tensor cores; set False to force the exact fp32 kernels (every shape has them)
         self.tensor_core_backward = True
 
     @staticmethod
@@ -502,6 +502,7 @@ def _check_cache_shape(p: FullAttentionParameters, cache: KeyValueCache) -> None
 
 
 _decode_workspaces = {}   # (device index, stream) -> (tensor, its address, its bytes)
+_NO_SCRATCH = (None, None, 0)
 
 
 def _scratch(index: int, stream: int, nbytes: int):
@@ -539,16 +540,22 @@ def CachedAttentionStep(p: FullAttentionParameters, cache: KeyValueCache, q_gate
 
 
 def _cached_step(p, cache, q_gate, k, v, q_norm, k_norm, output) -> None:
-    """The launches of CachedAttentionStep at the cache's position, which stays where it is.  Which form a
-    step takes is the library's to decide, so it always gets the scratch that the longer one needs."""
+    """The launches of CachedAttentionStep at the cache's position, which stays where it is.  Whether a step
+    needs scratch is the library's to decide: it gets what the stream has, and where it refuses for the want
+    of more (before any launch), that much is brought."""
     L = _capi.fast()
-    heads, kv_heads, width, position, stream = p.query_heads, p.key_value_heads, p.head_dim, cache.position_, _stream()
-    _, scratch, scratch_bytes = _scratch(output.get_device(), stream, L.pluto_cached_attention_step_workspace_bytes(
-        heads, kv_heads, width, position + 1))
-    check(L.pluto_cached_attention_step(
+    position, index, stream = cache.position_, output.get_device(), _stream()
+    _, scratch, size = _decode_workspaces.get((index, stream), _NO_SCRATCH)
+    code = L.pluto_cached_attention_step(
         stream, q_gate.data_ptr(), k.data_ptr(), v.data_ptr(), _dt(q_gate), q_norm.data_ptr(), k_norm.data_ptr(),
-        cache.packed_layout(), position, output.data_ptr(), _dt(output), scratch, scratch_bytes, heads,
-        kv_heads, width, p.rotary_dim, p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16)))
+        cache.packed_layout(), position, output.data_ptr(), _dt(output), scratch, size, p.query_heads,
+        p.key_value_heads, p.head_dim, p.rotary_dim, p.rms_norm_epsilon, p.rope_theta, int(p.round_to_bfloat16))
+    if code:
+        need = L.pluto_cached_attention_step_workspace_bytes(p.query_heads, p.key_value_heads, p.head_dim, position + 1)
+        if size >= need:
+            check(code)
+        _scratch(index, stream, need)
+        _cached_step(p, cache, q_gate, k, v, q_norm, k_norm, output)
 
 
 def _cached_probabilities(p, cache, q_gate, k, v, q_norm, k_norm, probabilities) -> None:
@@ -764,8 +771,8 @@ class QwenAttentionLayer(Layer):
     def __init__(self, parameters, q_norm, k_norm, sequence_length, cache):
         self.parameters_ = parameters
         self.norms_ = [q_norm, k_norm]                       # BlockParameter
-        # head widths 64/128 run the backward attention core on the tensor cores; set False to
-        # force the exact fp32 kernels (every shape has them)
+        # head widths 64/128 (bf16 operands) and 256 (fp32 operands in three bf16 parts) run the backward
+        # attention core on the tensor cores; set False to force the exact fp32 kernels (every shape has them)
         self.tensor_core_backward = True
         self.weights_ = [q_norm.value(), k_norm.value()]
         self.sequence_length_ = sequence_length
