@@ -10,7 +10,7 @@
 // 3.4e-7; the fp32 kernels in attn_generic.cu 0.9e-7 to 3.8e-7, 3.6e-7 to 5.4e-7, 0.5e-6 to 2.1e-6 and 0.4e-6
 // to 2.1e-6.  (With two parts and accumulators that live as long as the row: 1.5e-6 to 2.4e-6, 4e-6, 0.4e-5
 // to 1.3e-5, 0.4e-5 to 1.8e-5.)  At 1000 tokens of 24 heads the fp32 kernels took 1078 us forward, 2258 dQ and
-// 3798 dK/dV, these take 59, 83 and 116 + 10 (the two-part ones 44, 52 and 99 + 11).
+// 3798 dK/dV, these take 69 with a gate (59 without), 83 and 116 + 10 (the two-part ones 44, 52 and 99 + 11).
 // Reference: src/llm/layers/qwen_attention.cc:68-119 (forward), :140-190 (backward).
 //
 // The width decides the layout.  A bf16 tile of 128 rows x 256 channels takes 64 KB of the SM's shared

@@ -412,9 +412,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 // Gates and SiLUs, the same two functions in the sequence kernels and the single-token ones, so that a
-// token gets the same bits from both.  One IEEE division each: the reciprocal unit would be 10 to 15 % of
-// the streaming kernels' time cheaper, but is an ulp off, rounds x * sigmoid(x) twice and flushes the tail
-// below -87 to zero.
+// token gets the same bits from both.  One IEEE division each.  It sets the pace of the kernels that do little else (the
+// convolution of 1000 tokens x 10240 channels takes 31 us with it, 17 with the reciprocal unit), but the
+// reciprocal is an ulp off, x * sigmoid(x) rounds twice, and the tail below -87 comes out as zero.
 __device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 // Two-lane fp32 arithmetic (one instruction per pair of values).

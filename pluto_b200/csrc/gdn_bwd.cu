@@ -36,7 +36,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // accesses).  HBM bound: core, z, dy in, dcore, dz out.  The norm gradient is summed in registers
 // over the strip and leaves as one row of `parts` per CTA, so nothing of size [rows, dim] is
 // written and read again for it (the earlier form: a CTA per row, 90 us here and 45 us in the
-// reduction at 48000 rows of 128; now 20 + 4).
+// reduction at 48000 rows of 128; now 21 + 6).
 // ------------------------------------------------------------------------------------------------
 template <int kPer, int kOutChannels>   // kOutChannels: channels a lane owns, 4 up to width 128, 8 up to 256
 __global__ void __launch_bounds__(256) gdn_out_bwd_kernel(const void* __restrict__ core, int core_is_bf16,
@@ -475,8 +475,8 @@ __global__ void gdn_conv_weight_bwd_kernel(const void* input, int in_is_bf16, co
 // shared memory.  Every element of x and dpost is read once (plus W - 1 at the seams of the ranges)
 // and dpre is computed once; the two kernels above recompute it for every tap, and the weight one
 // leaves a channel to a single thread for the whole sequence (220 + 938 us at 1000 tokens x 10240
-// channels, 100 MB of traffic; 39 us in this form, where the sigmoid and the rounding of 10 M
-// elements keep the issue slots busy).
+// channels, 100 MB of traffic; 45 us in this form, where the sigmoid's division and the rounding of
+// 10 M elements keep the issue slots busy).
 constexpr int kConvWarps = 4, kConvCluster = 8;
 template <int P, bool BF16>
 __device__ __forceinline__ void load_channels(const void* p, size_t i, float (&v)[P]) {

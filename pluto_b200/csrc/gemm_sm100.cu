@@ -321,9 +321,6 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Tiled TMA load of the CTA's own operand part; the bytes are counted on the barrier at `mbar_addr`,
 // a shared::cluster address (CTA 0's barrier for both CTAs of the pair).
 __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, int c0, int c1, int c2,
@@ -408,7 +405,7 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
-  cluster_sync_all();   // both CTAs' barriers exist before either touches the other's
+  cluster_sync();   // both CTAs' barriers exist before either touches the other's
   tc_fence_after();
   const uint32_t tmem = bar->tmem_base;
   pdl_wait();   // (as in the one-SM kernel: the set-up above ran beside the kernel before)
@@ -502,7 +499,7 @@ gemm_sm100_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   }
   tc_fence_before();
-  cluster_sync_all();   // neither CTA leaves while the other may still signal it or read its tiles
+  cluster_sync();   // neither CTA leaves while the other may still signal it or read its tiles
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kPairTile) : "memory");
@@ -553,10 +550,10 @@ cast_pad_kernel(const In* __restrict__ src, uint16_t* __restrict__ dst, int rows
 }
 
 // The upstream gradient's cast (as cast_pad_kernel, fp32 in) and its column sums from one reading of it:
-// CTA (x, y) takes the rows y * 8 + warp, + 8 gridDim.y, ... of its 128 columns, a lane four of them
-// and four rows at a time (one row in flight per warp and 16 chunks left three quarters of
-// the bandwidth unused; 16.5 us for 8192 x 2304 with the cast); the eight warps are added in order into partial[y][cols], the second kernel adds the
-// partial rows in order.
+// CTA (x, y) takes the rows y * 8 + warp, + 8 gridDim.y, ... of its 128 columns, a lane four of them and
+// four rows at a time (one row in flight per warp and 16 chunks left three quarters of the bandwidth
+// unused; 16.5 us for 8192 x 2304 with the cast).  The eight warps are added in order into
+// partial[y][cols], the second kernel adds the partial rows in order.
 constexpr int kBiasChunks = 64, kLeastBiasChunks = 16, kCastRows = 4;
 template <bool kHalf>
 __global__ void __launch_bounds__(256)

@@ -9,7 +9,7 @@
 // table is computed once into shared memory and every warp then walks heads, a lane owning kPer
 // channels of every 32 * kPer (4 consecutive ones where width, rotary half and strides allow).  A
 // stream bound by HBM; a CTA per (token, head), each computing its own sines, took 60 us at 1000
-// tokens of 24 + 4 heads of 256, this 20.  Token (b, t) has RoPE position positions[b] + t.
+// tokens of 24 + 4 heads of 256, this 23.  Token (b, t) has RoPE position positions[b] + t.
 #include "common.cuh"
 #include "engine.h"
 #include "qk_rows.cuh"
@@ -136,7 +136,7 @@ cudaError_t qk_prepare(cudaStream_t stream, const PrepareArgs& a) {
                       a.token_stride % 4 == 0 && a.page_stride % 4 == 0 && a.k_bases == nullptr &&
                       aligned(a.q_in, in) && aligned(a.k_in, in) && aligned(a.v_in, in) &&
                       aligned(a.q_out, a.q_out_is_bf16 ? 8 : 16) && aligned(a.k_cache, kv) && aligned(a.v_cache, kv);
-  // a warp per head while that still leaves fewer CTAs than two per SM, otherwise one CTA per token
+  // with fewer tokens than two per SM, a CTA for every eight heads of a token; else one CTA per token
   const int slabs = tokens < 2 * 148 ? (heads + 7) / 8 : 1;
   const dim3 grid(tokens, slabs);
   if (vector) qk_prepare_kernel<4><<<grid, 256, 0, stream>>>(a);
