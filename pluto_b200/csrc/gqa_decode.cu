@@ -126,7 +126,8 @@ __device__ __forceinline__ void store_output(const DecodeArgs& a, int b, int hea
 // kCluster true: grid (kv_heads, batch, parts), the parts of a (sequence, KV head) are one cluster and
 //   cut the sequence's own length evenly; their partials meet in distributed shared memory and the
 //   output leaves from here, so the call is one launch and needs no scratch.
-template <int D, bool kCluster>
+// kThirds: P in three bf16 parts (24 bits) instead of two, see keeps_24_bits.
+template <int D, bool kCluster, bool kThirds>
 __global__ void __launch_bounds__(kDecodeThreads, 2)
 gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               DecodeArgs a) {
@@ -138,7 +139,6 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
   constexpr int kParts = kChannelParts<D>, kWarps = kTokenWarps * kParts;
   static_assert((kWarps + 1) * 32 == kDecodeThreads, "warps");
   constexpr int kOwnBlocks = D / 16 / kParts;     // 16-channel blocks of the accumulator a warp owns
-  constexpr bool kThirds = D == 256;              // P in three bf16 parts
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -297,8 +297,9 @@ gqa_decode_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
           s[nb][i] = token < end ? (s[nb][i] + s_odd[nb][i]) * scale_log2 : -INFINITY;
           tile_max[i >> 1] = fmaxf(tile_max[i >> 1], s[nb][i]);
         }
-      // P enters P V as a bf16 high part and a bf16 remainder, 16 bits, at head width 256 as a second
-      // remainder too, 24 bits; the extra MMAs are free in a bandwidth-bound kernel.
+      // P enters P V as a bf16 high part and a bf16 remainder, 16 bits, which is free in a bandwidth-bound
+      // kernel; with kThirds as a second remainder too, 24 bits, which is not (64 sequences of 32768 tokens,
+      // 8 KV heads of 128: 718 us with two, 796 with three).
       uint32_t pf[4], pl[4], pt[4];
       float correction[2];
 #pragma unroll
@@ -692,12 +693,18 @@ bool make_pool_map(CUtensorMap* map, const void* base, const DecodeArgs& a, int 
 
 }  // namespace
 
-// Head width 256 keeps the plain kernel for fp32 queries, which the tensor cores would round to bf16, and
-// for fp32 results that nothing rounds: P has 24 bits either way, but a score is a sum that the tensor
-// cores truncate (relative error of the result 2.1e-7 against 1.3e-7 at 64 tokens, 2.7e-7 against 1.9e-7 at
-// 500, equal from 4000 on).
+namespace {
+// Calls that the tensor-core form took over from the plain kernel keep its precision: P with 24 bits.  They are
+// head width 256 and contiguous caches of a length that 16 does not divide; all others have always had 16.
+bool keeps_24_bits(const DecodeArgs& a) { return a.head_dim == 256 || (a.block_table == nullptr && a.page_size % 16 != 0); }
+}  // namespace
+
+// Of those calls the plain kernel keeps fp32 queries, which the tensor cores would round to bf16, and fp32
+// results that nothing rounds: P has 24 bits either way, but a score is a sum that the tensor cores truncate
+// (width 256, relative error of the result 2.1e-7 against 1.3e-7 at 64 tokens, 2.7e-7 against 1.9e-7 at 500,
+// equal from 4000 on).
 bool gqa_decode_uses_tensor_cores(const DecodeArgs& a) {
-  if (a.head_dim == 256 && (!a.q_is_bf16 || (!a.round && !a.out_is_bf16))) return false;
+  if (keeps_24_bits(a) && (!a.q_is_bf16 || (!a.round && !a.out_is_bf16))) return false;
   const int group = a.q_heads / a.kv_heads;
   const int pages = a.block_table ? a.num_pages : a.batch;
   return a.k_bases == nullptr && a.kv_is_bf16 && (a.head_dim == 64 || a.head_dim == 128 || a.head_dim == 256) && group <= 16 &&
@@ -728,10 +735,10 @@ cudaError_t launch_decode(void (*kernel)(Params...), dim3 grid, int threads, siz
   return cudaLaunchKernelEx(&config, kernel, params...);
 }
 
-template <int D>
+template <int D, bool kThirds>
 cudaError_t launch_tc(cudaStream_t stream, const CUtensorMap& map_k, const CUtensorMap& map_v, const DecodeArgs& a,
                       int parts) {
-  auto kernel = parts > 0 ? gqa_decode_tc<D, true> : gqa_decode_tc<D, false>;
+  auto kernel = parts > 0 ? gqa_decode_tc<D, true, kThirds> : gqa_decode_tc<D, false, kThirds>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(decode_smem<D>()));
   if (e == cudaSuccess && parts > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -785,9 +792,11 @@ cudaError_t gqa_decode(cudaStream_t stream, const DecodeArgs& args) {
     if (!make_pool_map(&map_k, a.k_base, a, pages) || !make_pool_map(&map_v, a.v_base, a, pages))
       return cudaErrorInvalidValue;
     const int parts = cluster_parts(a);
-    e = a.head_dim == 256 ? launch_tc<256>(stream, map_k, map_v, a, parts)
-        : a.head_dim == 128 ? launch_tc<128>(stream, map_k, map_v, a, parts)
-                            : launch_tc<64>(stream, map_k, map_v, a, parts);
+    const bool thirds = keeps_24_bits(a);
+    auto launch = a.head_dim == 256 ? launch_tc<256, true>
+                  : a.head_dim == 128 ? (thirds ? launch_tc<128, true> : launch_tc<128, false>)
+                                      : (thirds ? launch_tc<64, true> : launch_tc<64, false>);
+    e = launch(stream, map_k, map_v, a, parts);
     if (e != cudaSuccess || parts > 0) return e;
   } else {
     e = launch_decode(gqa_decode_generic, dim3(a.q_heads, a.batch, a.splits), 128, 0, stream, 0, a);

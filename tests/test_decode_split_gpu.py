@@ -120,3 +120,29 @@ def test_width_256_on_the_tensor_cores(batch, hq, hkv, longest, page):
         assert ((got[b].double() - want).abs() <= half_ulp + 2e-6).all()
         assert torch.equal(got[b], got[b].bfloat16().float())
     assert _capi.kernel_status() == 0
+
+
+@pytest.mark.parametrize("dim,hq,hkv", [(64, 12, 12), (128, 10, 2)])
+@pytest.mark.parametrize("batch,capacity", [(3, 1), (5, 182), (2, 1455), (1, 20003)])
+def test_contiguous_caches_off_16_tokens_keep_24_bits(dim, hq, hkv, batch, capacity):
+    """Without a block table the cache may have any length.  Where 16 does not divide it, P keeps 24 bits: the
+    rounded result is the nearest bf16 value or, within 2e-6 of a tie, the other neighbour (two bf16 parts
+    leave 1e-5); an unrounded fp32 result and fp32 queries run in fp32 throughout."""
+    gen = torch.Generator(device="cuda").manual_seed(capacity)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    k, v = rnd(batch, capacity, hkv, dim).bfloat16(), rnd(batch, capacity, hkv, dim).bfloat16()
+    lens = torch.randint(1, capacity + 1, (batch,), device="cuda", generator=gen, dtype=torch.int32)
+    lens[0] = capacity
+    for q in (rnd(batch, hq, dim).bfloat16(), rnd(batch, hq, dim)):
+        new = lambda: torch.empty(batch, hq, dim, device="cuda")
+        rounded, lse = gqa_decode(q, k, v, lens, capacity, out=new(), want_lse=True)
+        plain = gqa_decode(q, k, v, lens, capacity, round_to_bfloat16=False, out=new())
+        for b, n in enumerate(lens.tolist()):
+            kk, vv = (x[b, :n].double().repeat_interleave(hq // hkv, 1) for x in (k, v))
+            s = torch.einsum("hd,thd->ht", q[b].double(), kk) / math.sqrt(dim)
+            want = torch.einsum("ht,thd->hd", torch.softmax(s, -1), vv)
+            assert (plain[b].double() - want).abs().max().item() < 3e-6
+            assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max().item() < 5e-6
+            half_ulp = 2.0 ** (torch.floor(torch.log2(want.abs().clamp(min=1e-30))) - 8)
+            assert ((rounded[b].double() - want).abs() <= half_ulp + 2e-6).all()
+    assert _capi.kernel_status() == 0
