@@ -284,8 +284,9 @@ size_t pluto_gqa_decode_workspace_bytes(int batch, int q_heads, int kv_heads, in
  *   max_seq_len  host upper bound of seq_lens (sizes the grid; no device read-back)
  *   out          [batch, Hq, D] (out_dtype);  lse optional fp32 [batch, Hq]
  *   workspace    >= pluto_gqa_decode_workspace_bytes(...) bytes, 16-byte aligned
- * bf16 cache with head_dim 64/128/256 takes the bandwidth-bound path (bulk copies + mma); anything
- * else the exact fp32 path.  The result does not depend on which SM ran which chunk. */
+ * bf16 cache with head_dim 64/128/256 takes the bandwidth-bound path (bulk copies + mma), at head_dim 256
+ * and for contiguous caches whose length 16 does not divide with bf16 queries and a rounded or bf16 result;
+ * anything else the exact fp32 path.  The result does not depend on which SM ran which chunk. */
 int pluto_gqa_decode(pluto_stream_t stream, const void* q, int q_dtype, const void* gate,
                      int gate_dtype, size_t gate_token_stride, size_t gate_head_stride,
                      const pluto_kv_cache* cache /* host */, const int32_t* seq_lens,
